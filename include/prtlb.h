@@ -136,7 +136,7 @@ int prt_flow_dev(prt_ctx* ctx, const uint8_t* d_mat, const prt_flow_params* p,
  * buffers but no allocator).  The caller passes d_mat and d_vel_out as
  * device pointers it owns and a cudaStream_t (NULL: the default stream); no
  * context is needed and nothing is allocated or freed.  All other scratch
- * (both lattices, masks, partial sums, control block) is one 48 MiB
+ * (the lattice, pore maps, partial sums, control block) is one 48 MiB
  * file-scope __device__ array in the library, which every GPU that loads
  * the library holds until exit; a grid that does not fit (64^3 D3Q19 at
  * float32 does) is refused with PRT_E_INVALID and a message giving both

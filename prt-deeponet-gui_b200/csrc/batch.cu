@@ -4,7 +4,7 @@
 // blocks of kFlowThreads slots and listed as tiles (job, first block, block
 // count).  One persistent launch walks the tile list and runs one LB iteration of every
 // job that is not done, each job at its own iteration count and parity.
-// The arithmetic per voxel is lb_cell_rw, the per-block |u_x| partials are
+// The arithmetic per voxel is lb_cell, the per-block |u_x| partials are
 // block_sum_store over the same blocks of slots, and the convergence update is
 // flow_ctrl_advance, so a job's iterations, decisions and final field are
 // bit-identical to the single-solve loop whatever else shares the batch.
@@ -72,13 +72,14 @@ __global__ void __launch_bounds__(kFlowThreads, M::batch_min_blocks)
             continue;
         }
         const int nf = sj.fm.nf;
-        const Lat<S> lat = lattices<L>(static_cast<S*>(sj.f), nf, (it & 1) != 0);
+        const Lat<S> lat = lattice<L>(static_cast<S*>(sj.f), sj.fm.rs, (it & 1) != 0);
 #pragma unroll 1
         for (int b = tl.b0; b < tl.b0 + tl.nb; ++b) {
             const int slot = b * kFlowThreads + threadIdx.x;
             double acc = 0.0;
-            if (slot < nf)
-                acc = lb_cell_rw<L, M>(lat, sj.fm, sj.g, job_constants<UNI>(kcu, sj.kc), slot);
+            int far[L::NP];
+            far_slots<L, Far::packed>(sj.fm, sj.g, slot, far);
+            if (slot < nf) acc = lb_cell<L, M>(lat, job_constants<UNI>(kcu, sj.kc), slot, far);
             if (check) block_sum_store(acc, sj.partials + b);
         }
         if (!advance) {  // uniform over the block

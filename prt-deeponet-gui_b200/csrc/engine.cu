@@ -218,26 +218,6 @@ int rebuild(prt_batch* b) {
         adr_cnt += (size_t)nbk + 1;
         b->h_done.push_back(&J.ctrl->done);
     }
-    // pull tables: each solve chose them against the whole L2 cache; in a
-    // batch they pay only while the flow jobs' lattices and tables together
-    // fit in half of it, otherwise the tables' bytes add to the DRAM traffic
-    // and the kernels look the upstream slots up through the maps (the same
-    // slots either way, so the fields do not change)
-    {
-        long long ws = 0, l2 = 0;
-        for (int i = 0; i < b->nflow; ++i) {
-            const prt_ctx* c = b->order[i];
-            const FlowState& F = c->flow;
-            const int q = F.p.nd == 3 ? 19 : 9;
-            const long long es = F.p.precision == PRT_FP64 ? 8 : F.p.precision == PRT_FP16 ? 2 : 4;
-            ws += 2ll * q * F.fm.nf * es + (F.fm.nbr ? flow_nbr_bytes(q, F.fm.nf) / 2 : 0);
-            l2 = c->l2_bytes;
-        }
-        const char* v = std::getenv("PRT_NBR_TABLE");
-        const bool forced = v && v[0] == '1';
-        if (!forced && ws > l2 / 2)
-            for (FlowJob& J : b->h_flow) J.fm.nbr = nullptr;
-    }
     for (int c = 0; c < kFlowClasses; ++c) b->flow_uni[c] = false;
     {
         bool seen[kFlowClasses] = {}, differ[kFlowClasses] = {};

@@ -93,17 +93,29 @@ struct Pop<__half> {
     }
 };
 
+// Whether the collision forms its store addresses again instead of keeping
+// those of the loads, which use the same places: 2 (Q - 1) registers that
+// spill in D3Q19's float64 arithmetic.  index: again from the slot numbers,
+// base: again from the lattice's address.  Measured on 128^3 / 64^3 packs (us
+// an iteration, none / index / base): float64 72.8 / 57.3 / 56.9 and 8.3 /
+// 6.6 / 6.1, float32 with float64 momentum 32.1 / 28.6 / 29.3 and 4.8 / 4.7 /
+// 4.9, float16 22.4 / 20.1 / 20.8 and - / 3.8 / 4.3; float32 alone fits its
+// registers either way (4.18 / 4.42 / - at 64^3).
+enum class Fresh { none, index, base };
+
 // Precision modes: storage type S, arithmetic R for the symmetric part and
 // RA for the momentum and the antisymmetric non-equilibrium part (a small
 // difference of two O(u) numbers), and the resident blocks of kFlowThreads
 // per SM the register budget is cut for (single-solve and batched steps).
+// `fresh`: see Fresh.
 // `staged`: the arrived populations go to shared memory by cp.async, so no
 // register waits on a gather load (4- and 8-byte populations only).
 struct ModeF64 {  // the reference's arithmetic
     using S = double;
     using R = double;
     using RA = double;
-    static constexpr int min_blocks = 6;
+    static constexpr int min_blocks = 7;
+    static constexpr Fresh fresh = Fresh::base;
     static constexpr int batch_min_blocks = 6;
     static constexpr bool staged = true;
 };
@@ -114,6 +126,7 @@ struct ModeF32 {  // float32 populations, float32 collision
     // 64 registers (8 blocks per SM): at 48 (10 blocks) an iteration took
     // 5.46 us at 64^3 and 4.73 at 48^3, at 64 it takes 4.58 and 3.17
     static constexpr int min_blocks = 8;
+    static constexpr Fresh fresh = Fresh::none;
     static constexpr int batch_min_blocks = 8;
     static constexpr bool staged = true;
 };
@@ -125,6 +138,7 @@ struct ModeF32D {  // float32 populations, float64 momentum
     // (917 blocks) still fits one wave at 8 blocks per SM (5.67 -> 5.41 us
     // per iteration; 128^3 unchanged)
     static constexpr int min_blocks = 8;
+    static constexpr Fresh fresh = Fresh::index;
     static constexpr int batch_min_blocks = 8;
     static constexpr bool staged = true;
 };
@@ -133,88 +147,154 @@ struct ModeF16 {  // scaled float16 populations, float32 collision
     using R = float;
     using RA = float;
     static constexpr int min_blocks = 6;
+    static constexpr Fresh fresh = Fresh::index;
     static constexpr int batch_min_blocks = 6;
     static constexpr bool staged = false;
 };
 
-// Slots of the upstream voxels x - e_i of pore slot k (periodic), -1 where
-// that voxel is rock.  The three candidate coordinates per axis are formed
-// once; each direction then costs one index and one imap load.
-template <class L>
-__device__ __forceinline__ void upstream_slots(const FlowMap& fm, const Grid& g, int k,
-                                               int (&src)[L::Q]) {
-    int x, y, z;
-    unpack_cell((unsigned)fm.cells[k], fm, x, y, z);
-    const int X[3] = {x == 0 ? g.nx - 1 : x - 1, x, x == g.nx - 1 ? 0 : x + 1};
-    const int Y[3] = {y == 0 ? g.ny - 1 : y - 1, y, y == g.ny - 1 ? 0 : y + 1};
-    const int Z[3] = {z == 0 ? g.nz - 1 : z - 1, z, z == g.nz - 1 ? 0 : z + 1};
-    src[0] = k;
-#pragma unroll
-    for (int i = 1; i < L::Q; ++i) {
-        const int a = 1 - L::c(i, 0), b = 1 - L::c(i, 1), c = 1 - L::c(i, 2);
-        src[i] = fm.imap[(X[a] * g.ny + Y[b]) * g.nz + Z[c]];
-    }
-}
-
-// Gather the arrived populations of pore voxel number k (see the file
-// comment).  Lattices hold the pore voxels only, in C order: voxel
-// cells[k] is slot k, and imap[voxel] is the slot of a pore voxel or -1.
-// The two lattices of a solve as one array and 32-bit element offsets: the
-// read lattice starts at element rd, the write lattice at wr (0 or Q*nf
-// each; 2*Q*nf < 2^31 is checked at set-up), so every address is one
-// 32-bit index and one wide multiply-add off the base.
+// One lattice, updated in place (see the file comment of lb_flow.cu).  Row i
+// holds one population of every pore slot (elements [0, nf)) and, behind
+// them, the pair's rock links; row i starts at element i * rs.  In an
+// iteration the pair (a, b), e_b = -e_a, of the voxel in slot k uses two
+// places: its own element k of row `b` (even iterations) or `a` (odd), and
+// element far of the other row, far being the slot of the voxel x + e_a or,
+// when that is rock, the link's own element.  f_a is read from the own place
+// and f_b written there; f_b is read from the far place and f_a written
+// there.  No other thread touches either place in the iteration.
+// Offsets are unsigned 32-bit: rs is at most the voxel count (a direction
+// has no more links than the grid has rock voxels) and at most 2 nf, and
+// 2 Q nf < 2^31 is checked at set-up.
 template <class S>
 struct Lat {
     S* f;
-    int rd, wr, nf;
-    __device__ const S* in(int i, int slot) const { return f + (rd + i * nf + slot); }
-    __device__ S* out(int i, int slot) const { return f + (wr + i * nf + slot); }
+    unsigned rs, own, far;  // far / own: element offset of the rows of the two places
+    __device__ S* at_own(int a, unsigned k) const { return f + (a * rs + own + k); }
+    __device__ S* at_far(int a, unsigned slot) const { return f + (a * rs + far + slot); }
 };
 
 template <class L, class S>
-__device__ __forceinline__ Lat<S> lattices(S* f, int nf, bool odd) {
-    const int qn = L::Q * nf;
-    return Lat<S>{f, odd ? qn : 0, odd ? 0 : qn, nf};
+__device__ __forceinline__ Lat<S> lattice(S* f, unsigned rs, bool odd) {
+    constexpr unsigned d = L::pb(0) - L::pa(0);  // the same for every pair
+    return Lat<S>{f, rs, odd ? 0u : d * rs, odd ? d * rs : 0u};
 }
 
-// The element offsets (into the two lattices) of the populations slot k
-// pulls in an iteration whose read lattice is `lat`: direction i from the
-// upstream slot src[i] of the read lattice, or, when that voxel is rock,
-// x's own value of two iterations back, opp(i) in the write lattice.
-template <class L, class S>
-__device__ __forceinline__ void pull_offsets(const Lat<S>& lat, int k, const int (&src)[L::Q],
-                                             int (&off)[L::Q]) {
-    off[0] = lat.rd + k;
+// The far places of slot k (see Lat), one per pair, from the packed cell and
+// the voxel map: the slot of x + e_a (periodic), or nf + the rank of this
+// link among the pair's links, which the warp forms from its first link's
+// rank (fm.link) and the lanes below.  Every lane of the warp calls it;
+// lanes beyond the last slot get nothing.
+template <class L>
+__device__ __forceinline__ void far_slots_map(const FlowMap& fm, const Grid& g, int k,
+                                              int (&far)[L::NP]) {
+    const bool live = k < fm.nf;
+    int x = 0, y = 0, z = 0;
+    if (live) unpack_cell((unsigned)fm.cells[k], fm, x, y, z);
+    // the candidate coordinates per axis are formed once; a direction then
+    // costs one index and one map load
+    const int X[3] = {x == 0 ? g.nx - 1 : x - 1, x, x == g.nx - 1 ? 0 : x + 1};
+    const int Y[3] = {y == 0 ? g.ny - 1 : y - 1, y, y == g.ny - 1 ? 0 : y + 1};
+    const int Z[3] = {z == 0 ? g.nz - 1 : z - 1, z, z == g.nz - 1 ? 0 : z + 1};
 #pragma unroll
-    for (int i = 1; i < L::Q; ++i)
-        off[i] = src[i] >= 0 ? lat.rd + i * lat.nf + src[i] : lat.wr + L::opp(i) * lat.nf + k;
-}
-
-// The same offsets from the pull tables fm.nbr, one per parity of the read
-// lattice (coalesced: entry i-1 of every slot is one contiguous row).
-template <class L, class S>
-__device__ __forceinline__ void pull_offsets_table(const FlowMap& fm, const Lat<S>& lat, int k,
-                                                   int (&off)[L::Q]) {
-    const int* tab = fm.nbr + (lat.rd != 0 ? (L::Q - 1) * fm.nf : 0);
-    off[0] = lat.rd + k;
+    for (int p = 0; p < L::NP; ++p) {
+        const int i = L::pa(p);
+        far[p] = 0;
+        if (live)
+            far[p] = fm.imap[(X[1 + L::c(i, 0)] * g.ny + Y[1 + L::c(i, 1)]) * g.nz +
+                             Z[1 + L::c(i, 2)]];
+    }
+    const unsigned below = (1u << (threadIdx.x & 31)) - 1u;
+    const int nw = (fm.nf + 31) >> 5;
 #pragma unroll
-    for (int i = 1; i < L::Q; ++i) off[i] = __ldg(tab + (i - 1) * fm.nf + k);
+    for (int p = 0; p < L::NP; ++p) {
+        const unsigned links = __ballot_sync(0xffffffffu, far[p] < 0);
+        if (far[p] < 0) far[p] = fm.nf + fm.link[p * nw + (k >> 5)] + __popc(links & below);
+    }
 }
 
-template <class L, class S>
-__device__ __forceinline__ void gather_from_offsets(const Lat<S>& lat, const int (&off)[L::Q],
-                                                    float inv, typename Pop<S>::H (&h)[L::Q]) {
+// The packed table of far places (fm.pack, see FlowMap) as one thread of a warp
+// holds it: its own words and its lane's share of the warp's bases.
+template <class L>
+struct Packed {
+    static constexpr int words = L::NP > 4 ? 3 : 2;
+    unsigned w[words];
+    int base;
+};
+
+// Ints before the bases of the packed table of nf slots.
+template <class L>
+__host__ __device__ inline long long packed_words(int nf) {
+    return (long long)Packed<L>::words * ((nf + 31) / 32 * 32);
+}
+
+template <class L>
+__device__ __forceinline__ Packed<L> load_packed(const FlowMap& fm, int k) {
+    Packed<L> q;
+    const unsigned nfp = (unsigned)(fm.nf + 31) / 32 * 32;
+    const int lane = threadIdx.x & 31;
+    q.base = 0;
+    if ((unsigned)k < nfp) {  // uniform over the warp
+        const uint2 v = __ldg(reinterpret_cast<const uint2*>(fm.pack) + k);
+        q.w[0] = v.x;
+        q.w[1] = v.y;
+        if (Packed<L>::words > 2) q.w[Packed<L>::words - 1] = __ldg(fm.pack + (2 * nfp + k));
+        if (lane < 2 * L::NP)
+            q.base = __ldg(fm.pack + (Packed<L>::words * nfp + (k >> 5) * (2 * L::NP) + lane));
+    } else {
 #pragma unroll
-    for (int i = 0; i < L::Q; ++i) h[i] = Pop<S>::ld(lat.f + off[i], inv);
+        for (int i = 0; i < Packed<L>::words; ++i) q.w[i] = 0;
+    }
+    return q;
 }
 
+// The far places of slot k from its packed words; a warp whose places do not
+// fit the packed form looks them up in the maps.  Every lane of the warp
+// calls it.
+template <class L>
+__device__ __forceinline__ void far_slots_packed(const FlowMap& fm, const Grid& g, int k,
+                                                 const Packed<L>& q, int (&far)[L::NP]) {
+    const unsigned last = q.w[Packed<L>::words - 1];
+    if ((int)last < 0) {  // uniform over the warp
+        far_slots_map<L>(fm, g, k, far);
+        return;
+    }
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        const int src = p + ((last >> (8 + p)) & 1u) * L::NP;
+        const unsigned d = (q.w[p / 4] >> (8 * (p % 4))) & 0xffu;
+        far[p] = __shfl_sync(0xffffffffu, q.base, src) + (int)d;
+    }
+}
+
+// How a launch finds its far places: from the plain table (one coalesced load
+// per pair and 36 B a slot in D3Q19), or from the packed table (14.3 B) and
+// the maps.  The plain table's chain is the shortest and wins while it and
+// the lattice stay in the L2 (flow_use_nbr): us an iteration, plain / packed
+// / maps alone, 64^3 float32 4.2 / 4.6 / 5.0, 96^3 float64 16.2 / 17.6 / 23.6,
+// 128^3 float16 20.3 / 21.7 / 26.2; beyond it the bytes decide: 128^3 float32
+// 26.7 / 24.9 / 30.7, 192^3 112 / 104 / 126.
+enum class Far { table, packed };
+
+template <class L, Far F>
+__device__ __forceinline__ void far_slots(const FlowMap& fm, const Grid& g, int k,
+                                          int (&far)[L::NP]) {
+    if constexpr (F == Far::table) {
+#pragma unroll
+        for (int p = 0; p < L::NP; ++p) far[p] = k < fm.nf ? __ldg(fm.nbr + p * fm.nf + k) : 0;
+    } else {
+        far_slots_packed<L>(fm, g, k, load_packed<L>(fm, k), far);
+    }
+}
+
+// The populations that arrive at slot k in this iteration.
 template <class L, class S>
-__device__ __forceinline__ void gather(const Lat<S>& lat, int k, const FlowMap& fm, const Grid& g,
+__device__ __forceinline__ void gather(const Lat<S>& lat, int k, const int (&far)[L::NP],
                                        float inv, typename Pop<S>::H (&h)[L::Q]) {
-    int src[L::Q], off[L::Q];
-    upstream_slots<L>(fm, g, k, src);
-    pull_offsets<L, S>(lat, k, src, off);
-    gather_from_offsets<L, S>(lat, off, inv, h);
+    h[0] = Pop<S>::ld(lat.f + k, inv);
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        h[L::pa(p)] = Pop<S>::ld(lat.at_own(L::pa(p), k), inv);
+        h[L::pb(p)] = Pop<S>::ld(lat.at_far(L::pa(p), far[p]), inv);
+    }
 }
 
 // 128-thread blocks: at 64^3 (458 blocks of 256 for 148 SMs) finer blocks
@@ -232,8 +312,12 @@ __device__ __forceinline__ void cp_async_pop(S* dst, const S* src) {
         asm volatile("cp.async.ca.shared.global [%0], [%1], 8;\n" ::"r"(d), "l"(src) : "memory");
 }
 
-__device__ __forceinline__ void cp_async_wait_all() {
-    asm volatile("cp.async.commit_group;\ncp.async.wait_group 0;\n" ::: "memory");
+__device__ __forceinline__ void cp_async_commit() {
+    asm volatile("cp.async.commit_group;\n" ::: "memory");
+}
+template <int N>
+__device__ __forceinline__ void cp_async_wait() {
+    asm volatile("cp.async.wait_group %0;\n" ::"n"(N) : "memory");
 }
 
 // The arrived populations of one thread in shared memory: element i of the
@@ -248,10 +332,15 @@ struct Staged {
 // thread's column of a [Q][kFlowThreads] shared array): the same sources,
 // but no register is held while a load is in flight.
 template <class L, class S>
-__device__ __forceinline__ void gather_staged(const Lat<S>& lat, const int (&off)[L::Q], S* col) {
+__device__ __forceinline__ void gather_staged(const Lat<S>& lat, int k, const int (&far)[L::NP],
+                                              S* col) {
+    cp_async_pop(col, lat.f + k);
 #pragma unroll
-    for (int i = 0; i < L::Q; ++i) cp_async_pop(col + i * kFlowThreads, lat.f + off[i]);
-    cp_async_wait_all();
+    for (int p = 0; p < L::NP; ++p) {
+        cp_async_pop(col + L::pa(p) * kFlowThreads, lat.at_own(L::pa(p), k));
+        cp_async_pop(col + L::pb(p) * kFlowThreads, lat.at_far(L::pa(p), far[p]));
+    }
+    cp_async_commit();
 }
 
 template <class R, class RA>
@@ -295,15 +384,26 @@ __device__ __forceinline__ Moments<R, RA> moments(const HA& h, double half_g) {
 // shifted variables, written with J = rho u so that rho cancels in the
 // antisymmetric equilibrium (w rho 3 e.u = 3 w e.J) and rho u u = J J / rho in
 // the symmetric one.  The new population is h + delta with delta summed
-// first, so the stored result rounds once; it goes to slot i of voxel c.
-template <class L, class S, class R, class RA, class HA>
-__device__ __forceinline__ void collide_store(const Lat<S>& lat, int c, const HA& h,
-                                              const Moments<R, RA>& m, const LbParams& kc) {
+// first, so the stored result rounds once; f_a goes to the pair's far place
+// and f_b to its own (see Lat).
+template <class L, Fresh F, class S, class R, class RA, class HA>
+__device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const int (&far)[L::NP],
+                                              const HA& h, const Moments<R, RA>& m,
+                                              const LbParams& kc) {
+    Lat<S> lat = lat0;
+    int to[L::NP];
+    if (F == Fresh::base) asm volatile("" : "+l"(lat.f));
+    if (F == Fresh::index) asm volatile("" : "+r"(k));
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        to[p] = far[p];
+        if (F == Fresh::index) asm volatile("" : "+r"(to[p]));
+    }
     const R omp = R(kc.omp);
     const R inv_rho = R(m.inv_rho);
     const R heq0 = R(L::w(0)) * (m.drho - R(1.5) * m.jsq);
     const R h0 = R(h[0]);
-    Pop<S>::st(lat.out(0, c), h0 - omp * (h0 - heq0), kc.scale);
+    Pop<S>::st(lat.f + k, h0 - omp * (h0 - heq0), kc.scale);
 #pragma unroll
     for (int p = 0; p < L::NP; ++p) {
         const int a = L::pa(p), b = L::pb(p);
@@ -321,58 +421,35 @@ __device__ __forceinline__ void collide_store(const Lat<S>& lat, int c, const HA
         const RA dma = RA(kc.omm) * (RA(0.5) * (RA(h[a]) - RA(h[b])) - RA(3.0 * L::w(a)) * eJ);
         const R dm = R(dma);
         const R gp = R(kc.guo[p]);
-        Pop<S>::st(lat.out(a, c), ha + ((gp - dp) - dm), kc.scale);
-        Pop<S>::st(lat.out(b, c), hb + ((dm - dp) - gp), kc.scale);
+        Pop<S>::st(lat.at_far(a, to[p]), ha + ((gp - dp) - dm), kc.scale);
+        Pop<S>::st(lat.at_own(a, k), hb + ((dm - dp) - gp), kc.scale);
     }
 }
 
-// One pore voxel (slot k) of one LB iteration from the read lattice into
-// the write lattice, the offsets of its pulls already found: gather,
-// moments, collision, store; returns |u_x| for the convergence mean.
+// One pore voxel (slot k) of one LB iteration, its far places already found:
+// gather, moments, collision, store; returns |u_x| for the convergence mean.
 template <class L, class M>
-__device__ __forceinline__ double lb_cell_offs(const Lat<typename M::S>& lat, const LbParams& kc,
-                                               int k, const int (&off)[L::Q]) {
+__device__ __forceinline__ double lb_cell(const Lat<typename M::S>& lat, const LbParams& kc, int k,
+                                          const int (&far)[L::NP]) {
     using S = typename M::S;
     using R = typename M::R;
     using RA = typename M::RA;
     if constexpr (M::staged) {
         __shared__ S stage[L::Q * kFlowThreads];
         S* col = stage + threadIdx.x;
-        gather_staged<L, S>(lat, off, col);
+        gather_staged<L, S>(lat, k, far, col);
+        cp_async_wait<0>();
         const Staged<S> h{col};
         const Moments<R, RA> m = moments<L, R, RA>(h, kc.half_g);
-        collide_store<L, S, R, RA>(lat, k, h, m, kc);
+        collide_store<L, L::Q == 19 ? M::fresh : Fresh::none, S, R, RA>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     } else {
         typename Pop<S>::H h[L::Q];
-        gather_from_offsets<L, S>(lat, off, kc.inv_scale, h);
+        gather<L, S>(lat, k, far, kc.inv_scale, h);
         const Moments<R, RA> m = moments<L, R, RA>(h, kc.half_g);
-        collide_store<L, S, R, RA>(lat, k, h, m, kc);
+        collide_store<L, L::Q == 19 ? M::fresh : Fresh::none, S, R, RA>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     }
-}
-
-// The offsets of slot k's pulls: from the pull tables when the solve has
-// them, else from the packed cell and the voxel map (the same offsets).
-template <class L, class S>
-__device__ __forceinline__ void find_pulls(const Lat<S>& lat, const FlowMap& fm, const Grid& g,
-                                           int k, int (&off)[L::Q]) {
-    if (fm.nbr) {
-        pull_offsets_table<L, S>(fm, lat, k, off);
-    } else {
-        int src[L::Q];
-        upstream_slots<L>(fm, g, k, src);
-        pull_offsets<L, S>(lat, k, src, off);
-    }
-}
-
-// The same, finding the pulls first.
-template <class L, class M>
-__device__ __forceinline__ double lb_cell_rw(const Lat<typename M::S>& lat, const FlowMap& fm,
-                                             const Grid& g, const LbParams& kc, int k) {
-    int off[L::Q];
-    find_pulls<L, typename M::S>(lat, fm, g, k, off);
-    return lb_cell_offs<L, M>(lat, kc, k, off);
 }
 
 // Block sum of one double per thread (warp shuffles, then the warp sums in

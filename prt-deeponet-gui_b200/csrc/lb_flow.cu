@@ -7,16 +7,21 @@
 //   solid voxels: post-collision = the reversed ARRIVED populations
 //   periodic streaming of every population (np.roll on every axis)
 //
-// Here one launch does one whole iteration as a pull from lattice Lr (the
-// post-collision populations of the previous iteration) into lattice Lw:
-// a pore voxel x gathers f_i from x - e_i, collides and writes its values
-// contiguously into its own slots of Lw.  When x - e_i is rock, the reference
-// rule "the solid voxel sends back what arrived there one iteration earlier"
-// makes the arriving value x's own post-collision population in direction
-// opp(i) from two iterations ago -- which is still in Lw[opp(i)][x], not yet
-// overwritten, and read by the same thread before it writes.  Solid voxels
-// therefore do no work at all, and the transient is the reference's, not
-// only its steady state.
+// Here one launch does one whole iteration in place, on one lattice: for each
+// pair of opposite directions (a, b) a voxel reads f_a from its own place
+// and f_b from the place of its neighbour x + e_a, and writes the collided
+// f_b and f_a to the same two places, swapped (the storage order of
+// "esoteric pull" streaming, M. Lehmann, Computation 10 (2022) 92).  The two
+// places swap rows with the iteration parity, which completes the streaming.
+// When x + e_a is rock, the reference rule "the solid voxel sends back what
+// arrived there one iteration earlier" is what the place does by itself: it
+// keeps the f_a written into it until the next iteration of the same parity
+// reads it as f_b.  The same holds for the own place when x - e_a is rock.
+// So rock voxels do no work, the transient is the reference's and not only
+// the steady state, and an iteration reads and writes every population once.
+// (Pulling from one lattice into another reads the two-iterations-old values
+// from partly used sectors of the lattice it is about to overwrite, about
+// one more lattice pass per iteration where the lattices exceed the L2.)
 //
 // Populations are stored shifted, h_i = f_i - w_i: the non-equilibrium part
 // that carries the viscous stress is of the order of the force (1e-7) and
@@ -27,35 +32,40 @@
 
 namespace prt {
 
-// One whole LB iteration t: lattice (t & 1) is read, lattice ((t + 1) & 1)
-// written; solid voxels do nothing.  late: the next iteration is let in
-// after this one's stores (see pdl_late).
-template <class L, class M, bool ODD, bool CHECK>
+// One whole LB iteration t (ODD = t & 1); solid voxels do nothing.  late: the
+// next iteration is let in after this one's stores (see pdl_late).
+//
+// Bound by the L2 and DRAM traffic where the lattice exceeds the L2 (192^3),
+// by latency below; in place it reads and writes each population once and
+// finds 9 places instead of 18.  Odd iterations walk the slots downwards, so
+// an iteration starts on what the one before left in the L2: 128^3 float32
+// 28.4 -> 26.8 us, float64 57.3 -> 48.3, 192^3 115 -> 105 and 174 -> 167.
+// From one lattice into another (the form before): 40.3, 65.1, 126.6, 206.5;
+// 96^3 float64 27.1 -> 16.2, float32 11.8 -> 10.7, 64^3 unchanged within 5 %.
+// A grid of one wave whose threads overlap the next voxel's loads with this
+// one's collision (two cp.async stages) was slower beyond the L2 (192^3 122).
+template <class L, class M, Far F, bool ODD, bool CHECK>
 __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
     lb_step_kernel(typename M::S* __restrict__ f, FlowMap fm, Grid g, LbParams kc,
                    const FlowCtrl* __restrict__ ctrl, int kstep, double* __restrict__ partials,
                    int late) {
     if (!late) griddep_launch_dependents();
-    const int k = blockIdx.x * kFlowThreads + threadIdx.x;
-    const Lat<typename M::S> lat = lattices<L>(f, fm.nf, ODD);
-    // the pore maps never change during a solve: the pulls (with tables) or
-    // the upstream slots (without) are looked up while the previous
-    // iteration may still be running
-    int off[L::Q], src[L::Q];
-    if (k < fm.nf) {
-        if (fm.nbr) pull_offsets_table<L>(fm, lat, k, off);
-        else upstream_slots<L>(fm, g, k, src);
-    }
+    const int b = ODD ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const int k = b * kFlowThreads + threadIdx.x;
+    const Lat<typename M::S> lat = lattice<L>(f, fm.rs, ODD);
+    // the pore maps never change during a solve: the far places are looked
+    // up while the previous iteration may still be running
+    int far[L::NP];
+    far_slots<L, F>(fm, g, k, far);
     griddep_wait();
     const long long it = ctrl->it_base + kstep;
     if (ctrl->done || it >= ctrl->nit) return;  // uniform over the grid
     double acc = 0.0;
     if (k < fm.nf) {
-        if (!fm.nbr) pull_offsets<L>(lat, k, src, off);
-        const double ux = lb_cell_offs<L, M>(lat, kc, k, off);
+        const double ux = lb_cell<L, M>(lat, kc, k, far);
         if (CHECK) acc = ux;
     }
-    if (CHECK) block_sum_store(acc, partials + blockIdx.x);
+    if (CHECK) block_sum_store(acc, partials + b);
     if (late) griddep_launch_dependents();
 }
 
@@ -94,7 +104,9 @@ __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
     using R = typename M::R;
     using RA = typename M::RA;
     const int kk = blockIdx.x * kFlowThreads + threadIdx.x;
-    const Lat<S> lat = lattices<L>(const_cast<S*>(f), fm.nf, ODD);
+    const Lat<S> lat = lattice<L>(const_cast<S*>(f), fm.rs, ODD);
+    int far[L::NP];
+    far_slots<L, Far::packed>(fm, g, kk, far);
     double sux = 0.0, srho = 0.0, ssp = 0.0, mx = 0.0, nonf = 0.0;
     if (kk < fm.nf) {
         // solid voxels of vel were zeroed before this launch
@@ -104,7 +116,7 @@ __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
         float vx = 0.f, vy = 0.f, vz = 0.f;
         {
             typename Pop<S>::H h[L::Q];
-            gather<L, S>(lat, kk, fm, g, k.inv_scale, h);
+            gather<L, S>(lat, kk, far, k.inv_scale, h);
             const Moments<R, RA> m = moments<L, R, RA>(h, k.half_g);
             const RA ux = m.jx * m.inv_rho, uy = m.jy * m.inv_rho, uz = m.jz * m.inv_rho;
             vx = (float)ux;
@@ -207,23 +219,102 @@ __global__ void imap_scatter_kernel(int* __restrict__ cells, int nf, int* __rest
     cells[k] = (int)(((unsigned)x << xs) | ((unsigned)y << ys) | (unsigned)z);
 }
 
-// The pull tables: for each parity p of the read lattice, nbr[p * (Q - 1) *
-// nf + (i - 1) * nf + k] = the element offset slot k pulls direction i from.
+// Links per warp of 32 slots and pair: cnt[p * nw + w] (nw warps).
+template <class L>
+__global__ void link_count_kernel(FlowMap fm, Grid g, int* __restrict__ cnt) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nw = (fm.nf + 31) >> 5;
+    int x = 0, y = 0, z = 0;
+    if (k < fm.nf) unpack_cell((unsigned)fm.cells[k], fm, x, y, z);
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        const int i = L::pa(p);
+        int xx = x + L::c(i, 0), yy = y + L::c(i, 1), zz = z + L::c(i, 2);
+        xx = xx < 0 ? g.nx - 1 : (xx == g.nx ? 0 : xx);
+        yy = yy < 0 ? g.ny - 1 : (yy == g.ny ? 0 : yy);
+        zz = zz < 0 ? g.nz - 1 : (zz == g.nz ? 0 : zz);
+        const bool rock = k < fm.nf && fm.imap[(xx * g.ny + yy) * g.nz + zz] < 0;
+        const unsigned links = __ballot_sync(0xffffffffu, rock);
+        if ((threadIdx.x & 31) == 0 && k < fm.nf) cnt[p * nw + (k >> 5)] = __popc(links);
+    }
+}
+
+// Each pair's counts to the rank of every warp's first link (exclusive sums,
+// in place), and the pair's total to total[p]; one block per pair.
+__global__ void __launch_bounds__(1024) link_scan_kernel(int* __restrict__ cnt, int nw,
+                                                         int* __restrict__ total) {
+    __shared__ int warp_sum[32];
+    int* c = cnt + (long long)blockIdx.x * nw;
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int at = 0; at < nw; at += 1024) {
+        const int i = at + threadIdx.x;
+        const int v = i < nw ? c[i] : 0;
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        if (lane == 31) warp_sum[w] = s;
+        __syncthreads();
+        int ws = warp_sum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, ws, o);
+            if (lane >= o) ws += t;
+        }
+        const int before = w ? __shfl_sync(0xffffffffu, ws, w - 1) : 0;
+        if (i < nw) c[i] = carry + before + s - v;
+        carry += __shfl_sync(0xffffffffu, ws, 31);
+        __syncthreads();
+    }
+    if (threadIdx.x == 0) total[blockIdx.x] = carry;
+}
+
+// The packed table of far places (see FlowMap), one thread per slot.
+template <class L>
+__global__ void pack_fill_kernel(FlowMap fm, Grid g, unsigned* __restrict__ nbr) {
+    const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    const int nfp = (fm.nf + 31) / 32 * 32;
+    if (k >= nfp) return;  // whole warps
+    int far[L::NP];
+    far_slots_map<L>(fm, g, k, far);
+    const bool live = k < fm.nf;
+    const int lane = threadIdx.x & 31;
+    constexpr int words = Packed<L>::words;
+    unsigned w[words] = {};
+    int mine = 0;  // this lane's share of the bases
+    bool fits = true;
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        const bool link = live && far[p] >= fm.nf;
+        const int lo = __reduce_min_sync(0xffffffffu, live && !link ? far[p] : 0x7fffffff);
+        const int hi = __reduce_max_sync(0xffffffffu, live && !link ? far[p] : -1);
+        const int lbase = fm.nf + fm.link[p * (nfp / 32) + (k >> 5)];
+        if (hi >= 0 && hi - lo > 255) fits = false;
+        const int base = hi >= 0 ? lo : 0;
+        if (lane == p) mine = base;
+        if (lane == L::NP + p) mine = lbase;
+        const unsigned d = live ? (unsigned)(far[p] - (link ? lbase : base)) & 0xffu : 0u;
+        w[p / 4] |= d << (8 * (p % 4));
+        if (link) w[words - 1] |= 1u << (8 + p);
+    }
+    if (!fits) w[words - 1] |= 1u << 31;  // uniform over the warp
+    reinterpret_cast<uint2*>(nbr)[k] = make_uint2(w[0], w[1]);
+    if (words > 2) nbr[2 * nfp + k] = w[words - 1];
+    if (lane < 2 * L::NP) nbr[words * nfp + (k >> 5) * (2 * L::NP) + lane] = (unsigned)mine;
+}
+
+// The plain table of far places: nbr[p * nf + k].
 template <class L>
 __global__ void nbr_fill_kernel(FlowMap fm, Grid g, int* __restrict__ nbr) {
     const int k = blockIdx.x * blockDim.x + threadIdx.x;
+    int far[L::NP];
+    far_slots_map<L>(fm, g, k, far);
     if (k >= fm.nf) return;
-    int src[L::Q];
-    upstream_slots<L>(fm, g, k, src);
 #pragma unroll
-    for (int p = 0; p < 2; ++p) {
-        const Lat<char> lat = lattices<L, char>(nullptr, fm.nf, p != 0);
-        int off[L::Q];
-        pull_offsets<L, char>(lat, k, src, off);
-        int* tab = nbr + p * (L::Q - 1) * fm.nf;
-#pragma unroll
-        for (int i = 1; i < L::Q; ++i) tab[(i - 1) * fm.nf + k] = off[i];
-    }
+    for (int p = 0; p < L::NP; ++p) nbr[p * fm.nf + k] = far[p];
 }
 
 // -------------------------------------------------------------------------
@@ -232,20 +323,35 @@ __global__ void nbr_fill_kernel(FlowMap fm, Grid g, int* __restrict__ nbr) {
 int flow_blocks(long long n) { return (int)((n + kFlowThreads - 1) / kFlowThreads); }
 
 // Step kernels go out with programmatic stream serialisation (pdl_enabled,
-// lb_core.cuh): kernel t+1 starts launching while kernel t drains, reads its
-// upstream slots (the maps do not change during a solve) and waits in
+// lb_core.cuh): kernel t+1 starts launching while kernel t drains, finds its
+// far places (the maps do not change during a solve) and waits in
 // griddepcontrol.wait for t's results.  Measured on the B200 with 128-thread
 // blocks: 64^3 float32 4.89 -> 4.82 us per iteration, float16 4.43 -> 4.18,
 // 128^3 float32 41.3 -> 40.6.  A grid of one resident wave releases the
 // next step only after its stores (pdl_late): 64^3 float32 collision
 // 4.60 -> 4.09 us.
 
+// Blocks of `kern` the device holds at once.
+template <class K>
+static long long resident_blocks(K kern) {
+    int per_sm = 0, dev = 0, sms = 0;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFlowThreads, 0) !=
+            cudaSuccess ||
+        cudaGetDevice(&dev) != cudaSuccess ||
+        cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
+        cudaGetLastError();
+        return 0;
+    }
+    return (long long)per_sm * sms;
+}
+
 template <class L, class M, bool ODD, bool CHECK>
 static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Grid& g,
                                    const LbParams& k, const FlowCtrl* ctrl, int kstep,
                                    double* partials, cudaStream_t s) {
+    const int nb = flow_blocks(fm.nf);
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(flow_blocks(fm.nf));
+    cfg.gridDim = dim3(nb);
     cfg.blockDim = dim3(kFlowThreads);
     cfg.dynamicSmemBytes = 0;
     cfg.stream = s;
@@ -254,20 +360,12 @@ static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Gr
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    auto kern = lb_step_kernel<L, M, ODD, CHECK>;
-    static const long long resident = [&] {
-        int per_sm = 0, dev = 0, sms = 0;
-        if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFlowThreads, 0) !=
-                cudaSuccess ||
-            cudaGetDevice(&dev) != cudaSuccess ||
-            cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
-            cudaGetLastError();
-            return 0ll;
-        }
-        return (long long)per_sm * sms;
-    }();
-    const int late = pdl_late(flow_blocks(fm.nf) <= resident) ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, f, fm, g, k, ctrl, kstep, partials, late);
+    auto kern = fm.nbr ? lb_step_kernel<L, M, Far::table, ODD, CHECK>
+                       : lb_step_kernel<L, M, Far::packed, ODD, CHECK>;
+    // both forms are held to the same register budget
+    static const long long resident = resident_blocks(kern);
+    return cudaLaunchKernelEx(&cfg, kern, f, fm, g, k, ctrl, kstep, partials,
+                              pdl_late(nb <= resident) ? 1 : 0);
 }
 
 template <class L, class M>
@@ -335,11 +433,31 @@ cudaError_t flow_launch_imap(int* cells, int nf, int* imap, const Grid& g, int y
     return cudaGetLastError();
 }
 
+cudaError_t flow_launch_links(int nd, const FlowMap& fm, const Grid& g, int* link, int* total,
+                              cudaStream_t s) {
+    if (fm.nf <= 0) return cudaMemsetAsync(total, 0, 9 * sizeof(int), s);
+    const unsigned nb = (unsigned)((fm.nf + 255) / 256);
+    const int nw = (fm.nf + 31) / 32;
+    if (nd == 3) link_count_kernel<D3Q19><<<nb, 256, 0, s>>>(fm, g, link);
+    else link_count_kernel<D2Q9><<<nb, 256, 0, s>>>(fm, g, link);
+    link_scan_kernel<<<nd == 3 ? D3Q19::NP : D2Q9::NP, 1024, 0, s>>>(link, nw, total);
+    return cudaGetLastError();
+}
+
 cudaError_t flow_launch_nbr(int nd, const FlowMap& fm, const Grid& g, int* nbr, cudaStream_t s) {
     if (fm.nf <= 0) return cudaSuccess;
     const unsigned nb = (unsigned)((fm.nf + 255) / 256);
     if (nd == 3) nbr_fill_kernel<D3Q19><<<nb, 256, 0, s>>>(fm, g, nbr);
     else nbr_fill_kernel<D2Q9><<<nb, 256, 0, s>>>(fm, g, nbr);
+    return cudaGetLastError();
+}
+
+cudaError_t flow_launch_pack(int nd, const FlowMap& fm, const Grid& g, int* pack, cudaStream_t s) {
+    if (fm.nf <= 0) return cudaSuccess;
+    const unsigned nb = (unsigned)((fm.nf + 255) / 256);
+    unsigned* out = reinterpret_cast<unsigned*>(pack);
+    if (nd == 3) pack_fill_kernel<D3Q19><<<nb, 256, 0, s>>>(fm, g, out);
+    else pack_fill_kernel<D2Q9><<<nb, 256, 0, s>>>(fm, g, out);
     return cudaGetLastError();
 }
 
@@ -349,6 +467,13 @@ cudaError_t flow_launch_final_reduce(const double* partials, int nb, double* out
 }
 
 // compile-time checks of the lattice tables
+template <class L>
+constexpr bool pairs_evenly_spaced() {
+    for (int p = 0; p < L::NP; ++p)
+        if (L::pb(p) - L::pa(p) != L::pb(0) - L::pa(0) || L::opp(L::pa(p)) != L::pb(p)) return false;
+    return true;
+}
+static_assert(pairs_evenly_spaced<D3Q19>() && pairs_evenly_spaced<D2Q9>(), "Lat's row offsets");
 static_assert(D3Q19::opp(7) == 8 && D3Q19::opp(18) == 17, "D3Q19 opposites");
 static_assert(D3Q19::c(13, 0) == 1 && D3Q19::c(13, 2) == -1, "D3Q19 e_13");
 static_assert(D3Q19::c(18, 1) == -1 && D3Q19::c(18, 2) == 1, "D3Q19 e_18");

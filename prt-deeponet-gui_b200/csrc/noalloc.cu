@@ -6,7 +6,7 @@
 // plug-in hosts that hand out device buffers for inputs and outputs but no
 // allocator.  They pass the material grid and the velocity output as device
 // pointers they already own, plus a stream; every other byte the solve needs
-// (both population lattices, the neighbour masks, the per-block partial sums
+// (the population lattice, the pore maps, the per-block partial sums
 // and the control block) lives in one file-scope __device__ array compiled
 // into the library.
 //
@@ -98,9 +98,13 @@ int noalloc_solve(const uint8_t* d_mat, const prt_flow_params* p, float* d_vel_o
         return fail(PRT_E_INVALID, "grid too large");
     const int Q = p->nd == 3 ? 19 : 9;
     const size_t es = p->precision == PRT_FP64 ? 8 : (p->precision == PRT_FP16 ? 2 : 4);
-    // scratch layout, sized for the worst case (every voxel pore):
-    // control | count | 5 reduced sums | block counts | partials | flags |
-    // pore list | voxel -> slot map | 2 lattices
+    // scratch layout, sized for any pore count: control | counts | 5 reduced
+    // sums | block counts | partials | flags | pore list | voxel -> slot map |
+    // link numbers | packed table | lattice.  A lattice row has at most n
+    // elements and its padding (a direction has at most n - nf links), and
+    // the other two take less than another Q n es, so they fit in the 2 Q n
+    // es bytes that a grid is admitted by (small grids, where the padding
+    // counts, are far below the limit).
     const int nb_max = flow_blocks(g.n);
     const size_t o_ctrl = 0;
     const size_t o_count = o_ctrl + up256(sizeof(FlowCtrl));
@@ -129,7 +133,6 @@ int noalloc_solve(const uint8_t* d_mat, const prt_flow_params* p, float* d_vel_o
     uint8_t* flag = sb + o_flag;
     int* cells = reinterpret_cast<int*>(sb + o_cells);
     int* imap = reinterpret_cast<int*>(sb + o_imap);
-    void* f = sb + o_lat;
 
     float scale = 1.f;
     if (p->precision == PRT_FP16) {
@@ -159,9 +162,28 @@ int noalloc_solve(const uint8_t* d_mat, const prt_flow_params* p, float* d_vel_o
     fm.nf = (int)nfluid;
     fm.cells = cells;
     fm.imap = imap;
+    fm.link = nullptr;
     fm.nbr = nullptr;
+    fm.pack = nullptr;
+    fm.rs = 0;
+    int* link = reinterpret_cast<int*>(sb + o_lat);
+    int* d_links = reinterpret_cast<int*>(sb + o_count + 64);  // links per pair
+    NCK(flow_launch_links(p->nd, fm, g, link, d_links, s));
+    int links[9] = {0};
+    NCK(cudaMemcpyAsync(links, d_links, (size_t)flow_pairs(Q) * 4, cudaMemcpyDeviceToHost, s));
+    NCK(cudaStreamSynchronize(s));
+    fm.link = link;
+    fm.rs = flow_row(nfluid, *std::max_element(links, links + 9));
+    const size_t o_pack = o_lat + up256((size_t)flow_link_ints(Q, nfluid) * 4);
+    const size_t o_rows = o_pack + up256((size_t)flow_pack_bytes(Q, nfluid));
+    const size_t lattice_bytes = (size_t)Q * fm.rs * es;
+    if (o_rows + lattice_bytes > kNoAllocScratchBytes)
+        return fail(PRT_E_INVALID, "the lattice exceeds the allocation-free solve's scratch");
+    NCK(flow_launch_pack(p->nd, fm, g, reinterpret_cast<int*>(sb + o_pack), s));
+    fm.pack = reinterpret_cast<int*>(sb + o_pack);
+    void* f = sb + o_rows;
     const int nb = std::max(flow_blocks(nfluid), 1);
-    NCK(cudaMemsetAsync(f, 0, (size_t)2 * Q * nfluid * es, s));
+    NCK(cudaMemsetAsync(f, 0, lattice_bytes, s));
     NCK(cudaMemsetAsync(d_vel_out, 0, (size_t)3 * g.n * sizeof(float), s));
     NCK(cudaMemsetAsync(parts, 0, (size_t)nb * 5 * sizeof(double), s));
     noalloc_ctrl_kernel<<<1, 1, 0, s>>>(ctrl, count, p->nit, p->tol, p->every);

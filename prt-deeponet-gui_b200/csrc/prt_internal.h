@@ -176,31 +176,55 @@ struct PairTree {
 // voxel in C order, whose coordinates are packed in cells[k] as
 // x << xs | y << ys | z (so a kernel finds its neighbours with shifts and
 // masks instead of divisions); imap[voxel] is the slot of a pore voxel, -1
-// for rock.  nbr, when not null, holds the pull tables, one per parity p of
-// the read lattice: nbr[p * (Q-1) * nf + (i - 1) * nf + k] = the element
-// offset (into the two lattices) slot k pulls direction i from -- the
-// upstream slot of the read lattice, or slot k's own opp(i) of the write
-// lattice when that voxel is rock (i = 1 .. Q-1).  The step kernel then
-// reads them in one coalesced pass instead of the packed cell, the imap
-// lookups and the choice between the two lattices.  Set up for solves whose
-// lattices and tables fit in half the L2 cache, where the latency of the
-// lookups, not the bytes of the tables, bounds an iteration.
+// for rock.  For each pair p of opposite directions (a, b) a slot whose
+// voxel x + e_a is rock has a link, numbered in slot order; link[p * nw + w]
+// is the number of the first link of the slots [32 w, 32 w + 32), nw =
+// ceil(nf / 32).  rs is the row stride of the lattice: nf slots and the links
+// of the pair with the most.
+// nbr, when not null, is the plain table of far places (nbr[p * nf + k]): the
+// slot of x + e_a or the link's own element (nf + number).
+// pack is the packed table of the same.  Per slot and pair one byte, the
+// distance from a base that the slot's warp shares -- the lowest far slot of
+// the warp, or the warp's first link -- and one bit that says which; per
+// warp and pair the two bases.  Words: D3Q19 [bytes 0-3, bytes 4-7] per
+// slot, then [byte 8, bits 8-16 the link bits] per slot, D2Q9 [bytes 0-3,
+// bits 8-11 the link bits] per slot; then 2 pairs bases per warp.  Bit 31 of
+// the last word: the warp's places span more than a byte (it crosses the end
+// of the grid, or a wide gap), it uses the maps instead.
 struct FlowMap {
     int nf;
     const int* cells;
     const int* imap;
     int ys, xs;  // bit offsets of y and x in a packed cell
     const int* nbr;
+    const int* pack;
+    const int* link;
+    unsigned rs;
 };
 
-// Bytes of the two pull tables of nf pore voxels (Q-1 ints each per parity).
-inline long long flow_nbr_bytes(int q, long long nf) { return 2ll * (q - 1) * nf * 4; }
+inline int flow_pairs(int q) { return (q - 1) / 2; }
 
-// Whether a solve with nf pore voxels and populations of es bytes gets the
-// pull tables on a device with l2_bytes of L2: when the two lattices and one
-// table (an iteration reads one) fit in half of it.
-inline bool flow_use_nbr(int q, long long nf, long long es, long long l2_bytes) {
-    return nf > 0 && 2 * q * nf * es + flow_nbr_bytes(q, nf) / 2 <= l2_bytes / 2;
+// Row stride for nf slots and at most `links` links a pair: rows start on
+// 64-element boundaries.
+inline unsigned flow_row(long long nf, long long links) {
+    return (unsigned)((nf + links + 63) / 64 * 64);
+}
+
+// Ints of the link numbers: one per pair and warp of slots.
+inline long long flow_link_ints(int q, long long nf) { return flow_pairs(q) * ((nf + 31) / 32); }
+
+// Bytes of the plain table of far places of nf pore voxels, and of the packed.
+inline long long flow_nbr_bytes(int q, long long nf) { return flow_pairs(q) * nf * 4; }
+inline long long flow_pack_bytes(int q, long long nf) {
+    const long long nw = (nf + 31) / 32;
+    return nw * (32 * (q > 9 ? 3 : 2) + 2 * flow_pairs(q)) * 4;
+}
+
+// Whether a solve with nf pore voxels, rows of rs elements and populations
+// of es bytes gets the plain table on a device with l2_bytes of L2: when the
+// lattice and the table fit in half of it.
+inline bool flow_use_nbr(int q, long long nf, long long rs, long long es, long long l2_bytes) {
+    return nf > 0 && q * rs * es + flow_nbr_bytes(q, nf) <= l2_bytes / 4 * 3;
 }
 
 // Constants of one flow solve (the TRT rates of _trt_minus and the Guo
@@ -252,9 +276,8 @@ __host__ __device__ inline void unpack_cell(unsigned cv, const FlowMap& fm, int&
 }
 
 // Kernel launchers (lb_flow.cu) ---------------------------------------------
-// Returns cudaSuccess or the launch error.  f holds the two lattices (read /
-// write swap with the iteration parity), Q * nf populations each.  Step and
-// moments launches have flow_blocks(nf) blocks (the partial-sum count).
+// Returns cudaSuccess or the launch error.  f holds the lattice, Q rows of
+// fm.rs populations.  Step and moments launches have flow_blocks(nf) blocks (the partial-sum count).
 cudaError_t flow_launch_step(int nd, int precision, bool odd, bool check, void* f,
                              const FlowMap& fm, const Grid& g, const LbParams& lbp,
                              const FlowCtrl* ctrl, int kstep, double* partials,
@@ -270,9 +293,15 @@ cudaError_t flow_launch_flags(const uint8_t* mat, long long n, int pore, uint8_t
 // packed coordinates of fm (imap must hold -1 everywhere before).
 cudaError_t flow_launch_imap(int* cells, int nf, int* imap, const Grid& g, int ys, int xs,
                              cudaStream_t s);
-// The pull tables of fm (cells and imap ready) into nbr,
+// The link numbers of fm (cells and imap ready) into link, flow_link_ints(Q,
+// fm.nf) ints, and the links of each pair into total (9 ints).
+cudaError_t flow_launch_links(int nd, const FlowMap& fm, const Grid& g, int* link, int* total,
+                              cudaStream_t s);
+// The table of far places of fm (cells, imap and link ready) into nbr,
 // flow_nbr_bytes(Q, fm.nf) bytes.
 cudaError_t flow_launch_nbr(int nd, const FlowMap& fm, const Grid& g, int* nbr, cudaStream_t s);
+// The packed table, flow_pack_bytes(Q, fm.nf) bytes.
+cudaError_t flow_launch_pack(int nd, const FlowMap& fm, const Grid& g, int* pack, cudaStream_t s);
 cudaError_t flow_launch_final_reduce(const double* partials, int nblocks, double* out,
                                      cudaStream_t s);
 int flow_blocks(long long n);

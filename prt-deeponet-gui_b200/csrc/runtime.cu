@@ -59,7 +59,7 @@ extern "C" void prt_destroy(prt_ctx* c) {
     c->prep.release();
     FlowState& f = c->flow;
     DevBuf* all[] = {&f.f,    &f.fluid, &f.partials, &f.ctrl, &f.out5, &f.count,
-                     &f.mat,  &f.vel,   &f.flag,     &f.cnt,  &f.cells, &f.nbr};
+                     &f.mat,  &f.vel,   &f.flag,     &f.cnt,  &f.cells, &f.nbr, &f.link, &f.pack};
     for (DevBuf* b : all) b->release();
     f.graph.release();
     for (int i = 0; i < 4; ++i)
@@ -102,15 +102,17 @@ extern "C" size_t prt_sizeof(int which) {
 // ===========================================================================
 // flow
 // ===========================================================================
-// The upstream-slot table: by the working set against the L2 cache
-// (flow_use_nbr), or always / never with PRT_NBR_TABLE=1 / 0.  Both ways
-// give the same slots, so the fields are bit-identical either way.
-static bool nbr_table_wanted(int q, long long nf, long long es, long long l2_bytes) {
+// The plain table of far places: by the working set against the L2 cache
+// (flow_use_nbr), or always / never with PRT_NBR_TABLE=1 / 0; a solve
+// without it has the packed table.  Both give the same places, so the fields
+// are bit-identical either way.
+static bool nbr_table_wanted(int q, long long nf, long long rs, long long es,
+                             long long l2_bytes) {
     if (nf <= 0) return false;
     const char* v = std::getenv("PRT_NBR_TABLE");
     if (v && v[0] == '1') return true;
     if (v && v[0] == '0') return false;
-    return flow_use_nbr(q, nf, es, l2_bytes);
+    return flow_use_nbr(q, nf, rs, es, l2_bytes);
 }
 
 // Flow solve in three parts, so the batched engine can run many set-up
@@ -167,21 +169,38 @@ int prt::flow_setup(prt_ctx* ctx, const uint8_t* d_mat, const prt_flow_params* p
     F.fm.cells = F.cells.as<int>();
     F.fm.imap = F.fluid.as<int>();
     F.fm.nbr = nullptr;
-    if (nbr_table_wanted(Q, nfluid, (long long)es, ctx->l2_bytes)) {
+    CK(F.link.ensure((size_t)(std::max(flow_link_ints(Q, nfluid), 1ll) + 9) * 4));
+    int* d_links = F.link.as<int>() + flow_link_ints(Q, nfluid);  // per pair
+    CK(flow_launch_links(p->nd, F.fm, g, F.link.as<int>(), d_links, s));
+    ctx->launches += 2;
+    int links[9] = {0};
+    CK(cudaMemcpyAsync(links, d_links, (size_t)flow_pairs(Q) * 4, cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    F.fm.link = F.link.as<int>();
+    F.fm.rs = flow_row(nfluid, *std::max_element(links, links + 9));
+    F.fm.pack = nullptr;
+    if (nfluid > 0) {
+        CK(F.pack.ensure((size_t)flow_pack_bytes(Q, nfluid)));
+        CK(flow_launch_pack(p->nd, F.fm, g, F.pack.as<int>(), s));
+        ctx->launches += 1;
+        F.fm.pack = F.pack.as<int>();
+    }
+    if (nbr_table_wanted(Q, nfluid, F.fm.rs, (long long)es, ctx->l2_bytes)) {
         CK(F.nbr.ensure((size_t)flow_nbr_bytes(Q, nfluid)));
         CK(flow_launch_nbr(p->nd, F.fm, g, F.nbr.as<int>(), s));
         ctx->launches += 1;
         F.fm.nbr = F.nbr.as<int>();
     }
     F.nb = std::max(flow_blocks(nfluid), 1);
-    CK(F.f.ensure((size_t)2 * Q * std::max(nfluid, 1ll) * es));  // two lattices
+    const size_t lattice_bytes = (size_t)Q * F.fm.rs * es;
+    CK(F.f.ensure(std::max(lattice_bytes, (size_t)1)));
     CK(F.partials.ensure((size_t)F.nb * 5 * sizeof(double)));
     CK(F.ctrl.ensure(sizeof(FlowCtrl)));
     CK(F.out5.ensure(8 * sizeof(double)));
 
-    // f = w_i everywhere, in both lattices: shifted storage h = 0; rock
-    // voxels of the output velocity are 0
-    CK(cudaMemsetAsync(F.f.p, 0, (size_t)2 * Q * nfluid * es, s));
+    // f = w_i everywhere: shifted storage h = 0; rock voxels of the output
+    // velocity are 0
+    CK(cudaMemsetAsync(F.f.p, 0, lattice_bytes, s));
     CK(cudaMemsetAsync(d_vel, 0, (size_t)3 * g.n * sizeof(float), s));
     CK(cudaMemsetAsync(F.partials.p, 0, (size_t)F.nb * 5 * sizeof(double), s));
     FlowCtrl hc{};
@@ -270,7 +289,8 @@ static int flow_graph(prt_ctx* ctx) {
     key.force = p.force; key.tau = p.tau; key.magic = p.magic; key.nit = p.nit;
     key.tol = p.tol; key.f = F.f.p;
     key.aux[0] = F.fluid.p; key.aux[1] = F.partials.p; key.aux[2] = F.ctrl.p;
-    key.aux[3] = F.cells.p; key.aux[4] = (void*)F.fm.nbr; key.nf = F.nfluid;
+    key.aux[3] = F.cells.p; key.aux[4] = (void*)F.fm.nbr; key.aux[5] = F.link.p; key.aux[6] = F.pack.p;
+    key.nf = F.nfluid; key.rs = F.fm.rs;
     key.pdl = pdl_key();
     if (!F.graph.exec || !(key == F.key)) {
         CK(build_while_graph(ctx->stream,

@@ -62,26 +62,28 @@ struct FlowKey {
     long long nit = -1;
     double tol = 0;
     void* f = nullptr;
-    void* aux[5] = {nullptr, nullptr, nullptr, nullptr, nullptr};
-    long long nf = -1;  // pore voxels: launch sizes and the lattice stride are baked in
+    void* aux[7] = {nullptr, nullptr, nullptr, nullptr, nullptr, nullptr, nullptr};
+    long long nf = -1;  // pore voxels (launch sizes) and the lattice row stride are baked in
+    unsigned rs = 0;
     int pdl = 0;        // the launch settings the step kernels were captured with (pdl_key)
     bool operator==(const FlowKey& o) const {
         return nd == o.nd && precision == o.precision && every == o.every && g.nx == o.g.nx &&
                g.ny == o.g.ny && g.nz == o.g.nz && force == o.force && tau == o.tau &&
                magic == o.magic && nit == o.nit && tol == o.tol && f == o.f && aux[0] == o.aux[0] &&
                aux[1] == o.aux[1] && aux[2] == o.aux[2] && aux[3] == o.aux[3] &&
-               aux[4] == o.aux[4] && nf == o.nf && pdl == o.pdl;
+               aux[4] == o.aux[4] && aux[5] == o.aux[5] && aux[6] == o.aux[6] && nf == o.nf && rs == o.rs &&
+               pdl == o.pdl;
     }
 };
 
 struct FlowState {
-    DevBuf f, fluid, partials, ctrl, out5, count, mat, vel, flag, cnt, cells, nbr;
+    DevBuf f, fluid, partials, ctrl, out5, count, mat, vel, flag, cnt, cells, nbr, link, pack;
     GraphHolder graph;
     FlowKey key;
     // the solve set up by flow_setup
     prt_flow_params p{};
     Grid g{0, 0, 0, 0};
-    FlowMap fm{0, nullptr, nullptr, 0, 0, nullptr};
+    FlowMap fm{0, nullptr, nullptr, 0, 0, nullptr, nullptr, nullptr, 0};
     LbParams kc{};
     int nb = 1;
     long long nfluid = 0;
@@ -90,7 +92,7 @@ struct FlowState {
     float* d_vel = nullptr;          // its output field (borrowed)
     bool field_ready = false;        // d_vel holds the final field
     void release_lattices() {
-        DevBuf* all[] = {&f, &fluid, &partials, &count, &flag, &cnt, &cells, &nbr};
+        DevBuf* all[] = {&f, &fluid, &partials, &count, &flag, &cnt, &cells, &nbr, &link, &pack};
         for (DevBuf* b : all) b->release();
         graph.release();
         key = FlowKey();

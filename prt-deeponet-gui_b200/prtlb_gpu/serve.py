@@ -34,8 +34,8 @@ def ladder_slots(limit, ratio):
 
 
 def footprint(req):
-    """Estimated peak device bytes of one request: the flow phase (two
-    lattices, maps) or the transport phase (state, faces, snapshot ladder),
+    """Estimated peak device bytes of one request: the flow phase (the
+    lattice, maps and tables) or the transport phase (state, faces, snapshot ladder),
     whichever is larger, plus the material grid and field kept by both."""
     mat = req.mat
     n = int(mat.size)
@@ -44,11 +44,14 @@ def footprint(req):
     q = 19 if nd == 3 else 9
     es = {"fp64": 8, "fp32": 4, "fp32f": 4, "fp16": 2}[req.flow["precision"]]
     common = n * (1 + 12)
-    flow = 2 * q * nf * es + 4 * nf + 4 * n + n + 5 * 8 * (nf // 256 + 1)
-    # the upstream-slot table of solves that fit in half the L2 cache,
+    # lattice rows hold the pore voxels and the rock links of one direction:
+    # no more than the pore voxels again, nor than the rock voxels
+    rows = min(2 * nf, n) + 64
+    flow = q * rows * es + (4 + 16) * nf + 4 * n + n + 5 * 8 * (nf // 128 + 1)
+    # the plain table of solves that fit in three quarters of the L2 cache,
     # counted up to an L2 of 256 MiB (an upper bound of the devices run on)
-    table = 4 * (q - 1) * nf
-    if 2 * q * nf * es + table <= (128 << 20):
+    table = 2 * (q - 1) * nf
+    if q * nf * es + table <= (192 << 20):
         flow += table
     adr = 0
     if req.adr is not None:

@@ -19,26 +19,29 @@ namespace prt {
 constexpr int kAdrThreads = 128;
 
 // One transport step n = n_base + kstep + 1 over every solute voxel (one
-// thread each; rock voxels are never touched and stay 0 in every buffer).
+// thread each; rock voxels are not in the state).
 // Launched with programmatic stream serialisation: what does not change
-// during a run (the voxel's index, flags, position and face velocities) is
-// read while the previous step drains; the control block and the
-// concentrations only after griddepcontrol.wait.
+// during a run (the neighbours' places and the face velocities) is read while
+// the previous step drains; the control block and the concentrations only
+// after griddepcontrol.wait.
 // late: the next step is let in after this one's stores (see pdl_late).
-template <int ND, int NS, bool BF>
+template <int ND, int NS, bool BF, bool WIDE>
 __global__ void __launch_bounds__(kAdrThreads) adr_step_kernel(AdrDev d, prt_adr_params p,
                                                                const AdrCtrl* __restrict__ ctrl,
                                                                int kstep, int late) {
     if (!late) griddep_launch_dependents();
-    const long long kk = (long long)blockIdx.x * kAdrThreads + threadIdx.x;
-    const bool live = kk < d.nm;
-    VoxelSetup s;
-    if (live) s = voxel_setup<ND>(d, kk);
+    // every other step walks the voxels downwards: it starts on what the step
+    // before left in the L2
+    const unsigned b = (kstep & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const unsigned k = b * kAdrThreads + threadIdx.x;
+    const bool live = k < (unsigned)d.nm;
+    VoxelSetup<ND> s;
+    if (live) s = voxel_setup<ND, BF, WIDE>(d, p, k);
     griddep_wait();
     const long long n = ctrl->n_base + kstep + 1;
     if (ctrl->done || n > ctrl->limit) return;  // uniform over the grid
     if (!live) return;
-    adr_voxel_step<ND, NS, BF>(d, p, n, s);
+    adr_voxel_step<ND, NS, BF>(d, p, n, k, s);
     if (late) griddep_launch_dependents();
 }
 
@@ -87,56 +90,124 @@ __global__ void adr_flags_kernel(const uint8_t* __restrict__ mat, Grid g, int nd
     mflag[c] = m ? 1 : 0;
 }
 
-// Face velocities u_f = 1/2 (u_lo + u_hi) on open faces, 0 on closed ones,
-// from u = vel / u_scale (float32 division) masked to the solute voxels
-// (prtlb_3d.py:860-865, 1092-1135).  Face f of axis a lies between voxels
-// clamp(f-1) and clamp(f); faces 0 and n_a are the domain faces.
-__global__ void adr_faces_kernel(const uint8_t* __restrict__ mat, const float* __restrict__ vcomp,
-                                 Grid g, int a, int pore, int bfc, float u_scale,
-                                 float* __restrict__ face) {
-    const int fa = extent(g, a) + 1;
-    const long long nf = g.n / extent(g, a) * fa;
-    const long long t = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (t >= nf) return;
-    int q[3];
-    const int dims[3] = {a == 0 ? fa : g.nx, a == 1 ? fa : g.ny, a == 2 ? fa : g.nz};
-    unsigned long long r = (unsigned long long)t;
-    q[2] = (int)(r % (unsigned)dims[2]);
-    r /= (unsigned)dims[2];
-    q[1] = (int)(r % (unsigned)dims[1]);
-    q[0] = (int)(r / (unsigned)dims[1]);
-    const int f = q[a];
-    const int n = extent(g, a);
-    const int plo = f - 1 < 0 ? 0 : f - 1;
-    const int phi = f > n - 1 ? n - 1 : f;
-    int ql[3] = {q[0], q[1], q[2]}, qh[3] = {q[0], q[1], q[2]};
-    ql[a] = plo;
-    qh[a] = phi;
-    const long long cl = ((long long)ql[0] * g.ny + ql[1]) * g.nz + ql[2];
-    const long long ch = ((long long)qh[0] * g.ny + qh[1]) * g.nz + qh[2];
-    const bool ml = is_m(mat, cl, pore, bfc), mh = is_m(mat, ch, pore, bfc);
-    float u = 0.f;
-    if (ml && mh) {
-        const float ul = vcomp[cl] / u_scale;
-        const float uh = vcomp[ch] / u_scale;
-        u = 0.5f * (ul + uh);
-    }
-    face[t] = u;
+// map[idx[k]] = k.
+__global__ void adr_map_kernel(const int* __restrict__ idx, long long nm, int* __restrict__ map) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k < nm) map[idx[k]] = (int)k;
 }
 
-// Initial state (initial(), prtlb_3d.py:1425-1440) into buffer 0 and slot 0.
-__global__ void adr_init_kernel(const uint32_t* __restrict__ flags, Grid g, prt_adr_params p,
-                                float* __restrict__ buf0, float* __restrict__ slot0) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= g.n) return;
-    const uint32_t fl = flags[c];
+// The neighbours of solute voxel k along axis i as AdrDev has them (far low,
+// low, high, far high), from the open / far flags at clamped positions.
+__device__ __forceinline__ int4 neighbours(const AdrDev& d, const int* __restrict__ map, int k,
+                                           int i, uint32_t fl, const VoxelPos& v) {
+    const int a = (d.nd == 3) ? i : (i == 0 ? 0 : 2);
+    const int p = v.p[a], n = extent(d.g, a), s = stride(d.g, a), c = v.c;
+    const int pm1 = p > 0 ? 1 : 0, pm2 = p > 1 ? 2 : pm1;
+    const int pp1 = p < n - 1 ? 1 : 0, pp2 = p < n - 2 ? 2 : pp1;
+    int4 q;
+    q.y = (fl & f_open_lo(a)) ? map[c - pm1 * s] : k;
+    q.z = (fl & f_open_hi(a)) ? map[c + pp1 * s] : k;
+    q.x = (fl & f_far_lo(a)) ? map[c - pm2 * s] : q.y;
+    q.w = (fl & f_far_hi(a)) ? map[c + pp2 * s] : q.z;
+    return q;
+}
+
+// *reach = the largest distance between a voxel and its neighbours.
+__global__ void adr_reach_kernel(AdrDev d, const int* __restrict__ map, unsigned* reach) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    unsigned far = 0;
+    if (k < d.nm) {
+        const int c = d.idx[k];
+        const VoxelPos v = voxel_pos(c, d.g);
+        for (int i = 0; i < d.nd; ++i) {
+            const int4 q = neighbours(d, map, (int)k, i, d.flags[c], v);
+            far = max(far, (unsigned)max((int)k - q.x, q.w - (int)k));
+        }
+    }
+    far = __reduce_max_sync(0xffffffffu, far);
+    if ((threadIdx.x & 31) == 0 && far) atomicMax(reach, far);
+}
+
+// The run's fixed data of each solute voxel.  Face velocities u_f = 1/2 (u_lo +
+// u_hi) on open faces, 0 on closed ones, from u = vel / u_scale (float32
+// division) at the clamped positions of the face's two voxels
+// (prtlb_3d.py:860-865, 1092-1135).
+__global__ void adr_tables_kernel(const float* __restrict__ vel, AdrDev d, float u_scale,
+                                  const int* __restrict__ map, uint2* __restrict__ near,
+                                  int4* __restrict__ nb, float2* __restrict__ face,
+                                  uint32_t* __restrict__ cflags) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.nm) return;
+    const Grid& g = d.g;
+    const int c = d.idx[k];
+    const uint32_t fl = d.flags[c];
+    cflags[k] = fl;
+    const VoxelPos v = voxel_pos(c, g);
+    for (int i = 0; i < d.nd; ++i) {
+        const int a = (d.nd == 3) ? i : (i == 0 ? 0 : 2);
+        const long long at = (long long)i * d.nm + k;
+        const int4 q = neighbours(d, map, (int)k, i, fl, v);
+        if (near) {
+            const unsigned u = (unsigned)k;
+            near[at] = make_uint2((u - (unsigned)q.x) | ((u - (unsigned)q.y) << 16),
+                                  ((unsigned)q.z - u) | (((unsigned)q.w - u) << 16));
+        } else {
+            nb[at] = q;
+        }
+        // velocity component of storage axis a: 3D -> a; 2D -> x: 0, y (stored as z): 1
+        const float* vc = vel + (long long)((d.nd == 3) ? a : (a == 0 ? 0 : 1)) * g.n;
+        const int s = stride(g, a);
+        const float u = vc[c] / u_scale;
+        float2 f = make_float2(0.f, 0.f);
+        if (fl & f_open_lo(a)) f.x = 0.5f * (vc[v.p[a] > 0 ? c - s : c] / u_scale + u);
+        if (fl & f_open_hi(a))
+            f.y = 0.5f * (u + vc[v.p[a] < extent(g, a) - 1 ? c + s : c] / u_scale);
+        face[at] = f;
+    }
+}
+
+// Initial state (initial(), prtlb_3d.py:1425-1440) into buffer 0.
+__global__ void adr_init_kernel(AdrDev d, prt_adr_params p, float* __restrict__ buf0) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.nm) return;
+    const uint32_t fl = d.flags[d.idx[k]];
     for (int j = 0; j < p.ns; ++j) {
         float v = 0.f;
         if (p.init_mode[j] == 1 && (fl & F_M)) v = p.init_value[j];
         if (p.init_mode[j] == 2 && (fl & F_BF)) v = p.init_value[j];
-        buf0[(long long)j * g.n + c] = v;
-        if (slot0) slot0[(long long)j * g.n + c] = v;
+        float* row = buf0 + (long long)j * d.ms;
+        row[solute_place((unsigned)k, (unsigned)d.n0, (unsigned)d.nm)] = v;
+        if (k < d.n0) row[k] = ((p.pinned_mask >> j) & 1u) ? p.feed[j] : v;
     }
+}
+
+// Ladder rows (stride nm) from the state's.
+__global__ void adr_rows_kernel(AdrDev d, const float* __restrict__ buf, float* __restrict__ rows) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= d.nm) return;
+    const unsigned at = solute_place((unsigned)k, (unsigned)d.n0, (unsigned)d.nm);
+    for (int j = 0; j < d.ns; ++j) rows[j * d.nm + k] = buf[(long long)j * d.ms + at];
+}
+
+// out[j * n + idx[k]] = rows[j * nm + k].
+__global__ void adr_expand_kernel(const float* __restrict__ rows, const int* __restrict__ idx,
+                                  long long nm, long long n, int ns, float* __restrict__ out) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nm) return;
+    const int c = idx[k];
+    for (int j = 0; j < ns; ++j) out[(long long)j * n + c] = rows[(long long)j * nm + k];
+}
+
+// *n0 = how many of the nm voxel indices lie below `plane` (they ascend).
+__global__ void adr_inlet_count_kernel(const int* __restrict__ idx, long long nm, int plane,
+                                       int* __restrict__ n0) {
+    long long lo = 0, hi = nm;
+    while (lo < hi) {
+        const long long mid = (lo + hi) / 2;
+        if (idx[mid] < plane) lo = mid + 1;
+        else hi = mid;
+    }
+    *n0 = (int)lo;
 }
 
 // Order-preserving compaction of the solute voxels (C order), in three passes.
@@ -175,71 +246,67 @@ __global__ void scatter_kernel(const uint8_t* __restrict__ mflag, long long n,
 
 // ---------------------------------------------------------------------------
 // numpy float32 pairwise means (the stop rule's `C[j][m].mean()`), per
-// species: leaf sums (leaf_sum) then the tree levels (tree_mean)
+// species: leaf sums (warp_leaf_sum) then the tree levels (tree_means)
 // ---------------------------------------------------------------------------
-__global__ void means_leaf_kernel(const float* __restrict__ src, long long N,
-                                  const int* __restrict__ idx, PairTree t, int ns,
-                                  float* __restrict__ vals) {
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= (long long)t.nleaf * ns) return;
-    const int leaf = (int)(tid % t.nleaf);
-    const int j = (int)(tid / t.nleaf);
-    vals[(long long)j * (t.nleaf + t.ninner) + leaf] = leaf_sum(src + (long long)j * N, idx, t, leaf);
+constexpr int kLeafThreads = 256;
+constexpr int kTreeThreads = 512;
+
+// One warp per leaf and chemical.
+__device__ __forceinline__ void block_of_leaves(const float* __restrict__ src, long long row,
+                                                unsigned n0, unsigned nm, const PairTree& t,
+                                                int ns, float* __restrict__ vals) {
+    __shared__ float sh[kLeafThreads / 32][128];
+    const int w = threadIdx.x >> 5;
+    const long long item = (long long)blockIdx.x * (kLeafThreads / 32) + w;
+    if (item >= (long long)t.nleaf * ns) return;  // whole warps
+    const int leaf = (int)(item % t.nleaf);
+    const int j = (int)(item / t.nleaf);
+    const float v = warp_leaf_sum(src + j * row, n0, nm, t.leaf_start[leaf], t.leaf_len[leaf], sh[w]);
+    if ((threadIdx.x & 31) == 0) vals[(long long)j * (t.nleaf + t.ninner) + leaf] = v;
 }
 
-__global__ void means_tree_kernel(PairTree t, long long nm, float* __restrict__ vals,
-                                  float* __restrict__ means) {
-    const int j = blockIdx.x;
-    tree_mean(t, nm, vals + (long long)j * (t.nleaf + t.ninner), means + j);
+__global__ void __launch_bounds__(kLeafThreads)
+    means_leaf_kernel(const float* __restrict__ src, long long row, long long nm, PairTree t, int ns,
+                      float* __restrict__ vals) {
+    block_of_leaves(src, row, 0u, (unsigned)nm, t, ns, vals);
 }
 
-__global__ void adr_stop_kernel(AdrCtrl* ctrl, const float* __restrict__ means, ProgressRec* log,
-                                int log_cap, cudaGraphConditionalHandle h, int use_handle) {
-    if (threadIdx.x != 0) return;
+__global__ void __launch_bounds__(kTreeThreads)
+    means_tree_kernel(PairTree t, long long nm, int ns, float* __restrict__ vals,
+                      float* __restrict__ means) {
+    tree_means(t, nm, ns, vals, means);
+}
+
+// The leaves of the state at the end of the current chunk, when its means are
+// due.
+__global__ void __launch_bounds__(kLeafThreads)
+    chunk_leaf_kernel(const AdrCtrl* __restrict__ ctrl, AdrDev d) {
+    if (ctrl->done) return;
+    const long long end = min(ctrl->n_base + (long long)ctrl->check, ctrl->limit);
+    if (end % ctrl->check != 0) return;
+    block_of_leaves(d.buf[end & 1], d.ms, (unsigned)d.n0, (unsigned)d.nm, d.tree, d.ns, d.tree_vals);
+}
+
+// The tree levels and means, where due, then the stop rule, the step count and
+// the while-graph's condition.
+__global__ void __launch_bounds__(kTreeThreads)
+    chunk_end_kernel(AdrCtrl* ctrl, AdrDev d, float* __restrict__ means,
+                     cudaGraphConditionalHandle h, int use_handle) {
     if (ctrl->done) {
-        if (use_handle) cudaGraphSetConditional(h, 0);
+        if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, 0);
         return;
     }
     const long long base = ctrl->n_base;
     const long long end = min(base + (long long)ctrl->check, ctrl->limit);
-    if (end > base && end % ctrl->check == 0) adr_check(ctrl, means, end, log, log_cap);
+    const bool due = end > base && end % ctrl->check == 0;
+    if (due) tree_means(d.tree, d.nm, d.ns, d.tree_vals, means);
+    __syncthreads();  // the means are written, and every thread has read ctrl
+    if (threadIdx.x != 0) return;
+    if (due) adr_check(ctrl, means, end, d.log, d.log_cap);
     ctrl->n_base = end;
     if (end >= ctrl->limit) ctrl->done = 1;
     const int go = (!ctrl->done && end < ctrl->n_pause) ? 1 : 0;
     if (use_handle) cudaGraphSetConditional(h, go);
-}
-
-__global__ void adr_means_pick_kernel(const AdrCtrl* ctrl, const float* buf0, const float* buf1,
-                                      const float** out) {
-    // chooses the buffer holding the state at the end of the current chunk
-    const long long end = min(ctrl->n_base + (long long)ctrl->check, ctrl->limit);
-    *out = (end & 1) ? buf1 : buf0;
-}
-
-// means over the buffer the device picked (graph body: pointer comes from device memory)
-__global__ void means_leaf_indirect_kernel(const AdrCtrl* __restrict__ ctrl, const float* const* src_p,
-                                           long long N, const int* __restrict__ idx, PairTree t,
-                                           int ns, float* __restrict__ vals) {
-    if (ctrl->done) return;
-    const long long base = ctrl->n_base;
-    const long long end = min(base + (long long)ctrl->check, ctrl->limit);
-    if (!(end > base && end % ctrl->check == 0)) return;
-    const long long tid = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (tid >= (long long)t.nleaf * ns) return;
-    const int leaf = (int)(tid % t.nleaf);
-    const int j = (int)(tid / t.nleaf);
-    vals[(long long)j * (t.nleaf + t.ninner) + leaf] =
-        leaf_sum(*src_p + (long long)j * N, idx, t, leaf);
-}
-
-__global__ void means_tree_cond_kernel(const AdrCtrl* __restrict__ ctrl, PairTree t, long long nm,
-                                       float* __restrict__ vals, float* __restrict__ means) {
-    if (ctrl->done) return;
-    const long long base = ctrl->n_base;
-    const long long end = min(base + (long long)ctrl->check, ctrl->limit);
-    if (!(end > base && end % ctrl->check == 0)) return;
-    const int j = blockIdx.x;
-    tree_mean(t, nm, vals + (long long)j * (t.nleaf + t.ninner), means + j);
 }
 
 // ---------------------------------------------------------------------------
@@ -270,7 +337,10 @@ template <int ND, int NS>
 static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl, int k,
                           cudaStream_t s) {
     if (d.nm <= 0) return cudaSuccess;
-    auto kern = d.has_bf ? adr_step_kernel<ND, NS, true> : adr_step_kernel<ND, NS, false>;
+    auto kern = d.near ? (d.has_bf ? adr_step_kernel<ND, NS, true, false>
+                                   : adr_step_kernel<ND, NS, false, false>)
+                       : (d.has_bf ? adr_step_kernel<ND, NS, true, true>
+                                   : adr_step_kernel<ND, NS, false, true>);
     const long long nb = (d.nm + kAdrThreads - 1) / kAdrThreads;
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3((unsigned)nb);
@@ -306,19 +376,26 @@ cudaError_t adr_launch_step(const AdrDev& d, const prt_adr_params& p, AdrCtrl* c
     return d.nd == 3 ? step_nd<3>(d, p, ctrl, kstep, s) : step_nd<2>(d, p, ctrl, kstep, s);
 }
 
-// float32 speed sqrt((v0^2 + v1^2) [+ v2^2]) the way numpy forms it
-__global__ void speed_kernel(const float* __restrict__ vel, Grid g, int nd,
-                             float* __restrict__ sp) {
-    const long long c = (long long)blockIdx.x * blockDim.x + threadIdx.x;
-    if (c >= g.n) return;
+// The axial velocity (which 0) or the float32 speed sqrt((v0^2 + v1^2) [+ v2^2])
+// the way numpy forms it (which 1) of each solute voxel.
+__global__ void vel_rows_kernel(const float* __restrict__ vel, const int* __restrict__ idx,
+                                long long nm, long long n, int nd, int which,
+                                float* __restrict__ row) {
+    const long long k = (long long)blockIdx.x * blockDim.x + threadIdx.x;
+    if (k >= nm) return;
+    const long long c = idx[k];
     const float v0 = vel[c];
-    const float v1 = vel[g.n + c];
+    if (which == 0) {
+        row[k] = v0;
+        return;
+    }
+    const float v1 = vel[n + c];
     float s = v0 * v0 + v1 * v1;
     if (nd == 3) {
-        const float v2 = vel[2 * g.n + c];
+        const float v2 = vel[2 * n + c];
         s = s + v2 * v2;
     }
-    sp[c] = sqrtf(s);
+    row[k] = sqrtf(s);
 }
 
 // max |vel[a]| over the solute voxels (order-free: max is exact)
@@ -352,25 +429,27 @@ cudaError_t adr_launch_flags(const uint8_t* mat, const Grid& g, int nd, int pore
     return cudaGetLastError();
 }
 
+static unsigned leaf_blocks(const PairTree& t, int ns) {
+    return (unsigned)(((long long)t.nleaf * ns + kLeafThreads / 32 - 1) / (kLeafThreads / 32));
+}
+
 // mean_axial, mean_speed (numpy float32 pairwise means over the solute
 // voxels) into means[0..1]; max |v_a| bits into vmax_bits[0..2]; biofilm
-// voxel count into *nbf.  tmp: n floats of scratch.
+// voxel count into *nbf, the inlet plane's solute voxels into *n0.  tmp: n
+// floats of scratch.
 cudaError_t adr_launch_vel_stats(const float* vel, const AdrDev& d, float* tmp, float* means,
-                                 unsigned* vmax_bits, unsigned long long* nbf, cudaStream_t s) {
+                                 unsigned* vmax_bits, unsigned long long* nbf, int* n0, cudaStream_t s) {
     const Grid& g = d.g;
     const unsigned nb = (unsigned)((g.n + 255) / 256);
     cudaError_t e;
     for (int which = 0; which < 2; ++which) {
-        const float* src = vel;
-        if (which == 1) {
-            speed_kernel<<<nb, 256, 0, s>>>(vel, g, d.nd, tmp);
-            src = tmp;
+        if (d.nm > 0) {
+            vel_rows_kernel<<<(unsigned)((d.nm + 255) / 256), 256, 0, s>>>(
+                vel, d.idx, d.nm, g.n, d.nd, which, tmp);
+            means_leaf_kernel<<<leaf_blocks(d.tree, 1), kLeafThreads, 0, s>>>(tmp, 0, d.nm, d.tree,
+                                                                             1, d.tree_vals);
         }
-        if (d.tree.nleaf > 0) {
-            means_leaf_kernel<<<(unsigned)((d.tree.nleaf + 255) / 256), 256, 0, s>>>(
-                src, g.n, d.idx, d.tree, 1, d.tree_vals);
-        }
-        means_tree_kernel<<<1, 256, 0, s>>>(d.tree, d.nm, d.tree_vals, means + which);
+        means_tree_kernel<<<1, kTreeThreads, 0, s>>>(d.tree, d.nm, 1, d.tree_vals, means + which);
         e = cudaGetLastError();
         if (e != cudaSuccess) return e;
     }
@@ -378,28 +457,41 @@ cudaError_t adr_launch_vel_stats(const float* vel, const AdrDev& d, float* tmp, 
         vmax_kernel<<<(unsigned)((d.nm + 255) / 256), 256, 0, s>>>(vel, d.idx, d.nm, g.n, d.nd,
                                                                   vmax_bits);
     count_bf_kernel<<<nb, 256, 0, s>>>(d.flags, g.n, nbf);
+    adr_inlet_count_kernel<<<1, 1, 0, s>>>(d.idx, d.nm, g.ny * g.nz, n0);
     return cudaGetLastError();
 }
 
-// Face velocities and the initial state; the flags are already built.
-cudaError_t adr_launch_setup(const uint8_t* mat, const float* vel, const prt_adr_params& p,
-                             const AdrDev& d, cudaStream_t s) {
-    const Grid& g = d.g;
-    const unsigned nb = (unsigned)((g.n + 255) / 256);
-    cudaError_t e;
-    for (int i = 0; i < d.nd; ++i) {
-        const int a = (d.nd == 3) ? i : (i == 0 ? 0 : 2);
-        const int ext = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-        const long long nf = g.n / ext * (ext + 1);
-        // velocity component of storage axis a: 3D -> a; 2D -> x: 0, y (stored as z): 1
-        const int comp = (d.nd == 3) ? a : (a == 0 ? 0 : 1);
-        adr_faces_kernel<<<(unsigned)((nf + 255) / 256), 256, 0, s>>>(
-            mat, vel + (long long)comp * g.n, g, a, p.pore_code, p.biofilm_code, p.u_scale,
-            const_cast<float*>(d.face[a]));
-        e = cudaGetLastError();
-        if (e != cudaSuccess) return e;
-    }
-    adr_init_kernel<<<nb, 256, 0, s>>>(d.flags, g, p, d.buf[0], d.ladder);
+cudaError_t adr_launch_map(const AdrDev& d, int* map, unsigned* reach, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(reach, 0, sizeof(*reach), s);
+    if (e != cudaSuccess || d.nm <= 0) return e;
+    const unsigned nb = (unsigned)((d.nm + 255) / 256);
+    adr_map_kernel<<<nb, 256, 0, s>>>(d.idx, d.nm, map);
+    adr_reach_kernel<<<nb, 256, 0, s>>>(d, map, reach);
+    return cudaGetLastError();
+}
+
+cudaError_t adr_launch_setup(const float* vel, const prt_adr_params& p, const AdrDev& d,
+                             const int* map, cudaStream_t s) {
+    if (d.nm <= 0) return cudaSuccess;
+    const unsigned nb = (unsigned)((d.nm + 255) / 256);
+    adr_tables_kernel<<<nb, 256, 0, s>>>(vel, d, p.u_scale, map, const_cast<uint2*>(d.near),
+                                         const_cast<int4*>(d.nb), const_cast<float2*>(d.face),
+                                         const_cast<uint32_t*>(d.cflags));
+    adr_init_kernel<<<nb, 256, 0, s>>>(d, p, d.buf[0]);
+    return cudaGetLastError();
+}
+
+cudaError_t adr_launch_rows(const AdrDev& d, const float* buf, float* rows, cudaStream_t s) {
+    if (d.nm <= 0) return cudaSuccess;
+    adr_rows_kernel<<<(unsigned)((d.nm + 255) / 256), 256, 0, s>>>(d, buf, rows);
+    return cudaGetLastError();
+}
+
+cudaError_t adr_launch_expand(const AdrDev& d, const float* rows, float* out, cudaStream_t s) {
+    cudaError_t e = cudaMemsetAsync(out, 0, (size_t)d.g.n * d.ns * sizeof(float), s);
+    if (e != cudaSuccess || d.nm <= 0) return e;
+    adr_expand_kernel<<<(unsigned)((d.nm + 255) / 256), 256, 0, s>>>(rows, d.idx, d.nm, d.g.n, d.ns,
+                                                                    out);
     return cudaGetLastError();
 }
 
@@ -412,35 +504,21 @@ cudaError_t adr_launch_compact(const uint8_t* mflag, long long n, int* cnt, long
     return cudaGetLastError();
 }
 
-cudaError_t adr_launch_means(const AdrDev& d, AdrCtrl* ctrl, int slot, float* means_out,
-                             cudaStream_t s) {
-    // explicit means of ladder slot `slot` (slot >= 0), outside the time loop
-    (void)ctrl;
-    const float* src = d.ladder + (long long)slot * d.ns * d.g.n;
-    if (d.tree.nleaf > 0) {
-        const long long nt = (long long)d.tree.nleaf * d.ns;
-        means_leaf_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(src, d.g.n, d.idx, d.tree, d.ns,
-                                                                       d.tree_vals);
-    }
-    means_tree_kernel<<<d.ns, 256, 0, s>>>(d.tree, d.nm, d.tree_vals, means_out);
+cudaError_t adr_launch_means(const AdrDev& d, int slot, float* means_out, cudaStream_t s) {
+    // the means of ladder slot `slot`, outside the time loop
+    const float* src = d.ladder + (long long)slot * d.ns * d.nm;
+    if (d.tree.nleaf > 0)
+        means_leaf_kernel<<<leaf_blocks(d.tree, d.ns), kLeafThreads, 0, s>>>(
+            src, d.nm, d.nm, d.tree, d.ns, d.tree_vals);
+    means_tree_kernel<<<1, kTreeThreads, 0, s>>>(d.tree, d.nm, d.ns, d.tree_vals, means_out);
     return cudaGetLastError();
 }
 
-cudaError_t adr_launch_chunk_means(const AdrDev& d, AdrCtrl* ctrl, const float** src_slot,
-                                   float* means_out, cudaStream_t s) {
-    adr_means_pick_kernel<<<1, 1, 0, s>>>(ctrl, d.buf[0], d.buf[1], src_slot);
-    if (d.tree.nleaf > 0) {
-        const long long nt = (long long)d.tree.nleaf * d.ns;
-        means_leaf_indirect_kernel<<<(unsigned)((nt + 255) / 256), 256, 0, s>>>(
-            ctrl, src_slot, d.g.n, d.idx, d.tree, d.ns, d.tree_vals);
-    }
-    means_tree_cond_kernel<<<d.ns, 256, 0, s>>>(ctrl, d.tree, d.nm, d.tree_vals, means_out);
-    return cudaGetLastError();
-}
-
-cudaError_t adr_launch_stop(const AdrDev& d, AdrCtrl* ctrl, const float* means,
-                            cudaGraphConditionalHandle h, int use_handle, cudaStream_t s) {
-    adr_stop_kernel<<<1, 32, 0, s>>>(ctrl, means, d.log, d.log_cap, h, use_handle);
+cudaError_t adr_launch_chunk_end(const AdrDev& d, AdrCtrl* ctrl, float* means,
+                                 cudaGraphConditionalHandle h, int use_handle, cudaStream_t s) {
+    if (d.tree.nleaf > 0)
+        chunk_leaf_kernel<<<leaf_blocks(d.tree, d.ns), kLeafThreads, 0, s>>>(ctrl, d);
+    chunk_end_kernel<<<1, kTreeThreads, 0, s>>>(ctrl, d, means, h, use_handle);
     return cudaGetLastError();
 }
 

@@ -22,20 +22,22 @@ __device__ __forceinline__ float min_nan(float a, float b) {
     return r;
 }
 
-// _muscl (prtlb_3d.py:650-705): up + 1/2 minmod(down - up, up - upup), the
-// minmod written as 1/2 (sgn a + sgn b) min(|a|, |b|).  The signs are taken
-// from the sign bits (copysign(1, d)), which differs from numpy's sign()
-// only at d = +-0; there min(|a|, |b|) = 0, the slope is a zero of either
-// sign, and up + 1/2 slope is up exactly unless up is -0.  No concentration
-// is ever -0 (states start at +0 or above, a sum is -0 only of two -0
-// operands, and the clip keeps its operand), so the result is numpy's bit
-// for bit; NaN reaches it through the min.
-__device__ __forceinline__ float muscl(float up, float upup, float down) {
-    const float d1 = down - up;
-    const float d2 = up - upup;
-    const float slope =
-        (0.5f * (copysignf(1.f, d1) + copysignf(1.f, d2))) * min_nan(fabsf(d1), fabsf(d2));
-    return up + 0.5f * slope;
+// The upwind face value of _muscl (prtlb_3d.py:650-705), up + 1/2 minmod(down -
+// up, up - upup), from the two differences along the axis, taken upwards: for
+// flow up the axis they are (down - up, up - upup) themselves and s = 1, for
+// flow down it both are negated, which negates the slope exactly, and s = -1.
+// The reference forms minmod as 1/2 (sgn a + sgn b) min(|a|, |b|) and halves
+// it; (1/4 sgn a + 1/4 sgn b) min rounds the same once (1/2 min or 0), and s
+// x is exact inside the fused add.  The signs are taken from the sign bits,
+// which differs from numpy's sign() only at +-0; there the product is a zero,
+// and up + zero is up exactly unless up is -0.  No concentration is ever -0
+// (states start at +0 or above, a sum is -0 only of two -0 operands, and the
+// clip keeps its operand), so the result is numpy's bit for bit; NaN and
+// infinities reach it through the min and the product.
+__device__ __forceinline__ float limited(float up, float a, float b, float s) {
+    const float q = copysignf(0.25f, a) + copysignf(0.25f, b);
+    const float x = q * min_nan(fabsf(a), fabsf(b));
+    return __fmaf_rn(s, x, up);
 }
 
 template <int ND>
@@ -70,159 +72,118 @@ __device__ __forceinline__ VoxelPos voxel_pos(int c, const Grid& g) {
     return v;
 }
 
-// The same with the run's precomputed divisors (c < 2^31).
-__device__ __forceinline__ VoxelPos voxel_pos(int c, const FastDiv& dz, const FastDiv& dy) {
-    VoxelPos v;
-    v.c = c;
-    const unsigned t = (unsigned)c;
-    const unsigned q = fast_div(t, dz);
-    v.p[2] = (int)(t - q * dz.d);
-    const unsigned x = fast_div(q, dy);
-    v.p[1] = (int)(q - x * dy.d);
-    v.p[0] = (int)x;
-    return v;
-}
-
-// A load that is always issued, before the flags that decide whether its
-// value is used are known: the address is in bounds either way (an
-// edge-clamped neighbour), and the buffer is not written by this launch.
-__device__ __forceinline__ float ld_early(const float* p) {
-    float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
-    return v;
-}
-
 __device__ __forceinline__ int extent(const Grid& g, int a) {
     return a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
 }
 __device__ __forceinline__ int stride(const Grid& g, int a) {
     return a == 0 ? g.ny * g.nz : (a == 1 ? g.nz : 1);
 }
-// index of the low face of voxel v along axis a in the (n_a + 1)-long face array
-__device__ __forceinline__ int face_lo(const Grid& g, const VoxelPos& v, int a) {
-    if (a == 0) return v.c;
-    if (a == 1) return (v.p[0] * (g.ny + 1) + v.p[1]) * g.nz + v.p[2];
-    return (v.p[0] * g.ny + v.p[1]) * (g.nz + 1) + v.p[2];
+
+// A load through the read-only path (the buffer is not written by this
+// launch), issued where it stands; and the same only where u >= 0, or only
+// where it is not, else 0: the far value that the upwind side does not need
+// is not read.
+__device__ __forceinline__ float ld_early(const float* p) {
+    float v;
+    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    return v;
 }
-__device__ __forceinline__ int face_step(const Grid& g, int a) {
-    return a == 0 ? g.ny * g.nz : (a == 1 ? g.nz : 1);
+__device__ __forceinline__ float ld_if_up(const float* p, float u) {
+    float v;
+    asm volatile(
+        "{\n.reg .pred q;\nsetp.ge.f32 q, %2, 0f00000000;\nmov.f32 %0, 0f00000000;\n"
+        "@q ld.global.nc.f32 %0, [%1];\n}"
+        : "=&f"(v)
+        : "l"(p), "f"(u));
+    return v;
+}
+__device__ __forceinline__ float ld_if_down(const float* p, float u) {
+    float v;
+    asm volatile(
+        "{\n.reg .pred q;\nsetp.ltu.f32 q, %2, 0f00000000;\nmov.f32 %0, 0f00000000;\n"
+        "@q ld.global.nc.f32 %0, [%1];\n}"
+        : "=&f"(v)
+        : "l"(p), "f"(u));
+    return v;
 }
 
-// A neighbour value of chemical j.  Every neighbour that is actually read is a
-// solute voxel (the open / far flags guarantee it), so it is on the inlet
-// plane exactly when its x is 0; there the pinned feed replaces the stored
-// value (step(), prtlb_3d.py:1392-1400, pins before transport).
-__device__ __forceinline__ float ld_c(const float* __restrict__ Cj, int c, int x, bool pin,
-                                      float feed) {
-    const float v = ld_early(Cj + c);
-    return (pin && x == 0) ? feed : v;
-}
-
-// One axis of transport() at one voxel (prtlb_3d.py:1182-1208), from the
-// four neighbour values along the axis (clamped positions, inlet feed already
-// applied), the two face velocities and the voxel's flags: adds the axis'
-// diffusion and advection to `out` and its velocity difference to `divu`, in
-// the reference's operation order.  BF: the run has biofilm; without it no
-// voxel carries a biofilm flag, every face takes the pore diffusivity, and
-// the biofilm count is not formed.  Every transport kernel calls this, so
-// they compute the same function bit for bit.
-template <bool BF>
-__device__ __forceinline__ void transport_axis(float& out, float& divu, float Cc, float vm1,
-                                               float vm2, float vp1, float vp2, float uL,
-                                               float uH, uint32_t fl, int a,
-                                               const float (&dj)[3]) {
-    const bool oL = fl & f_open_lo(a), oH = fl & f_open_hi(a);
-    const bool fL = fl & f_far_lo(a), fH = fl & f_far_hi(a);
-    const float Cm1 = oL ? vm1 : Cc;
-    const float Cp1 = oH ? vp1 : Cc;
-    const float Cm2 = fL ? vm2 : Cm1;
-    const float Cp2 = fH ? vp2 : Cp1;
-    float DL, DH;
-    if constexpr (BF) {
-        const int bf = (fl & F_BF) ? 1 : 0;
-        // face diffusivity by the biofilm count of its two voxels (0, 1,
-        // 2); selected, not indexed, so the table stays in registers
-        const int nl = bf + ((fl & f_nbf_lo(a)) ? 1 : 0);
-        const int nh = bf + ((fl & f_nbf_hi(a)) ? 1 : 0);
-        DL = oL ? (nl == 0 ? dj[0] : (nl == 1 ? dj[1] : dj[2])) : 0.f;
-        DH = oH ? (nh == 0 ? dj[0] : (nh == 1 ? dj[1] : dj[2])) : 0.f;
-    } else {
-        DL = oL ? dj[0] : 0.f;
-        DH = oH ? dj[0] : 0.f;
-    }
-    // out += D_hi (C+1 - C) + D_lo (C-1 - C)
-    out = out + (DH * (Cp1 - Cc) + DL * (Cm1 - Cc));
-    // upwind face values: the stencil is chosen first and limited once
-    // (the same function of the same three values as choosing between
-    // the two limited candidates)
-    const bool rH = uH >= 0.f, rL = uL >= 0.f;
-    const float fh = muscl(rH ? Cc : Cp1, rH ? Cm1 : Cp2, rH ? Cp1 : Cc);
-    const float flo = muscl(rL ? Cm1 : Cc, rL ? Cm2 : Cp1, rL ? Cc : Cm1);
-    // out -= u_hi f_hi - u_lo f_lo
-    out = out - (uH * fh - uL * flo);
-    divu = divu + (uH - uL);
-}
-
-// transport() of one chemical at one voxel (prtlb_3d.py:1182-1208), loading
-// its neighbours and faces from global memory (the compacted-list kernels).
-// INNER: the voxel is at least three planes from the inlet and two from
-// every other face of the grid, so no neighbour position needs clamping and
-// no neighbour lies on the inlet plane (no feed to substitute): the same
-// values from fewer instructions.
-// The face velocities of one voxel, low and high face of each of its ND axes
-// (in Axes<ND> order).  They do not change during a run.
-struct VoxelFaces {
-    float lo[3], hi[3];
+// What one transport step needs of solute voxel k that does not change during
+// a run: per axis its neighbours' places (x, y, z, w = far low, low, high, far
+// high) and its low and high face velocity, and its flags where the run
+// reads them.  WIDE: from AdrDev::nb instead of AdrDev::near.
+template <int ND>
+struct VoxelSetup {
+    int4 nb[ND];
+    float2 fc[ND];
+    uint32_t fl;
 };
 
-template <int ND>
-__device__ __forceinline__ VoxelFaces load_faces(const Grid& g, const VoxelPos& v,
-                                                 const float* const* __restrict__ face) {
-    VoxelFaces fc;
+template <int ND, bool BF, bool WIDE>
+__device__ __forceinline__ VoxelSetup<ND> voxel_setup(const AdrDev& d, const prt_adr_params& p,
+                                                      unsigned k) {
+    VoxelSetup<ND> s;
+    const unsigned nm = (unsigned)d.nm;
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        const int a = Axes<ND>::ax(i);
-        const int fi = face_lo(g, v, a);
-        fc.lo[i] = ld_early(face[a] + fi);
-        fc.hi[i] = ld_early(face[a] + fi + face_step(g, a));
+        if constexpr (WIDE) {
+            s.nb[i] = __ldg(d.nb + (i * nm + k));
+        } else {
+            const uint2 q = __ldg(d.near + (i * nm + k));
+            s.nb[i] = make_int4((int)(k - (q.x & 0xffffu)), (int)(k - (q.x >> 16)),
+                                (int)(k + (q.y & 0xffffu)), (int)(k + (q.y >> 16)));
+        }
+        s.fc[i] = __ldg(d.face + (i * nm + k));
     }
-    return fc;
+    s.fl = (BF || (p.abio_on && p.surface_only)) ? __ldg(d.cflags + k) : 0u;
+    return s;
 }
 
-template <int ND, bool BF, bool INNER = false>
-__device__ __forceinline__ float transport_one(const float* __restrict__ Cj, const Grid& g,
-                                               const VoxelPos& v, uint32_t fl,
-                                               const VoxelFaces& fc, float Cc,
-                                               bool pin, float feed, const float (&dj)[3]) {
+// transport() of one chemical at one voxel (prtlb_3d.py:1182-1208): per axis
+// the diffusion and advection are added to the sum in the reference's
+// operation order.  The places of closed neighbours are the voxel's own (its
+// near one for a far neighbour), so their differences vanish as the
+// reference's replaced values do.  BF: the run has biofilm; without it every
+// face takes the pore diffusivity.  Every transport kernel calls this, so
+// they compute the same function bit for bit.
+template <int ND, bool BF>
+__device__ __forceinline__ float transport_one(const float* __restrict__ Cj,
+                                               const VoxelSetup<ND>& s, float Cc,
+                                               const float (&dj)[3]) {
+    float m2[ND], m1[ND], p1[ND], p2[ND];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+        m1[i] = ld_early(Cj + (unsigned)s.nb[i].y);
+        p1[i] = ld_early(Cj + (unsigned)s.nb[i].z);
+        m2[i] = ld_if_up(Cj + (unsigned)s.nb[i].x, s.fc[i].x);
+        p2[i] = ld_if_down(Cj + (unsigned)s.nb[i].w, s.fc[i].y);
+    }
     float out = 0.f;
     float divu = 0.f;
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        const int a = Axes<ND>::ax(i);
-        const int s = stride(g, a);
-        float vm1, vp1, vm2, vp2;
-        if constexpr (INNER) {
-            vm1 = ld_early(Cj + (v.c - s));
-            vp1 = ld_early(Cj + (v.c + s));
-            vm2 = ld_early(Cj + (v.c - 2 * s));
-            vp2 = ld_early(Cj + (v.c + 2 * s));
-        } else {
-            const int p = v.p[a];
-            const int n = extent(g, a);
-            // clamped (edge-replicated) neighbour positions
-            const int pm1 = p > 0 ? p - 1 : 0, pm2 = p > 1 ? p - 2 : 0;
-            const int pp1 = p < n - 1 ? p + 1 : n - 1, pp2 = p < n - 2 ? p + 2 : n - 1;
-            const int x0 = v.p[0];
-            const int xm1 = (a == 0) ? pm1 : x0, xm2 = (a == 0) ? pm2 : x0;
-            const int xp1 = (a == 0) ? pp1 : x0, xp2 = (a == 0) ? pp2 : x0;
-            // all four neighbours are loaded before the flags choose among
-            // them (clamped addresses are always in the grid)
-            vm1 = ld_c(Cj, v.c + (pm1 - p) * s, xm1, pin, feed);
-            vp1 = ld_c(Cj, v.c + (pp1 - p) * s, xp1, pin, feed);
-            vm2 = ld_c(Cj, v.c + (pm2 - p) * s, xm2, pin, feed);
-            vp2 = ld_c(Cj, v.c + (pp2 - p) * s, xp2, pin, feed);
+        const float uL = s.fc[i].x, uH = s.fc[i].y;
+        float DL = dj[0], DH = dj[0];
+        if constexpr (BF) {
+            // face diffusivity by the biofilm count of its two voxels (0, 1,
+            // 2); selected, not indexed, so the table stays in registers
+            const int a = Axes<ND>::ax(i);
+            const bool bf = s.fl & F_BF;
+            const float pore = bf ? dj[1] : dj[0], film = bf ? dj[2] : dj[1];
+            DL = (s.fl & f_nbf_lo(a)) ? film : pore;
+            DH = (s.fl & f_nbf_hi(a)) ? film : pore;
         }
-        transport_axis<BF>(out, divu, Cc, vm1, vm2, vp1, vp2, fc.lo[i], fc.hi[i], fl, a, dj);
+        // differences upwards along the axis
+        const float below = Cc - m1[i], above = p1[i] - Cc;
+        // out += D_hi (C+1 - C) + D_lo (C-1 - C)
+        out = out + (DH * above - DL * below);
+        const bool rH = uH >= 0.f, rL = uL >= 0.f;
+        const float fh = limited(rH ? Cc : p1[i], above, rH ? below : p2[i] - p1[i],
+                                 rH ? 1.f : -1.f);
+        const float flo = limited(rL ? m1[i] : Cc, below, rL ? m1[i] - m2[i] : above,
+                                  rL ? 1.f : -1.f);
+        // out -= u_hi f_hi - u_lo f_lo
+        out = out - (uH * fh - uL * flo);
+        divu = divu + (uH - uL);
     }
     return out + Cc * divu;
 }
@@ -320,87 +281,54 @@ __device__ __forceinline__ void adr_update(const float (&C)[NS], const float (&T
     }
 }
 
-// step() at one solute voxel (see adr_voxel), its flags and position known.
-template <int ND, int NS, bool BF, bool INNER>
-__device__ __forceinline__ void adr_voxel_body(const AdrDev& d, const prt_adr_params& p,
-                                               long long n, int c, uint32_t fl,
-                                               const VoxelPos& v, const VoxelFaces& fc) {
-    const int N = (int)d.g.n;
+// One transport step of solute voxel k (compacted C order) at step n: reads the
+// state after step n-1 from buf[(n-1)&1], writes the state after step n to
+// buf[n&1] and, when n is a snapshot step, to its ladder slot.  On the inlet
+// plane the pinned feed replaces a value before transport (step(),
+// prtlb_3d.py:1392-1400), so that is what the next step is given; the value
+// itself goes behind the row.
+template <int ND, int NS, bool BF>
+__device__ __forceinline__ void adr_voxel_step(const AdrDev& d, const prt_adr_params& p,
+                                               long long n, unsigned k,
+                                               const VoxelSetup<ND>& s) {
+    const unsigned ms = d.ms;
     const float* __restrict__ Cin = d.buf[(n - 1) & 1];
     float* __restrict__ Cout = d.buf[n & 1];
-    const bool x0 = fl & F_X0;
     float C[NS];
 #pragma unroll
-    for (int j = 0; j < NS; ++j) {
-        const bool pin = (p.pinned_mask >> j) & 1u;
-        C[j] = (pin && x0) ? p.feed[j] : Cin[j * N + c];
-    }
+    for (int j = 0; j < NS; ++j) C[j] = Cin[j * ms + k];
     float T[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
         T[j] = 0.f;
         if ((p.moving_mask >> j) & 1u) {
-            const bool pin = (p.pinned_mask >> j) & 1u;
             const float dj[3] = {p.dface[j][0], p.dface[j][1], p.dface[j][2]};
-            T[j] = transport_one<ND, BF, INNER>(Cin + j * N, d.g, v, fl, fc, C[j], pin,
-                                                p.feed[j], dj);
+            T[j] = transport_one<ND, BF>(Cin + j * ms, s, C[j], dj);
         }
     }
     float cn[NS];
-    adr_update<ND, NS>(C, T, fl, p, cn);
+    adr_update<ND, NS>(C, T, s.fl, p, cn);
     const int slot = d.slot_of_step[n];
-    float* __restrict__ lad = slot >= 0 ? d.ladder + (long long)slot * NS * N : nullptr;
+    if (slot >= 0) {
+        float* __restrict__ lad = d.ladder + (long long)slot * NS * d.nm;
 #pragma unroll
-    for (int j = 0; j < NS; ++j) {
-        Cout[j * N + c] = cn[j];
-        if (lad) lad[j * N + c] = cn[j];
+        for (int j = 0; j < NS; ++j) lad[j * d.nm + k] = cn[j];
     }
+    if (k < (unsigned)d.n0) {
+#pragma unroll
+        for (int j = 0; j < NS; ++j) {
+            Cout[j * ms + (unsigned)d.nm + k] = cn[j];
+            if ((p.pinned_mask >> j) & 1u) cn[j] = p.feed[j];
+        }
+    }
+#pragma unroll
+    for (int j = 0; j < NS; ++j) Cout[j * ms + k] = cn[j];
 }
 
-// What one transport step needs of solute voxel number kk (compacted C-order
-// list) that does not change during a run: its voxel index, flags,
-// position and face velocities.
-struct VoxelSetup {
-    int c;
-    uint32_t fl;
-    VoxelPos v;
-    VoxelFaces fc;
-};
-
-template <int ND>
-__device__ __forceinline__ VoxelSetup voxel_setup(const AdrDev& d, long long kk) {
-    VoxelSetup s;
-    s.c = d.idx[kk];
-    s.fl = d.flags[s.c];
-    s.v = voxel_pos(s.c, d.div_z, d.div_y);
-    s.fc = load_faces<ND>(d.g, s.v, d.face);
-    return s;
-}
-
-// One transport step of a solute voxel at step n: reads the state after
-// step n-1 from buf[(n-1)&1], writes the state after step n to buf[n&1]
-// and, when n is a snapshot step, to its ladder slot.  A warp whose voxels
-// all lie inside the grid's interior (see transport_one) takes the interior
-// form; the two forms give the same bits.
-template <int ND, int NS, bool BF = true>
-__device__ __forceinline__ void adr_voxel_step(const AdrDev& d, const prt_adr_params& p,
-                                               long long n, const VoxelSetup& s) {
-    const Grid& g = d.g;
-    const VoxelPos& v = s.v;
-    const bool inner = v.p[0] >= 3 && v.p[0] <= g.nx - 3 &&
-                       (ND == 2 || (v.p[1] >= 2 && v.p[1] <= g.ny - 3)) && v.p[2] >= 2 &&
-                       v.p[2] <= g.nz - 3;
-    if (__all_sync(__activemask(), inner))
-        adr_voxel_body<ND, NS, BF, true>(d, p, n, s.c, s.fl, v, s.fc);
-    else
-        adr_voxel_body<ND, NS, BF, false>(d, p, n, s.c, s.fl, v, s.fc);
-}
-
-// The same for solute voxel number kk (compacted C-order list).
-template <int ND, int NS, bool BF = true>
+template <int ND, int NS, bool BF, bool WIDE>
 __device__ __forceinline__ void adr_voxel(const AdrDev& d, const prt_adr_params& p, long long n,
-                                          long long kk) {
-    adr_voxel_step<ND, NS, BF>(d, p, n, voxel_setup<ND>(d, kk));
+                                          unsigned k) {
+    adr_voxel_step<ND, NS, BF>(d, p, n, k, voxel_setup<ND, BF, WIDE>(d, p, k));
 }
 
 // The check of the time loop at step `end` (prtlb_3d.py:1499-1543), in
@@ -451,54 +379,60 @@ __device__ inline void adr_check(AdrCtrl* ctrl, const float* __restrict__ means,
     }
 }
 
-// Sum of leaf `leaf` of numpy's float32 pairwise tree over the solute
-// values s[idx[...]]: under 8 values sequentially from 0, otherwise eight
-// interleaved accumulators ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)) and a tail.
-__device__ inline float leaf_sum(const float* __restrict__ s, const int* __restrict__ idx,
-                                 const PairTree& t, int leaf) {
-    const int* ix = idx + t.leaf_start[leaf];
-    const int len = t.leaf_len[leaf];
+// Sum of the leaf [start, start + len) (at most 128 values) of numpy's float32
+// pairwise tree over the solute values of a row, by one warp: under 8 values
+// sequentially from 0, otherwise eight interleaved accumulators
+// ((r0+r1)+(r2+r3))+((r4+r5)+(r6+r7)) and a tail.  The lanes load the values
+// into `sh` (through L2: other blocks of the launch may have written them),
+// lanes 0-7 run the accumulators and every lane then combines them and adds
+// the tail.  The result is the same in every lane.
+__device__ __forceinline__ float warp_leaf_sum(const float* __restrict__ row, unsigned n0,
+                                               unsigned nm, int start, int len, float* sh) {
+    const int lane = threadIdx.x & 31;
+    for (int i = lane; i < len; i += 32)
+        sh[i] = __ldcg(row + solute_place((unsigned)(start + i), n0, nm));
+    __syncwarp();
     float res;
     if (len < 8) {
         res = 0.f;
-        for (int i = 0; i < len; ++i) res = res + s[ix[i]];
+        for (int i = 0; i < len; ++i) res = res + sh[i];
     } else {
-        float r0 = s[ix[0]], r1 = s[ix[1]], r2 = s[ix[2]], r3 = s[ix[3]];
-        float r4 = s[ix[4]], r5 = s[ix[5]], r6 = s[ix[6]], r7 = s[ix[7]];
-        int i = 8;
-        for (; i < len - (len % 8); i += 8) {
-            r0 = r0 + s[ix[i + 0]];
-            r1 = r1 + s[ix[i + 1]];
-            r2 = r2 + s[ix[i + 2]];
-            r3 = r3 + s[ix[i + 3]];
-            r4 = r4 + s[ix[i + 4]];
-            r5 = r5 + s[ix[i + 5]];
-            r6 = r6 + s[ix[i + 6]];
-            r7 = r7 + s[ix[i + 7]];
+        const int body = len - (len % 8);
+        float r = 0.f;
+        if (lane < 8) {
+            r = sh[lane];
+            for (int i = 8 + lane; i < body; i += 8) r = r + sh[i];
         }
-        res = ((r0 + r1) + (r2 + r3)) + ((r4 + r5) + (r6 + r7));
-        for (; i < len; ++i) res = res + s[ix[i]];
+        float q[8];
+#pragma unroll
+        for (int k = 0; k < 8; ++k) q[k] = __shfl_sync(0xffffffffu, r, k);
+        res = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
+        for (int i = body; i < len; ++i) res = res + sh[i];
     }
+    __syncwarp();  // sh is reused by the warp's next leaf
     return res;
 }
 
-// The inner levels of the tree for one species (the whole block takes
-// part), then mean = (0 + sum) / nm in float32 as ndarray.mean() does.
-// L2: the node values are read through L2 (other blocks of the launch wrote
-// the leaves).
-template <bool L2 = false>
-__device__ inline void tree_mean(const PairTree& t, long long nm, float* v, float* mean) {
+// The inner levels of the tree for ns chemicals at once (the whole block takes
+// part; chemical j's node values at v + j * (nleaf + ninner)), then mean = (0
+// + sum) / nm in float32 as ndarray.mean() does.  The leaves are read through
+// L2 (other blocks may have written them).
+__device__ inline void tree_means(const PairTree& t, long long nm, int ns, float* v,
+                                  float* means) {
+    const int nodes = t.nleaf + t.ninner;
     for (int h = 0; h < t.nlevel; ++h) {
-        for (int i = t.level_off[h] + threadIdx.x; i < t.level_off[h + 1]; i += blockDim.x) {
-            const float* a = v + t.inner_l[i];
-            const float* b = v + t.inner_r[i];
-            v[t.nleaf + i] = L2 ? __ldcg(a) + __ldcg(b) : *a + *b;
+        const int lo = t.level_off[h], width = t.level_off[h + 1] - lo;
+        for (int q = threadIdx.x; q < width * ns; q += blockDim.x) {
+            const int j = q / width, i = lo + q - j * width;
+            float* w = v + (long long)j * nodes;
+            w[t.nleaf + i] = __ldcg(w + t.inner_l[i]) + __ldcg(w + t.inner_r[i]);
         }
+        __threadfence_block();
         __syncthreads();
     }
-    if (threadIdx.x == 0) {
-        const float sum = t.root >= 0 ? 0.f + v[t.root] : 0.f;
-        *mean = sum / (float)nm;  // 0/0 -> NaN for an empty pore space, as numpy
+    if ((int)threadIdx.x < ns) {
+        const float sum = t.root >= 0 ? 0.f + __ldcg(v + (long long)threadIdx.x * nodes + t.root) : 0.f;
+        means[threadIdx.x] = sum / (float)nm;  // 0/0 -> NaN for an empty pore space, as numpy
     }
 }
 

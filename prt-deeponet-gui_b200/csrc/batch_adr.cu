@@ -28,38 +28,6 @@ constexpr int kWarps = kBatchAdrThreads / 32;
 constexpr int kBatchAdrMinBlocks = 4;
 }
 
-// leaf_sum of one leaf (at most 128 values) by one warp, with the same float
-// additions in the same order: the lanes gather the values into `sh` (loads
-// through L2: other blocks of the launch wrote some of them), lanes 0-7 run
-// the eight interleaved accumulators and every lane then combines them and
-// adds the tail.  The result is the same in every lane.
-__device__ __forceinline__ float warp_leaf_sum(const float* __restrict__ s,
-                                               const int* __restrict__ idx, int start, int len,
-                                               float* sh) {
-    const int lane = threadIdx.x & 31;
-    for (int i = lane; i < len; i += 32) sh[i] = __ldcg(s + idx[start + i]);
-    __syncwarp();
-    float res;
-    if (len < 8) {
-        res = 0.f;
-        for (int i = 0; i < len; ++i) res = res + sh[i];
-    } else {
-        const int body = len - (len % 8);
-        float r = 0.f;
-        if (lane < 8) {
-            r = sh[lane];
-            for (int i = 8 + lane; i < body; i += 8) r = r + sh[i];
-        }
-        float q[8];
-#pragma unroll
-        for (int k = 0; k < 8; ++k) q[k] = __shfl_sync(0xffffffffu, r, k);
-        res = ((q[0] + q[1]) + (q[2] + q[3])) + ((q[4] + q[5]) + (q[6] + q[7]));
-        for (int i = body; i < len; ++i) res = res + sh[i];
-    }
-    __syncwarp();  // sh is reused by the warp's next leaf
-    return res;
-}
-
 // The leaves of block b of job J on a check step n, after the block's
 // voxels of step n are stored: the leaves that start in the block and end
 // inside it, plus each leaf across one of its two seams when the block is
@@ -107,15 +75,15 @@ __device__ __noinline__ void block_leaves(const AdrJob& J, int b, long long n, f
     const int nitems = ninside + (s_lo >= 0) + (s_hi >= 0);
     const int warp = threadIdx.x >> 5;
     const float* src = J.d.buf[n & 1];
-    const long long N = J.d.g.n;
     for (int w = warp; w < nitems * NS; w += kWarps) {
         const int item = w / NS, sp = w % NS;
         int leaf;
         if (item < ninside) leaf = l0 + item;
         else if (item == ninside && s_lo >= 0) leaf = s_lo;
         else leaf = s_hi;
-        const float v = warp_leaf_sum(src + (long long)sp * N, J.d.idx, tr.leaf_start[leaf],
-                                      tr.leaf_len[leaf], sh[warp]);
+        const float v = warp_leaf_sum(src + (long long)sp * J.d.ms, (unsigned)J.d.n0,
+                                      (unsigned)J.d.nm, tr.leaf_start[leaf], tr.leaf_len[leaf],
+                                      sh[warp]);
         if ((threadIdx.x & 31) == 0)
             J.d.tree_vals[(long long)sp * (tr.nleaf + tr.ninner) + leaf] = v;
     }
@@ -131,10 +99,8 @@ __device__ __noinline__ void job_step_end(const AdrJob& J, long long n, long lon
     __threadfence();
     AdrCtrl* ctrl = J.ctrl;
     if (due) {
-        const PairTree& tr = J.d.tree;
-        for (int sp = 0; sp < NS; ++sp)
-            tree_mean<true>(tr, J.d.nm, J.d.tree_vals + (long long)sp * (tr.nleaf + tr.ninner),
-                            J.means + sp);
+        tree_means(J.d.tree, J.d.nm, NS, J.d.tree_vals, J.means);
+        __syncthreads();
     }
     if (threadIdx.x == 0) {
         if (due) adr_check(ctrl, J.means, n, J.d.log, J.d.log_cap);
@@ -194,10 +160,11 @@ __global__ void __launch_bounds__(kBatchAdrThreads, kBatchAdrMinBlocks)
         // selects (uniform over the block: J is the tile's job)
         const bool bf = J.d.has_bf != 0;
         for (int b = tl.b0; b < tl.b0 + tl.nb; ++b) {
-            const long long kk = (long long)b * kBatchAdrThreads + threadIdx.x;
-            if (kk < J.d.nm) {
-                if (bf) adr_voxel<ND, NS, true>(J.d, J.p, n, kk);
-                else adr_voxel<ND, NS, false>(J.d, J.p, n, kk);
+            const unsigned k = (unsigned)b * kBatchAdrThreads + threadIdx.x;
+            if (k < (unsigned)J.d.nm) {
+                if (J.d.near == nullptr) adr_voxel<ND, NS, true, true>(J.d, J.p, n, k);
+                else if (bf) adr_voxel<ND, NS, true, false>(J.d, J.p, n, k);
+                else adr_voxel<ND, NS, false, false>(J.d, J.p, n, k);
             }
             if (due) {
                 __syncthreads();  // the block's voxels of step n are stored

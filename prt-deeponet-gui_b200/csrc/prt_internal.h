@@ -314,18 +314,33 @@ cudaError_t adr_launch_compact(const uint8_t* mflag, long long n, int* cnt, long
 void set_noctx_error(const char* msg);
 
 // Kernel launchers (adr.cu) -------------------------------------------------
+// The transport state is compact: row j of a buffer (stride ms) holds chemical
+// j of the nm solute voxels in C order as their neighbours see them: the
+// voxels of the inlet plane (the first n0) hold the feed where it is pinned.
+// Their own values follow behind the nm (solute_place); only the means and
+// the snapshots read those.
+// near[i * nm + k]: the distances from voxel k to its two lower and two
+// higher neighbours along axis i (far low, low, high, far high; 16 bits
+// each, downwards the first two, upwards the others); 0 is a closed
+// neighbour, a closed far neighbour has the near one's.  Where a distance
+// exceeds 16 bits the run has nb instead, the neighbours' places themselves.
+// face[i * nm + k]: the low and high face velocity.
 struct AdrDev {
     Grid g;
-    FastDiv div_z, div_y;  // by nz and by ny (coordinates of a voxel index)
     int nd;
     int ns;
     int has_bf;  // the run has a biofilm material code (else no biofilm flag is set)
-    const uint32_t* flags;
-    const float* face[3];
+    int n0;      // solute voxels of the inlet plane
+    unsigned ms;
+    const uint32_t* flags;   // per voxel of the grid (set-up)
+    const uint32_t* cflags;  // per solute voxel
+    const uint2* near;  // null when the run has nb
+    const int4* nb;
+    const float2* face;
     float* buf[2];
-    float* ladder;              // slot s at ladder + s * ns * n
+    float* ladder;              // slot s at ladder + s * ns * nm, rows of nm
     const int* slot_of_step;    // -1 or ladder slot for step n
-    const int* idx;             // compressed solute voxel list
+    const int* idx;             // voxel index of each solute voxel
     long long nm;               // solute voxels
     PairTree tree;
     float* tree_vals;           // ns * (nleaf + ninner)
@@ -333,14 +348,28 @@ struct AdrDev {
     int log_cap;
 };
 
-cudaError_t adr_launch_setup(const uint8_t* mat, const float* vel, const prt_adr_params& p,
-                             const AdrDev& d, cudaStream_t s);
+// The place in a row of solute voxel k's own value.
+__host__ __device__ inline unsigned solute_place(unsigned k, unsigned n0, unsigned nm) {
+    return k < n0 ? nm + k : k;
+}
+
+// map[voxel] = solute voxel number (an int per voxel of the grid; set at the
+// solute voxels only), and the largest neighbour distance into *reach.
+cudaError_t adr_launch_map(const AdrDev& d, int* map, unsigned* reach, cudaStream_t s);
+// Neighbours, face velocities, compact flags and the initial state.
+cudaError_t adr_launch_setup(const float* vel, const prt_adr_params& p, const AdrDev& d,
+                             const int* map, cudaStream_t s);
+// Compact rows (ns x nm) to grids (ns x n), 0 outside the solute voxels.
+cudaError_t adr_launch_expand(const AdrDev& d, const float* rows, float* out, cudaStream_t s);
 cudaError_t adr_launch_step(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl,
                             int kstep, cudaStream_t s);
-cudaError_t adr_launch_means(const AdrDev& d, AdrCtrl* ctrl, int slot_or_neg, float* means_out,
-                             cudaStream_t s);
-cudaError_t adr_launch_stop(const AdrDev& d, AdrCtrl* ctrl, const float* means,
-                            cudaGraphConditionalHandle h, int use_handle, cudaStream_t s);
+cudaError_t adr_launch_means(const AdrDev& d, int slot, float* means_out, cudaStream_t s);
+// Ladder rows (ns x nm) from the state in buffer `buf`.
+cudaError_t adr_launch_rows(const AdrDev& d, const float* buf, float* rows, cudaStream_t s);
+// The end of a chunk of `check` steps: the means of the chunk's last step and
+// the stop rule, where they are due, and the WHILE condition when h is used.
+cudaError_t adr_launch_chunk_end(const AdrDev& d, AdrCtrl* ctrl, float* means,
+                                 cudaGraphConditionalHandle h, int use_handle, cudaStream_t s);
 
 // Batched solves (batch.cu, batch_adr.cu, engine.cu) ------------------------
 // A work-list entry: the blocks [b0, b0 + nb) of job `job` (kFlowThreads

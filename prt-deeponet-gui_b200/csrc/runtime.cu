@@ -443,8 +443,6 @@ extern "C" int prt_adr_stage_dev(prt_ctx* ctx, const uint8_t* d_mat, const float
     const Grid g = make_grid(geom->nd, geom->dims);
     const long long N = g.n;
     A.d.g = g;
-    A.d.div_z = make_fastdiv((unsigned)g.nz);
-    A.d.div_y = make_fastdiv((unsigned)g.ny);
     A.d.has_bf = geom->biofilm_code >= 0 ? 1 : 0;
     A.d.nd = geom->nd;
     CK(A.flags.ensure((size_t)N * 4));
@@ -530,7 +528,6 @@ extern "C" int prt_adr_stage_dev(prt_ctx* ctx, const uint8_t* d_mat, const float
     A.d.tree.level_off = A.tree_level_off.as<int>();
     A.d.tree_vals = A.tree_vals.as<float>();
     CK(A.means.ensure(PRT_MAX_SPECIES * 4));
-    CK(A.src_slot.ensure(sizeof(float*)));
     CK(A.ctrl.ensure(sizeof(AdrCtrl)));
     // velocity statistics for the host's set-up
     CK(A.tmp.ensure((size_t)N * 4));
@@ -539,11 +536,14 @@ extern "C" int prt_adr_stage_dev(prt_ctx* ctx, const uint8_t* d_mat, const float
     float* vs_means = A.vstats.as<float>();                                  // 2 floats
     unsigned* vs_max = reinterpret_cast<unsigned*>(A.vstats.as<char>() + 16);  // 3 uints
     unsigned long long* vs_bf = reinterpret_cast<unsigned long long*>(A.vstats.as<char>() + 32);
-    CK(adr_launch_vel_stats(d_vel, A.d, A.tmp.as<float>(), vs_means, vs_max, vs_bf, s));
-    ctx->launches += 8;
+    int* vs_n0 = reinterpret_cast<int*>(A.vstats.as<char>() + 48);
+    CK(adr_launch_vel_stats(d_vel, A.d, A.tmp.as<float>(), vs_means, vs_max, vs_bf, vs_n0, s));
+    ctx->launches += 9;
     unsigned char hv[64];
     CK(cudaMemcpyAsync(hv, A.vstats.p, 64, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));  // host vectors above go out of scope
+    memcpy(&A.d.n0, hv + 48, 4);
+    A.d.ms = (unsigned)((nm + A.d.n0 + 31) / 32 * 32);
     if (stats) {
         memset(stats, 0, sizeof(*stats));
         stats->solute_voxels = nm;
@@ -574,6 +574,13 @@ extern "C" int prt_adr_stage(prt_ctx* ctx, const uint8_t* mat, const float* vel,
     return prt_adr_stage_dev(ctx, A.mat.as<uint8_t>(), A.vel.as<float>(), geom, stats);
 }
 
+// PRT_ADR_WIDE=1: neighbour places instead of 16-bit distances whatever their
+// size (the same neighbours, so the same results).
+static bool wide_neighbours() {
+    const char* v = std::getenv("PRT_ADR_WIDE");
+    return v && v[0] == '1';
+}
+
 extern "C" int prt_adr_begin(prt_ctx* ctx, const prt_adr_params* p) {
     if (!ctx || !p) return fail(ctx, PRT_E_INVALID, "null argument");
     AdrState& A = ctx->adr;
@@ -593,27 +600,47 @@ extern "C" int prt_adr_begin(prt_ctx* ctx, const prt_adr_params* p) {
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
     A.p = *p;
-    const Grid g = A.d.g;
-    const long long N = g.n;
     A.d.ns = p->ns;
-    for (int a = 0; a < 3; ++a) {
-        const int ext = a == 0 ? g.nx : (a == 1 ? g.ny : g.nz);
-        const bool active = (p->nd == 3) || a != 1;
-        CK(A.face[a].ensure(active ? (size_t)(N / ext * (ext + 1)) * 4 : 4));
-        A.d.face[a] = A.face[a].as<float>();
+    const size_t nm = (size_t)std::max(A.d.nm, 1ll);
+    // the neighbours: 16-bit distances where they suffice, else places
+    int* map = A.tmp.as<int>();
+    unsigned* d_reach = reinterpret_cast<unsigned*>(A.vstats.as<char>() + 52);
+    CK(adr_launch_map(A.d, map, d_reach, s));
+    unsigned reach = 0;
+    CK(cudaMemcpyAsync(&reach, d_reach, sizeof(reach), cudaMemcpyDeviceToHost, s));
+    CK(cudaStreamSynchronize(s));
+    A.d.near = nullptr;
+    A.d.nb = nullptr;
+    if (reach <= 0xffffu && !wide_neighbours()) {
+        CK(A.near.ensure(nm * p->nd * sizeof(uint2)));
+        A.d.near = A.near.as<uint2>();
+    } else {
+        CK(A.nb.ensure(nm * p->nd * sizeof(int4)));
+        A.d.nb = A.nb.as<int4>();
     }
-    CK(A.buf[0].ensure((size_t)N * p->ns * 4));
-    CK(A.buf[1].ensure((size_t)N * p->ns * 4));
-    CK(cudaMemsetAsync(A.buf[1].p, 0, (size_t)N * p->ns * 4, s));
+    CK(A.face.ensure(nm * p->nd * sizeof(float2)));
+    CK(A.cflags.ensure(nm * 4));
+    A.d.face = A.face.as<float2>();
+    A.d.cflags = A.cflags.as<uint32_t>();
+    CK(A.buf[0].ensure((size_t)A.d.ms * p->ns * 4));
+    CK(A.buf[1].ensure((size_t)A.d.ms * p->ns * 4));
     A.d.buf[0] = A.buf[0].as<float>();
     A.d.buf[1] = A.buf[1].as<float>();
     A.d.ladder = nullptr;  // allocated by prt_adr_run
-    CK(adr_launch_setup(A.d_mat, A.d_vel, *p, A.d, s));
-    ctx->launches += p->nd + 1;
+    CK(adr_launch_setup(A.d_vel, *p, A.d, map, s));
+    ctx->launches += A.d.nm > 0 ? 4 : 0;
     CK(cudaStreamSynchronize(s));
     A.begun = true;
     A.ran = false;
     return PRT_OK;
+}
+
+static size_t slot_bytes(const AdrState& A) { return (size_t)A.d.nm * A.p.ns * 4; }
+
+// The state in buffer `buf` to ladder slot `slot`.
+static cudaError_t copy_rows(const AdrState& A, const DevBuf& buf, int slot, cudaStream_t s) {
+    return adr_launch_rows(A.d, buf.as<float>(),
+                           A.ladder.as<float>() + (size_t)A.d.nm * A.p.ns * slot, s);
 }
 
 // Transport time loop in three parts (see flow_setup): the ladder and the
@@ -626,7 +653,6 @@ int prt::adr_run_setup(prt_ctx* ctx, const prt_adr_run_params* rp, long long pau
         return fail(ctx, PRT_E_INVALID, "bad run parameters");
     CK(cudaSetDevice(ctx->device));
     cudaStream_t s = ctx->stream;
-    const long long N = A.d.g.n;
     const int ns = A.p.ns;
     const long long limit = rp->limit;
     // the snapshot ladder (prtlb_3d.py:1496-1498): record at n >= nxt,
@@ -643,10 +669,8 @@ int prt::adr_run_setup(prt_ctx* ctx, const prt_adr_run_params* rp, long long pau
     }
     const int K = (int)A.sched.size();
     A.nslots = K + 2;  // step 0, the schedule, and a final record
-    const size_t slot_bytes = (size_t)N * ns * 4;
-    CK(A.ladder.ensure(slot_bytes * A.nslots));
-    CK(cudaMemsetAsync(A.ladder.p, 0, slot_bytes * A.nslots, s));
-    CK(cudaMemcpyAsync(A.ladder.p, A.buf[0].p, slot_bytes, cudaMemcpyDeviceToDevice, s));
+    CK(A.ladder.ensure(slot_bytes(A) * A.nslots));
+    CK(copy_rows(A, A.buf[0], 0, s));
     std::vector<int> sos((size_t)limit + 1, -1);
     for (int k = 0; k < K; ++k) sos[(size_t)A.sched[k]] = k + 1;
     CK(A.slot_of_step.ensure(sos.size() * 4));
@@ -687,7 +711,6 @@ int prt::adr_run_finish(prt_ctx* ctx, prt_adr_result* res) {
     CK(cudaStreamSynchronize(s));
     const long long n = cur.n_base;
     const int K = (int)A.sched.size();
-    const size_t slot_bytes = (size_t)A.d.g.n * A.p.ns * 4;
     // keep_steps = [0] + ladder steps <= n, plus n itself when not one of them
     A.keep_steps.clear();
     A.slot_of_index.clear();
@@ -698,8 +721,7 @@ int prt::adr_run_finish(prt_ctx* ctx, prt_adr_result* res) {
         A.slot_of_index.push_back(k + 1);
     }
     if (A.keep_steps.back() != n) {
-        CK(cudaMemcpyAsync(A.ladder.as<char>() + slot_bytes * (K + 1), A.buf[n & 1].p, slot_bytes,
-                           cudaMemcpyDeviceToDevice, s));
+        CK(copy_rows(A, A.buf[n & 1], K + 1, s));
         A.keep_steps.push_back(n);
         A.slot_of_index.push_back(K + 1);
     }
@@ -723,14 +745,11 @@ static cudaError_t adr_emit(prt_ctx* ctx, cudaGraphConditionalHandle h, int use)
     AdrState& A = ctx->adr;
     AdrCtrl* dctrl = A.ctrl.as<AdrCtrl>();
     float* dmeans = A.means.as<float>();
-    const float** srcp = (const float**)A.src_slot.p;
     for (int k = 0; k < A.rp.check; ++k) {
         cudaError_t e = adr_launch_step(A.d, A.p, dctrl, k, ctx->stream);
         if (e != cudaSuccess) return e;
     }
-    cudaError_t e = adr_launch_chunk_means(A.d, dctrl, srcp, dmeans, ctx->stream);
-    if (e != cudaSuccess) return e;
-    return adr_launch_stop(A.d, dctrl, dmeans, h, use, ctx->stream);
+    return adr_launch_chunk_end(A.d, dctrl, dmeans, h, use, ctx->stream);
 }
 
 // Everything the transport loop graph bakes into its nodes: the device
@@ -738,7 +757,7 @@ static cudaError_t adr_emit(prt_ctx* ctx, cudaGraphConditionalHandle h, int use)
 // the buffers of the means and the stop rule, and the launch attribute.
 static std::vector<unsigned char> adr_graph_key(prt_ctx* ctx) {
     AdrState& A = ctx->adr;
-    const void* ptrs[3] = {A.means.p, A.src_slot.p, A.ctrl.p};
+    const void* ptrs[2] = {A.means.p, A.ctrl.p};
     const int ints[2] = {A.rp.check, pdl_key()};
     std::vector<unsigned char> k(sizeof(AdrDev) + sizeof(prt_adr_params) + sizeof(ptrs) +
                                  sizeof(ints));
@@ -801,7 +820,7 @@ extern "C" int prt_adr_run(prt_ctx* ctx, const prt_adr_run_params* rp, prt_progr
     auto emit = [&](cudaGraphConditionalHandle h, int use) -> cudaError_t {
         return adr_emit(ctx, h, use);
     };
-    const int per_chunk = check + 3 + (D.tree.nleaf > 0 ? 1 : 0);
+    const int per_chunk = check + 1 + (D.tree.nleaf > 0 ? 1 : 0);
     std::vector<ProgressRec> logbuf;
     int delivered = 0;
     AdrCtrl cur;
@@ -875,7 +894,7 @@ static int slot_ptr(prt_ctx* ctx, int32_t slot, const float** out) {
     if (!A.ran) return fail(ctx, PRT_E_STATE, "no finished run");
     if (slot < 0 || slot >= (int)A.slot_of_index.size())
         return fail(ctx, PRT_E_INVALID, "snapshot index out of range");
-    *out = A.ladder.as<float>() + (size_t)A.slot_of_index[slot] * A.d.g.n * A.p.ns;
+    *out = A.ladder.as<float>() + (size_t)A.slot_of_index[slot] * A.d.nm * A.p.ns;
     return PRT_OK;
 }
 
@@ -886,7 +905,10 @@ extern "C" int prt_adr_fetch(prt_ctx* ctx, int32_t slot, float* out) {
     if (rc) return rc;
     CK(cudaSetDevice(ctx->device));
     const size_t bytes = (size_t)ctx->adr.d.g.n * ctx->adr.p.ns * 4;
-    CK(cudaMemcpyAsync(out, src, bytes, cudaMemcpyDeviceToHost, ctx->stream));
+    CK(ctx->adr.dense.ensure(bytes));
+    CK(adr_launch_expand(ctx->adr.d, src, ctx->adr.dense.as<float>(), ctx->stream));
+    ctx->launches += 1;
+    CK(cudaMemcpyAsync(out, ctx->adr.dense.p, bytes, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
@@ -897,8 +919,8 @@ extern "C" int prt_adr_fetch_dev(prt_ctx* ctx, int32_t slot, float* d_out) {
     int rc = slot_ptr(ctx, slot, &src);
     if (rc) return rc;
     CK(cudaSetDevice(ctx->device));
-    const size_t bytes = (size_t)ctx->adr.d.g.n * ctx->adr.p.ns * 4;
-    CK(cudaMemcpyAsync(d_out, src, bytes, cudaMemcpyDeviceToDevice, ctx->stream));
+    CK(adr_launch_expand(ctx->adr.d, src, d_out, ctx->stream));
+    ctx->launches += 1;
     CK(cudaStreamSynchronize(ctx->stream));
     return PRT_OK;
 }
@@ -910,8 +932,7 @@ extern "C" int prt_adr_means(prt_ctx* ctx, int32_t slot, float* means) {
     if (slot < 0 || slot >= (int)A.slot_of_index.size())
         return fail(ctx, PRT_E_INVALID, "snapshot index out of range");
     CK(cudaSetDevice(ctx->device));
-    CK(adr_launch_means(A.d, A.ctrl.as<AdrCtrl>(), A.slot_of_index[slot], A.means.as<float>(),
-                        ctx->stream));
+    CK(adr_launch_means(A.d, A.slot_of_index[slot], A.means.as<float>(), ctx->stream));
     ctx->launches += 2;
     CK(cudaMemcpyAsync(means, A.means.p, (size_t)A.p.ns * 4, cudaMemcpyDeviceToHost, ctx->stream));
     CK(cudaStreamSynchronize(ctx->stream));

@@ -15,12 +15,10 @@
 #include "prt_internal.h"
 
 namespace prt {
-cudaError_t adr_launch_chunk_means(const AdrDev& d, AdrCtrl* ctrl, const float** src_slot,
-                                   float* means_out, cudaStream_t s);
 cudaError_t adr_launch_flags(const uint8_t* mat, const Grid& g, int nd, int pore, int bfc,
                              uint32_t* flags, uint8_t* mflag, cudaStream_t s);
 cudaError_t adr_launch_vel_stats(const float* vel, const AdrDev& d, float* tmp, float* means,
-                                 unsigned* vmax_bits, unsigned long long* nbf, cudaStream_t s);
+                                 unsigned* vmax_bits, unsigned long long* nbf, int* n0, cudaStream_t s);
 
 struct DevBuf {
     void* p = nullptr;
@@ -104,9 +102,9 @@ struct AdrState {
     bool ran = false;
     prt_adr_params p{};
     AdrDev d{};
-    DevBuf mat, vel, flags, mflag, face[3], buf[2], ladder, slot_of_step, idx, cnt, total;
+    DevBuf mat, vel, flags, cflags, mflag, near, nb, face, buf[2], ladder, dense, slot_of_step, idx, cnt, total;
     DevBuf tree_leaf_start, tree_leaf_len, tree_inner_l, tree_inner_r, tree_level_off, tree_vals;
-    DevBuf means, src_slot, ctrl, log;
+    DevBuf means, ctrl, log;
     // for the batch engine: blk_leaf[b] = the first leaf starting at or after
     // solute voxel kBatchAdrBlock * b (b = 0 .. nbk), see AdrJob
     DevBuf blk_leaf;
@@ -130,10 +128,10 @@ struct AdrState {
     // and initialises what it reads), so back-to-back solves on one context
     // do not pay cudaFree / cudaMalloc each time; larger ones are freed.
     void release(size_t keep_bytes = 0) {
-        DevBuf* all[] = {&mat, &vel, &flags, &mflag, &face[0], &face[1], &face[2], &buf[0], &buf[1],
-                         &ladder, &slot_of_step, &idx, &cnt, &total, &tree_leaf_start,
+        DevBuf* all[] = {&mat, &vel, &flags, &cflags, &mflag, &near, &nb, &face, &buf[0], &buf[1], &ladder, &dense,
+                         &slot_of_step, &idx, &cnt, &total, &tree_leaf_start,
                          &tree_leaf_len, &tree_inner_l, &tree_inner_r, &tree_level_off, &tree_vals,
-                         &means, &src_slot, &ctrl, &log, &tmp, &vstats, &blk_leaf};
+                         &means, &ctrl, &log, &tmp, &vstats, &blk_leaf};
         bool freed = false;
         for (DevBuf* b : all)
             if (b->bytes > keep_bytes) {

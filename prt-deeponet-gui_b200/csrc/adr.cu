@@ -20,6 +20,15 @@ constexpr int kAdrThreads = 128;
 
 // One transport step n = n_base + kstep + 1 over every solute voxel (one
 // thread each; rock voxels are not in the state).
+//
+// Bound by instruction issue (about 370 warp instructions per 32 voxels with
+// one Monod chemical) up to the L2's size, by DRAM beyond it.  Neighbour
+// distances instead of flags and positions on dense grids, one set of
+// differences per axis for diffusion and both limiters, no division for a cap
+// that is certainly not met: 64^3 / 128^3 / 192^3 Monod 3.96 / 16.6 / 67.4 ->
+// 3.3 / 11.8 / 54.1 us a step, four chemicals 7.8 / 45.5 -> 4.9 / 26.9, with
+// biofilm 10.3 / 65.5 -> 5.7 / 34.1.  Places instead of 16-bit distances take
+// 24 B more a voxel: 3.4 / 12.4 / 60.7.
 // Launched with programmatic stream serialisation: what does not change
 // during a run (the neighbours' places and the face velocities) is read while
 // the previous step drains; the control block and the concentrations only
@@ -326,12 +335,13 @@ static long long resident_blocks(K kern) {
     return (long long)per_sm * sms;
 }
 
-// Steps go out with programmatic stream serialisation.  One whose blocks
-// exceed one resident wave lets the next step launch at its start (128^3:
-// 16.2 -> 15.3 us per step, four chemicals 44.5 -> 40.5); one that fits in
-// one wave only after its stores (pdl_late), because released at the start
-// the next step's blocks, all resident early, slowed the running one (64^3:
-// 4.32 -> 5.56 us) where released at the end they cut the step to 3.66 us.
+// Steps go out with programmatic stream serialisation.  A step whose blocks
+// exceed one resident wave lets the next step launch at its start (128^3
+// Monod: 11.8 us a step against 12.6 at the end), and so does one that fills
+// at most half a wave, because the next step's blocks then find room beside
+// it (24^3: 2.35 -> 2.02, 40^3 2.43 -> 2.11, 128^2 first order 2.36 -> 2.05);
+// between the two only after its stores (pdl_late), or the next step's blocks
+// would slow the running one (64^3, four chemicals: 4.85 against 5.55).
 // PRT_PDL=0 launches every step plainly.
 template <int ND, int NS>
 static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl, int k,
@@ -350,7 +360,8 @@ static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctr
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    const int late = pdl_late(nb <= resident_blocks(kern)) ? 1 : 0;
+    const long long resident = resident_blocks(kern);
+    const int late = pdl_late(nb <= resident && 2 * nb > resident) ? 1 : 0;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, d, p, ctrl, k, late);
 }

@@ -79,6 +79,14 @@ __device__ __forceinline__ int stride(const Grid& g, int a) {
     return a == 0 ? g.ny * g.nz : (a == 1 ? g.nz : 1);
 }
 
+// p + B * n bytes as one multiply-add (B may be negative).
+template <int B>
+__device__ __forceinline__ const float* apart(const float* p, int n) {
+    const float* q;
+    asm("mad.wide.s32 %0, %1, %2, %3;" : "=l"(q) : "r"(n), "n"(B), "l"(p));
+    return q;
+}
+
 // A load through the read-only path (the buffer is not written by this
 // launch), issued where it stands; and the same only where u >= 0, or only
 // where it is not, else 0: the far value that the upwind side does not need
@@ -108,8 +116,8 @@ __device__ __forceinline__ float ld_if_down(const float* p, float u) {
 }
 
 // What one transport step needs of solute voxel k that does not change during
-// a run: per axis its neighbours' places (x, y, z, w = far low, low, high, far
-// high) and its low and high face velocity, and its flags where the run
+// a run: per axis the distances to its neighbours (x, y down to the far low and
+// the low, z, w up to the high and the far high) and its low and high face velocity, and its flags where the run
 // reads them.  WIDE: from AdrDev::nb instead of AdrDev::near.
 template <int ND>
 struct VoxelSetup {
@@ -126,11 +134,11 @@ __device__ __forceinline__ VoxelSetup<ND> voxel_setup(const AdrDev& d, const prt
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
         if constexpr (WIDE) {
-            s.nb[i] = __ldg(d.nb + (i * nm + k));
+            const int4 q = __ldg(d.nb + (i * nm + k));
+            s.nb[i] = make_int4((int)k - q.x, (int)k - q.y, q.z - (int)k, q.w - (int)k);
         } else {
             const uint2 q = __ldg(d.near + (i * nm + k));
-            s.nb[i] = make_int4((int)(k - (q.x & 0xffffu)), (int)(k - (q.x >> 16)),
-                                (int)(k + (q.y & 0xffffu)), (int)(k + (q.y >> 16)));
+            s.nb[i] = make_int4(q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16);
         }
         s.fc[i] = __ldg(d.face + (i * nm + k));
     }
@@ -146,16 +154,16 @@ __device__ __forceinline__ VoxelSetup<ND> voxel_setup(const AdrDev& d, const prt
 // face takes the pore diffusivity.  Every transport kernel calls this, so
 // they compute the same function bit for bit.
 template <int ND, bool BF>
-__device__ __forceinline__ float transport_one(const float* __restrict__ Cj,
+__device__ __forceinline__ float transport_one(const float* __restrict__ Ck,
                                                const VoxelSetup<ND>& s, float Cc,
                                                const float (&dj)[3]) {
     float m2[ND], m1[ND], p1[ND], p2[ND];
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        m1[i] = ld_early(Cj + (unsigned)s.nb[i].y);
-        p1[i] = ld_early(Cj + (unsigned)s.nb[i].z);
-        m2[i] = ld_if_up(Cj + (unsigned)s.nb[i].x, s.fc[i].x);
-        p2[i] = ld_if_down(Cj + (unsigned)s.nb[i].w, s.fc[i].y);
+        m1[i] = ld_early(apart<-4>(Ck, s.nb[i].y));
+        p1[i] = ld_early(apart<4>(Ck, s.nb[i].z));
+        m2[i] = ld_if_up(apart<-4>(Ck, s.nb[i].x), s.fc[i].x);
+        p2[i] = ld_if_down(apart<4>(Ck, s.nb[i].w), s.fc[i].y);
     }
     float out = 0.f;
     float divu = 0.f;
@@ -188,6 +196,24 @@ __device__ __forceinline__ float transport_one(const float* __restrict__ Cj,
     return out + Cc * divu;
 }
 
+// Whether r <= 1/2 (c / t) rounded as the reference rounds it is certain without
+// the division (t > 0).  r t <= 0.49 c with c not tiny: the two roundings of
+// the products and the two of the reference's cap move either side by less
+// than 1e-6 of it, and the least product that passes, 4.9e-31, is far above
+// the subnormal range.  r <= 0 <= c: the cap is at least +0.  A NaN or an
+// infinite r fails both.
+__device__ __forceinline__ bool below_half(float r, float c, float t) {
+    return (r * t <= 0.49f * c && c >= 1e-30f) || (r <= 0.f && c >= 0.f);
+}
+
+// a / b with the zero numerators of a front that has not arrived (b > 0: +0)
+// kept out of the division's path for special operands.
+__device__ __forceinline__ float ratio(float a, float b) {
+    const bool none = a == 0.f && b > 0.f;
+    const float q = (none ? b : a) / b;
+    return none ? a : q;
+}
+
 // The reaction terms (rate_biotic, rate_abiotic, reaction: prtlb_3d.py:1224-1367)
 // at one voxel, plus the reversible-sorption exchange (no reference counterpart).
 template <int NS>
@@ -197,14 +223,19 @@ __device__ __forceinline__ void reaction(const float (&C)[NS], float surf,
     for (int j = 0; j < NS; ++j) dC[j] = 0.f;
     float R = 0.f;
     if (p.biotic_on) {
-        R = p.ks_donor_pos ? (p.k * C[0]) / (p.ks_donor + C[0]) : p.k * C[0];
-        if (NS > 1) R = R * (p.ks_acceptor_pos ? C[NS > 1 ? 1 : 0] / (p.ks_acceptor + C[NS > 1 ? 1 : 0])
-                                               : C[NS > 1 ? 1 : 0]);
+        R = p.ks_donor_pos ? ratio(p.k * C[0], p.ks_donor + C[0]) : p.k * C[0];
+        if (NS > 1) R = R * (p.ks_acceptor_pos
+                                 ? ratio(C[NS > 1 ? 1 : 0], p.ks_acceptor + C[NS > 1 ? 1 : 0])
+                                 : C[NS > 1 ? 1 : 0]);
         if (NS > 3 && p.coupled) R = (R * C[NS > 3 ? 3 : 0]) / p.c3_init;
         // caps: R <= 1/2 min(C0 / dt, C1 / (alpha dt))
-        float lim = C[0] / p.dt;
-        if (NS > 1 && p.alpha_cap) lim = np_min(lim, C[NS > 1 ? 1 : 0] / p.alpha_dt);
-        R = np_min(R, 0.5f * lim);
+        const bool c1 = NS > 1 && p.alpha_cap;
+        if (!(below_half(R, C[0], p.dt) &&
+              (!c1 || (p.alpha_dt > 0.f && below_half(R, C[NS > 1 ? 1 : 0], p.alpha_dt))))) {
+            float lim = C[0] / p.dt;
+            if (c1) lim = np_min(lim, C[NS > 1 ? 1 : 0] / p.alpha_dt);
+            R = np_min(R, 0.5f * lim);
+        }
     }
     float Ra = 0.f;
     if (p.abio_on) {
@@ -213,7 +244,7 @@ __device__ __forceinline__ void reaction(const float (&C)[NS], float surf,
         for (int j = 0; j < NS; ++j)
             if (j == p.j_ab) cj = C[j];
         Ra = p.surface_only ? (p.ka * cj) * surf : p.ka * cj;
-        Ra = np_min(Ra, (0.5f * cj) / p.dt);
+        if (!below_half(Ra, cj, p.dt)) Ra = np_min(Ra, (0.5f * cj) / p.dt);
     }
     if (p.biotic_on) {
         dC[0] = -R;
@@ -241,8 +272,10 @@ __device__ __forceinline__ void reaction(const float (&C)[NS], float surf,
             if (j == p.j_s) s = C[j];
         }
         float r = p.k_sorp * (c - s * p.inv_kd_sorp);
-        r = np_min(r, (0.5f * c) / p.dt);
-        r = np_max(r, -((0.5f * s) / p.dt));
+        if (!(below_half(r, c, p.dt) && below_half(-r, s, p.dt))) {
+            r = np_min(r, (0.5f * c) / p.dt);
+            r = np_max(r, -((0.5f * s) / p.dt));
+        }
 #pragma unroll
         for (int j = 0; j < NS; ++j) {
             if (j == p.j_c) dC[j] = dC[j] - r;
@@ -292,18 +325,18 @@ __device__ __forceinline__ void adr_voxel_step(const AdrDev& d, const prt_adr_pa
                                                long long n, unsigned k,
                                                const VoxelSetup<ND>& s) {
     const unsigned ms = d.ms;
-    const float* __restrict__ Cin = d.buf[(n - 1) & 1];
+    const float* __restrict__ Ck = d.buf[(n - 1) & 1] + k;
     float* __restrict__ Cout = d.buf[n & 1];
     float C[NS];
 #pragma unroll
-    for (int j = 0; j < NS; ++j) C[j] = Cin[j * ms + k];
+    for (int j = 0; j < NS; ++j) C[j] = Ck[j * ms];
     float T[NS];
 #pragma unroll
     for (int j = 0; j < NS; ++j) {
         T[j] = 0.f;
         if ((p.moving_mask >> j) & 1u) {
             const float dj[3] = {p.dface[j][0], p.dface[j][1], p.dface[j][2]};
-            T[j] = transport_one<ND, BF>(Cin + j * ms, s, C[j], dj);
+            T[j] = transport_one<ND, BF>(Ck + j * ms, s, C[j], dj);
         }
     }
     float cn[NS];

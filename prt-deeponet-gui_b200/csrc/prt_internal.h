@@ -67,9 +67,10 @@ inline bool pdl_enabled() {
 // Where a single-solve step kernel lets the next step launch
 // (griddepcontrol.launch_dependents): after its own stores when its grid
 // fits in one resident wave -- the next step's blocks then arrive as this
-// one drains instead of sitting beside it (64^3: flow 4.60 -> 4.09 us per
-// iteration, transport 4.11 -> 3.66 us per step) -- and at its start when
-// it does not, so later waves overlap the next step's set-up.
+// one drains instead of sitting beside it (64^3 float32 flow: 4.3 against 4.7
+// us per iteration, 48^3 float64 3.6 against 5.6) -- and at its start when
+// it does not, so later waves overlap the next step's set-up (128^3 float32
+// 26.8 against 27.2).  The transport step draws the line elsewhere (adr.cu).
 // PRT_PDL_LATE=all / none puts it at the end / the start for every grid.
 inline bool pdl_late(bool one_wave) {
     const char* v = std::getenv("PRT_PDL_LATE");

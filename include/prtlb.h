@@ -304,8 +304,9 @@ int prt_flow_finish(prt_ctx* ctx, float* vel_out, prt_flow_info* info);
  * own flow solve (after prt_flow_finish). */
 int prt_adr_stage_flow(prt_ctx* ctx, const prt_adr_geom* geom, prt_adr_stats* stats);
 
-/* Frees the flow lattices and maps of ctx (keeps the material grid and the
- * field staged for transport).  A context in a batch may call it once its
+/* Ends the flow phase of ctx: its lattice, maps and tables are freed, those of
+ * at most 32 MiB stay for the context's next solve (the material grid and the
+ * field staged for transport are kept).  A context in a batch may call it once its
  * flow solve is finished (prt_flow_finish). */
 int prt_flow_release(prt_ctx* ctx);
 

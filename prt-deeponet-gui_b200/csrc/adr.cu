@@ -227,16 +227,36 @@ __global__ void count_kernel(const uint8_t* __restrict__ mflag, long long n, int
     v = __syncthreads_count(v);
     if (threadIdx.x == 0) cnt[blockIdx.x] = v;
 }
-__global__ void scan_counts_kernel(int* __restrict__ cnt, int nb, long long* __restrict__ total) {
-    // one thread: the block counts are few (n / 1024)
-    if (threadIdx.x != 0 || blockIdx.x != 0) return;
-    long long acc = 0;
-    for (int i = 0; i < nb; ++i) {
-        const int v = cnt[i];
-        cnt[i] = (int)acc;
-        acc += v;
+// The counts to exclusive sums, in place, and their total; one block.  (One
+// thread walking them took 0.4 us a count: 0.8 ms at 128^3, 2.8 ms at 192^3.)
+__global__ void __launch_bounds__(kScanBlock)
+    scan_counts_kernel(int* __restrict__ cnt, int nb, long long* __restrict__ total) {
+    __shared__ int warp_sum[32];
+    const int lane = threadIdx.x & 31, w = threadIdx.x >> 5;
+    int carry = 0;
+    for (int at = 0; at < nb; at += kScanBlock) {
+        const int i = at + threadIdx.x;
+        const int v = i < nb ? cnt[i] : 0;
+        int s = v;
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, s, o);
+            if (lane >= o) s += t;
+        }
+        if (lane == 31) warp_sum[w] = s;
+        __syncthreads();
+        int ws = warp_sum[lane];
+#pragma unroll
+        for (int o = 1; o < 32; o <<= 1) {
+            const int t = __shfl_up_sync(0xffffffffu, ws, o);
+            if (lane >= o) ws += t;
+        }
+        const int before = w ? __shfl_sync(0xffffffffu, ws, w - 1) : 0;
+        if (i < nb) cnt[i] = carry + before + s - v;
+        carry += __shfl_sync(0xffffffffu, ws, 31);
+        __syncthreads();
     }
-    *total = acc;
+    if (threadIdx.x == 0) *total = carry;
 }
 __global__ void scatter_kernel(const uint8_t* __restrict__ mflag, long long n,
                                const int* __restrict__ off, int* __restrict__ idx) {
@@ -506,12 +526,18 @@ cudaError_t adr_launch_expand(const AdrDev& d, const float* rows, float* out, cu
     return cudaGetLastError();
 }
 
-cudaError_t adr_launch_compact(const uint8_t* mflag, long long n, int* cnt, long long* total,
-                               int* idx, cudaStream_t s) {
+cudaError_t adr_launch_count(const uint8_t* mflag, long long n, int* cnt, long long* total,
+                             cudaStream_t s) {
     const int nb = (int)((n + kScanBlock - 1) / kScanBlock);
     count_kernel<<<nb, kScanBlock, 0, s>>>(mflag, n, cnt);
-    scan_counts_kernel<<<1, 32, 0, s>>>(cnt, nb, total);
-    if (idx) scatter_kernel<<<nb, kScanBlock, 0, s>>>(mflag, n, cnt, idx);
+    scan_counts_kernel<<<1, kScanBlock, 0, s>>>(cnt, nb, total);
+    return cudaGetLastError();
+}
+
+cudaError_t adr_launch_scatter(const uint8_t* mflag, long long n, const int* cnt, int* idx,
+                               cudaStream_t s) {
+    const int nb = (int)((n + kScanBlock - 1) / kScanBlock);
+    scatter_kernel<<<nb, kScanBlock, 0, s>>>(mflag, n, cnt, idx);
     return cudaGetLastError();
 }
 

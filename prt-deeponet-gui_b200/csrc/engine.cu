@@ -407,7 +407,7 @@ extern "C" int prt_flow_start(prt_ctx* ctx, const uint8_t* mat, const prt_flow_p
     FlowState& F = ctx->flow;
     CK(F.mat.ensure((size_t)g.n));
     CK(F.vel.ensure((size_t)g.n * 3 * sizeof(float)));
-    CK(cudaMemcpyAsync(F.mat.p, mat, (size_t)g.n, cudaMemcpyHostToDevice, ctx->stream));
+    CK(copy_in(ctx, F.mat.p, mat, (size_t)g.n));
     ctx->flow_armed = false;
     int rc = flow_setup(ctx, F.mat.as<uint8_t>(), p, F.vel.as<float>());
     if (rc != PRT_OK) return rc;
@@ -437,11 +437,7 @@ extern "C" int prt_flow_finish(prt_ctx* ctx, float* vel_out, prt_flow_info* info
     if (rc != PRT_OK) return rc;
     ctx->flow_armed = false;
     ctx->timing[1] = (double)res.iters;
-    if (vel_out) {
-        CK(cudaMemcpyAsync(vel_out, F.d_vel, (size_t)F.g.n * 3 * sizeof(float),
-                           cudaMemcpyDeviceToHost, ctx->stream));
-        CK(cudaStreamSynchronize(ctx->stream));
-    }
+    if (vel_out) CK(copy_out(ctx, vel_out, F.d_vel, (size_t)F.g.n * 3 * sizeof(float)));
     return PRT_OK;
 }
 
@@ -457,6 +453,9 @@ extern "C" int prt_adr_stage_flow(prt_ctx* ctx, const prt_adr_geom* geom, prt_ad
     return prt_adr_stage_dev(ctx, F.d_mat, F.d_vel, geom, stats);
 }
 
+// Flow buffers up to this size outlive prt_flow_release on their context.
+constexpr size_t kFlowKeepBytes = size_t(32) << 20;
+
 extern "C" int prt_flow_release(prt_ctx* ctx) {
     if (!ctx) return PRT_E_INVALID;
     // a context in a batch may drop its lattices once its flow solve is
@@ -465,7 +464,7 @@ extern "C" int prt_flow_release(prt_ctx* ctx) {
         return fail(ctx, PRT_E_STATE, "the context's flow solve is in a batch");
     CK(cudaSetDevice(ctx->device));
     CK(cudaStreamSynchronize(ctx->stream));
-    ctx->flow.release_lattices();
+    ctx->flow.release_lattices(kFlowKeepBytes);
     ctx->flow_armed = false;
     return PRT_OK;
 }

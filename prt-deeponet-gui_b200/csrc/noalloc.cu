@@ -147,13 +147,13 @@ int noalloc_solve(const uint8_t* d_mat, const prt_flow_params* p, float* d_vel_o
     // pore-only layout: flags, count, pore list, voxel -> slot map
     launched = true;
     NCK(flow_launch_flags(d_mat, g.n, 2, flag, s));
-    NCK(adr_launch_compact(flag, g.n, cnt, count, nullptr, s));
+    NCK(adr_launch_count(flag, g.n, cnt, count, s));
     long long nfluid = 0;
     NCK(cudaMemcpyAsync(&nfluid, count, sizeof(nfluid), cudaMemcpyDeviceToHost, s));
     NCK(cudaStreamSynchronize(s));
     if ((long long)2 * Q * nfluid >= (1ll << 31))
         return fail(PRT_E_INVALID, "more pore voxels than the 32-bit lattice offsets hold");
-    NCK(adr_launch_compact(flag, g.n, cnt, count, cells, s));
+    NCK(adr_launch_scatter(flag, g.n, cnt, cells, s));
     NCK(cudaMemsetAsync(imap, 0xff, (size_t)g.n * 4, s));
     FlowMap fm;
     fm.ys = coord_bits(g.nz);

@@ -214,8 +214,8 @@ extern "C" int prt_physics_stage(prt_ctx* ctx, const float* out, const uint8_t* 
     const long long nf = (long long)n_t * ns * g.n;
     CK(P.out.ensure((size_t)nf * 4));
     CK(P.mat.ensure((size_t)g.n));
-    CK(cudaMemcpyAsync(P.out.p, out, (size_t)nf * 4, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(P.mat.p, mat, (size_t)g.n, cudaMemcpyHostToDevice, ctx->stream));
+    CK(copy_in(ctx, P.out.p, out, (size_t)nf * 4));
+    CK(copy_in(ctx, P.mat.p, mat, (size_t)g.n));
     P.staged_out = nf;
     P.staged_mat = g.n;
     return PRT_OK;

@@ -157,7 +157,7 @@ extern "C" int prt_label_materials(prt_ctx* ctx, const uint8_t* solid, int32_t n
     P.staged_mat = -1;
     uint8_t* d_solid = P.mat.as<uint8_t>();
     uint8_t* d_out = d_solid + g.n;
-    CK(cudaMemcpyAsync(d_solid, solid, (size_t)g.n, cudaMemcpyHostToDevice, s));
+    CK(copy_in(ctx, d_solid, solid, (size_t)g.n));
     WalkGrid w;
     w.g = g;
     w.dz = make_fastdiv((unsigned)g.nz);
@@ -168,8 +168,7 @@ extern "C" int prt_label_materials(prt_ctx* ctx, const uint8_t* solid, int32_t n
     label_materials_kernel<<<nb, kWalkThreads, 0, s>>>(d_solid, w, d_out);
     CK(cudaGetLastError());
     ctx->launches += 1;
-    CK(cudaMemcpyAsync(mat_out, d_out, (size_t)g.n, cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    CK(copy_out(ctx, mat_out, d_out, (size_t)g.n));
     return PRT_OK;
 }
 
@@ -197,7 +196,7 @@ extern "C" int prt_walk_from_plane(prt_ctx* ctx, const uint8_t* mat, int32_t nd,
     CK(P.steps.ensure((size_t)g.n * 4));
     CK(P.flags.ensure(kLevelsPerChunk * sizeof(int)));
     CK(P.counts.ensure(2 * sizeof(unsigned long long)));
-    CK(cudaMemcpyAsync(P.mat.p, mat, (size_t)g.n, cudaMemcpyHostToDevice, s));
+    CK(copy_in(ctx, P.mat.p, mat, (size_t)g.n));
     P.staged_mat = -1;  // the buffer now holds the walk's grid
     CK(cudaMemsetAsync(P.counts.p, 0, 2 * sizeof(unsigned long long), s));
     WalkGrid w;
@@ -230,9 +229,8 @@ extern "C" int prt_walk_from_plane(prt_ctx* ctx, const uint8_t* mat, int32_t nd,
     CK(cudaGetLastError());
     ctx->launches += 1;
     unsigned long long hc[2];
-    CK(cudaMemcpyAsync(steps_out, steps, (size_t)g.n * 4, cudaMemcpyDeviceToHost, s));
     CK(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s));
-    CK(cudaStreamSynchronize(s));
+    CK(copy_out(ctx, steps_out, steps, (size_t)g.n * 4));  // waits for both
     if (n_pore) *n_pore = (int64_t)hc[0];
     if (n_reached) *n_reached = (int64_t)hc[1];
     return PRT_OK;

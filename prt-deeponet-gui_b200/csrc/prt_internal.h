@@ -306,10 +306,12 @@ cudaError_t flow_launch_pack(int nd, const FlowMap& fm, const Grid& g, int* pack
 cudaError_t flow_launch_final_reduce(const double* partials, int nblocks, double* out,
                                      cudaStream_t s);
 int flow_blocks(long long n);
-// order-preserving compaction of a 0/1 flag array (adr.cu): with idx == NULL
-// only counts (cnt: one int per 1024 flags, *total on the device)
-cudaError_t adr_launch_compact(const uint8_t* mflag, long long n, int* cnt, long long* total,
-                               int* idx, cudaStream_t s);
+// order-preserving compaction of a 0/1 flag array (adr.cu): the block offsets
+// (cnt: one int per 1024 flags) and *total on the device, then the indices
+cudaError_t adr_launch_count(const uint8_t* mflag, long long n, int* cnt, long long* total,
+                             cudaStream_t s);
+cudaError_t adr_launch_scatter(const uint8_t* mflag, long long n, const int* cnt, int* idx,
+                               cudaStream_t s);
 
 // Sets what prt_last_error(NULL) returns on the calling thread (runtime.cu).
 void set_noctx_error(const char* msg);

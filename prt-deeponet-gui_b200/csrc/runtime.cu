@@ -57,6 +57,7 @@ extern "C" void prt_destroy(prt_ctx* c) {
     cudaStreamSynchronize(c->stream);
     c->adr.release();
     c->prep.release();
+    c->transfer.release();
     FlowState& f = c->flow;
     DevBuf* all[] = {&f.f,    &f.fluid, &f.partials, &f.ctrl, &f.out5, &f.count,
                      &f.mat,  &f.vel,   &f.flag,     &f.cnt,  &f.cells, &f.nbr, &f.link, &f.pack};
@@ -147,21 +148,19 @@ int prt::flow_setup(prt_ctx* ctx, const uint8_t* d_mat, const prt_flow_params* p
     CK(F.cnt.ensure((size_t)((g.n + 1023) / 1024) * 4));
     CK(F.count.ensure(sizeof(long long)));
     CK(flow_launch_flags(d_mat, g.n, 2, F.flag.as<uint8_t>(), s));
-    CK(adr_launch_compact(F.flag.as<uint8_t>(), g.n, F.cnt.as<int>(), F.count.as<long long>(),
-                          nullptr, s));
+    CK(adr_launch_count(F.flag.as<uint8_t>(), g.n, F.cnt.as<int>(), F.count.as<long long>(), s));
     long long nfluid = 0;
     CK(cudaMemcpyAsync(&nfluid, F.count.p, sizeof(nfluid), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     CK(F.cells.ensure((size_t)std::max(nfluid, 1ll) * 4));
     CK(F.fluid.ensure((size_t)g.n * 4));  // imap
-    CK(adr_launch_compact(F.flag.as<uint8_t>(), g.n, F.cnt.as<int>(), F.count.as<long long>(),
-                          F.cells.as<int>(), s));
+    CK(adr_launch_scatter(F.flag.as<uint8_t>(), g.n, F.cnt.as<int>(), F.cells.as<int>(), s));
     CK(cudaMemsetAsync(F.fluid.p, 0xff, (size_t)g.n * 4, s));
     F.fm.ys = coord_bits(g.nz);
     F.fm.xs = F.fm.ys + coord_bits(g.ny);
     CK(flow_launch_imap(F.cells.as<int>(), (int)nfluid, F.fluid.as<int>(), g, F.fm.ys, F.fm.xs,
                         s));
-    ctx->launches += 7;
+    ctx->launches += 5;
     if ((long long)2 * Q * nfluid >= (1ll << 31))
         return fail(ctx, PRT_E_INVALID,
                     "more pore voxels than the 32-bit lattice offsets hold (2 Q nf >= 2^31)");
@@ -387,12 +386,10 @@ extern "C" int prt_flow(prt_ctx* ctx, const uint8_t* mat, const prt_flow_params*
     FlowState& F = ctx->flow;
     CK(F.mat.ensure((size_t)g.n));
     CK(F.vel.ensure((size_t)g.n * 3 * sizeof(float)));
-    CK(cudaMemcpyAsync(F.mat.p, mat, (size_t)g.n, cudaMemcpyHostToDevice, ctx->stream));
+    CK(copy_in(ctx, F.mat.p, mat, (size_t)g.n));
     int rc = prt_flow_dev(ctx, F.mat.as<uint8_t>(), p, F.vel.as<float>(), info);
     if (rc != PRT_OK) return rc;
-    CK(cudaMemcpyAsync(vel_out, F.vel.p, (size_t)g.n * 3 * sizeof(float), cudaMemcpyDeviceToHost,
-                       ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copy_out(ctx, vel_out, F.vel.p, (size_t)g.n * 3 * sizeof(float)));
     return PRT_OK;
 }
 
@@ -454,15 +451,13 @@ extern "C" int prt_adr_stage_dev(prt_ctx* ctx, const uint8_t* d_mat, const float
     const int nbs = (int)((N + 1023) / 1024);
     CK(A.cnt.ensure((size_t)nbs * 4));
     CK(A.total.ensure(8));
-    CK(adr_launch_compact(A.mflag.as<uint8_t>(), N, A.cnt.as<int>(), A.total.as<long long>(),
-                          nullptr, s));
+    CK(adr_launch_count(A.mflag.as<uint8_t>(), N, A.cnt.as<int>(), A.total.as<long long>(), s));
     long long nm = 0;
     CK(cudaMemcpyAsync(&nm, A.total.p, 8, cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     CK(A.idx.ensure((size_t)std::max(nm, 1ll) * 4));
-    CK(adr_launch_compact(A.mflag.as<uint8_t>(), N, A.cnt.as<int>(), A.total.as<long long>(),
-                          A.idx.as<int>(), s));
-    ctx->launches += 6;
+    CK(adr_launch_scatter(A.mflag.as<uint8_t>(), N, A.cnt.as<int>(), A.idx.as<int>(), s));
+    ctx->launches += 4;
     A.d.idx = A.idx.as<int>();
     A.d.nm = nm;
     // numpy pairwise tree over nm values
@@ -569,8 +564,8 @@ extern "C" int prt_adr_stage(prt_ctx* ctx, const uint8_t* mat, const float* vel,
     AdrState& A = ctx->adr;
     CK(A.mat.ensure((size_t)g.n));
     CK(A.vel.ensure((size_t)g.n * 3 * 4));
-    CK(cudaMemcpyAsync(A.mat.p, mat, (size_t)g.n, cudaMemcpyHostToDevice, ctx->stream));
-    CK(cudaMemcpyAsync(A.vel.p, vel, (size_t)g.n * 3 * 4, cudaMemcpyHostToDevice, ctx->stream));
+    CK(copy_in(ctx, A.mat.p, mat, (size_t)g.n));
+    CK(copy_in(ctx, A.vel.p, vel, (size_t)g.n * 3 * 4));
     return prt_adr_stage_dev(ctx, A.mat.as<uint8_t>(), A.vel.as<float>(), geom, stats);
 }
 
@@ -908,8 +903,7 @@ extern "C" int prt_adr_fetch(prt_ctx* ctx, int32_t slot, float* out) {
     CK(ctx->adr.dense.ensure(bytes));
     CK(adr_launch_expand(ctx->adr.d, src, ctx->adr.dense.as<float>(), ctx->stream));
     ctx->launches += 1;
-    CK(cudaMemcpyAsync(out, ctx->adr.dense.p, bytes, cudaMemcpyDeviceToHost, ctx->stream));
-    CK(cudaStreamSynchronize(ctx->stream));
+    CK(copy_out(ctx, out, ctx->adr.dense.p, bytes));
     return PRT_OK;
 }
 

@@ -41,6 +41,17 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
+// Pinned chunks of a context for copies from and to pageable memory
+// (transfer.cu), one per copying thread; made at the first large copy.
+struct Transfer {
+    static constexpr int kWorkers = 8;
+    void* pin[kWorkers] = {};
+    cudaEvent_t ev[kWorkers] = {};
+    int n = 0;
+    cudaError_t ensure(int workers, size_t chunk);
+    void release();
+};
+
 struct GraphHolder {
     cudaGraph_t graph = nullptr;
     cudaGraphExec_t exec = nullptr;
@@ -89,11 +100,22 @@ struct FlowState {
     const uint8_t* d_mat = nullptr;  // material grid of the solve (borrowed)
     float* d_vel = nullptr;          // its output field (borrowed)
     bool field_ready = false;        // d_vel holds the final field
-    void release_lattices() {
+    // Ends the flow phase of a solve that goes on to its transport.  Device
+    // buffers of at most keep_bytes stay with the context for its next solve
+    // (set-up sizes them with ensure() and initialises what it reads), so a
+    // batch of small solves does not pay cudaFree / cudaMalloc for each.
+    void release_lattices(size_t keep_bytes) {
         DevBuf* all[] = {&f, &fluid, &partials, &count, &flag, &cnt, &cells, &nbr, &link, &pack};
-        for (DevBuf* b : all) b->release();
-        graph.release();
-        key = FlowKey();
+        bool freed = false;
+        for (DevBuf* b : all)
+            if (b->bytes > keep_bytes) {
+                b->release();
+                freed = true;
+            }
+        if (freed) {  // the cached loop graph holds device pointers
+            graph.release();
+            key = FlowKey();
+        }
     }
 };
 
@@ -176,6 +198,7 @@ struct prt_ctx {
     prt::FlowState flow;
     prt::AdrState adr;
     prt::PrepState prep;
+    prt::Transfer transfer;
     bool flow_armed = false;  // flow set up, its time loop not finished
     bool adr_armed = false;   // transport run set up, its time loop not finished
     prt_batch* batch = nullptr;  // the batch holding this context, if any
@@ -286,6 +309,11 @@ int adr_run_finish(prt_ctx* ctx, prt_adr_result* res);
 // context's stream without waiting (runtime.cu).
 int flow_loop_async(prt_ctx* ctx);
 int adr_loop_async(prt_ctx* ctx);
+// Copies on the context's stream between device memory and the caller's
+// (transfer.cu).  copy_out returns with the data in place; after copy_in the
+// caller's memory has been read.
+cudaError_t copy_out(prt_ctx* ctx, void* host, const void* dev, size_t bytes);
+cudaError_t copy_in(prt_ctx* ctx, void* dev, const void* host, size_t bytes);
 // Takes ctx out of its batch (engine.cu); used by prt_destroy.
 void batch_detach(prt_ctx* ctx);
 

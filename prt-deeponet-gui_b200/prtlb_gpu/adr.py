@@ -424,14 +424,14 @@ def outputs(ctx, S, n_t, n, ks, picked, steps, max_steps, info, da, da_abio, end
     L = _lib.lib()
     total = int(max(n, 1))
     repeated = n_t - len(set(picked))
-    out = np.zeros((n_t, S.ns) + S.shape, np.float32)
-    cache = {}
+    out = np.empty((n_t, S.ns) + S.shape, np.float32)
+    first = {}
     for j, i in enumerate(picked):
-        if i not in cache:
-            buf = np.empty((S.ns,) + S.shape, np.float32)
-            ctx.check(L.prt_adr_fetch(ctx.handle, int(i), buf.ctypes.data_as(ctypes.c_void_p)))
-            cache[i] = buf
-        out[j] = cache[i]
+        if i in first:
+            out[j] = out[first[i]]
+        else:
+            ctx.check(L.prt_adr_fetch(ctx.handle, int(i), out[j].ctypes.data_as(ctypes.c_void_p)))
+            first[i] = j
     if end:
         L.prt_adr_end(ctx.handle)
     t_norm = (ks[picked].astype(np.float32) / total).astype(np.float32)

@@ -33,10 +33,14 @@ def ladder_slots(limit, ratio):
     return k + 2
 
 
+# what prt_flow_release keeps of a flow phase at most: ten buffers of 32 MiB
+_FLOW_KEEP = 10 * (32 << 20)
+
+
 def footprint(req):
     """Estimated peak device bytes of one request: the flow phase (the
-    lattice, maps and tables) or the transport phase (state, faces, snapshot ladder),
-    whichever is larger, plus the material grid and field kept by both."""
+    lattice, maps and tables) or the transport phase (state, faces, snapshot
+    ladder), whichever is larger, plus the material grid and field kept by both."""
     mat = req.mat
     n = int(mat.size)
     nf = int(np.count_nonzero(mat == 2))
@@ -60,7 +64,8 @@ def footprint(req):
         limit = int(a["steps"]) if a["steps"] is not None else int(a["max_steps"])
         slots = ladder_slots(limit, float(a["ratio"]))
         adr = n * (4 + 1 + 4 + 12 + 8 * ns) + 4 * nf * 2 + 4 * n * ns * slots + 4 * (limit + 1)
-    return common + max(flow, adr) + (1 << 20)
+    # the flow's small buffers stay with the context during its transport
+    return common + max(flow, adr + min(flow, _FLOW_KEEP)) + (1 << 20)
 
 
 def device_memory(device=0):

@@ -63,33 +63,33 @@ struct D2Q9 {
 };
 
 // storage conversions ------------------------------------------------------
-// Pop<S>::H is the register type a stored population is held in; st() rounds
+// Pop<S>::H is the register type a stored population is held in; enc() rounds
 // the collision result to the storage type once.
 template <class S>
 struct Pop;
 template <>
 struct Pop<double> {
     using H = double;
-    __device__ static double ld(const double* p, float) { return *p; }
+    __device__ static double dec(double v, float) { return v; }
     template <class R>
-    __device__ static void st(double* p, R v, float) { *p = (double)v; }
+    __device__ static double enc(R v, float) { return (double)v; }
 };
 template <>
 struct Pop<float> {
     using H = float;
-    __device__ static float ld(const float* p, float) { return *p; }
+    __device__ static float dec(float v, float) { return v; }
     template <class R>
-    __device__ static void st(float* p, R v, float) { *p = (float)v; }
+    __device__ static float enc(R v, float) { return (float)v; }
 };
 template <>
 struct Pop<__half> {
     using H = float;
-    __device__ static float ld(const __half* p, float inv) { return __half2float(*p) * inv; }
+    __device__ static float dec(__half v, float inv) { return __half2float(v) * inv; }
     template <class R>
-    __device__ static void st(__half* p, R v, float scale) {
+    __device__ static __half enc(R v, float scale) {
         float s = (float)v * scale;
         s = fminf(fmaxf(s, -65504.f), 65504.f);
-        *p = __float2half_rn(s);
+        return __float2half_rn(s);
     }
 };
 
@@ -289,11 +289,11 @@ __device__ __forceinline__ void far_slots(const FlowMap& fm, const Grid& g, int 
 template <class L, class S>
 __device__ __forceinline__ void gather(const Lat<S>& lat, int k, const int (&far)[L::NP],
                                        float inv, typename Pop<S>::H (&h)[L::Q]) {
-    h[0] = Pop<S>::ld(lat.f + k, inv);
+    h[0] = Pop<S>::dec(lat.f[k], inv);
 #pragma unroll
     for (int p = 0; p < L::NP; ++p) {
-        h[L::pa(p)] = Pop<S>::ld(lat.at_own(L::pa(p), k), inv);
-        h[L::pb(p)] = Pop<S>::ld(lat.at_far(L::pa(p), far[p]), inv);
+        h[L::pa(p)] = Pop<S>::dec(*lat.at_own(L::pa(p), k), inv);
+        h[L::pb(p)] = Pop<S>::dec(*lat.at_far(L::pa(p), far[p]), inv);
     }
 }
 
@@ -384,26 +384,16 @@ __device__ __forceinline__ Moments<R, RA> moments(const HA& h, double half_g) {
 // shifted variables, written with J = rho u so that rho cancels in the
 // antisymmetric equilibrium (w rho 3 e.u = 3 w e.J) and rho u u = J J / rho in
 // the symmetric one.  The new population is h + delta with delta summed
-// first, so the stored result rounds once; f_a goes to the pair's far place
-// and f_b to its own (see Lat).
-template <class L, Fresh F, class S, class R, class RA, class HA>
-__device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const int (&far)[L::NP],
-                                              const HA& h, const Moments<R, RA>& m,
-                                              const LbParams& kc) {
-    Lat<S> lat = lat0;
-    int to[L::NP];
-    if (F == Fresh::base) asm volatile("" : "+l"(lat.f));
-    if (F == Fresh::index) asm volatile("" : "+r"(k));
-#pragma unroll
-    for (int p = 0; p < L::NP; ++p) {
-        to[p] = far[p];
-        if (F == Fresh::index) asm volatile("" : "+r"(to[p]));
-    }
+// first, so the stored result rounds once.  put(i, p, v) takes the new
+// population i, of pair p (-1: the rest population).
+template <class L, class R, class RA, class HA, class Put>
+__device__ __forceinline__ void collide(const HA& h, const Moments<R, RA>& m, const LbParams& kc,
+                                        Put put) {
     const R omp = R(kc.omp);
     const R inv_rho = R(m.inv_rho);
     const R heq0 = R(L::w(0)) * (m.drho - R(1.5) * m.jsq);
     const R h0 = R(h[0]);
-    Pop<S>::st(lat.f + k, h0 - omp * (h0 - heq0), kc.scale);
+    put(0, -1, h0 - omp * (h0 - heq0));
 #pragma unroll
     for (int p = 0; p < L::NP; ++p) {
         const int a = L::pa(p), b = L::pb(p);
@@ -421,9 +411,32 @@ __device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const i
         const RA dma = RA(kc.omm) * (RA(0.5) * (RA(h[a]) - RA(h[b])) - RA(3.0 * L::w(a)) * eJ);
         const R dm = R(dma);
         const R gp = R(kc.guo[p]);
-        Pop<S>::st(lat.at_far(a, to[p]), ha + ((gp - dp) - dm), kc.scale);
-        Pop<S>::st(lat.at_own(a, k), hb + ((dm - dp) - gp), kc.scale);
+        put(a, p, ha + ((gp - dp) - dm));
+        put(b, p, hb + ((dm - dp) - gp));
     }
+}
+
+// The collision of slot k with its results stored in the lattice: f_a to the
+// pair's far place and f_b to its own (see Lat).
+template <class L, Fresh F, class S, class R, class RA, class HA>
+__device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const int (&far)[L::NP],
+                                              const HA& h, const Moments<R, RA>& m,
+                                              const LbParams& kc) {
+    Lat<S> lat = lat0;
+    int to[L::NP];
+    if (F == Fresh::base) asm volatile("" : "+l"(lat.f));
+    if (F == Fresh::index) asm volatile("" : "+r"(k));
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        to[p] = far[p];
+        if (F == Fresh::index) asm volatile("" : "+r"(to[p]));
+    }
+    collide<L, R, RA>(h, m, kc, [&](int i, int p, R v) {
+        const S q = Pop<S>::enc(v, kc.scale);
+        if (p < 0) lat.f[k] = q;
+        else if (i == L::pa(p)) *lat.at_far(i, to[p]) = q;
+        else *lat.at_own(L::pa(p), k) = q;
+    });
 }
 
 // One pore voxel (slot k) of one LB iteration, its far places already found:

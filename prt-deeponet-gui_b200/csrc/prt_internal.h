@@ -283,6 +283,12 @@ cudaError_t flow_launch_step(int nd, int precision, bool odd, bool check, void* 
                              const FlowMap& fm, const Grid& g, const LbParams& lbp,
                              const FlowCtrl* ctrl, int kstep, double* partials,
                              cudaStream_t s);
+// The whole loop of the set-up solve as one cluster's kernel (cluster_flow.cu),
+// or cudaErrorNotSupported (nothing launched) when the lattice does not fit or
+// the device cannot place the cluster.
+cudaError_t flow_launch_cluster(int nd, int precision, void* f, const FlowMap& fm, const Grid& g,
+                                const LbParams& k, FlowCtrl* ctrl, double* partials, int nb,
+                                cudaStream_t s);
 cudaError_t flow_launch_check(FlowCtrl* ctrl, const double* partials, int nblocks,
                               cudaGraphConditionalHandle h, int use_handle, cudaStream_t s);
 cudaError_t flow_launch_moments(int nd, int precision, bool odd, const void* f,

@@ -301,6 +301,21 @@ static int flow_graph(prt_ctx* ctx) {
     return PRT_OK;
 }
 
+// Whether small solves run their loops inside one cluster (PRT_CLUSTER=0:
+// never; the results are bit-identical either way).
+static bool cluster_enabled() {
+    const char* v = std::getenv("PRT_CLUSTER");
+    return !(v && v[0] == '0');
+}
+
+// The set-up solve's loop as one cluster's kernel, or cudaErrorNotSupported.
+static cudaError_t flow_cluster(prt_ctx* ctx) {
+    FlowState& F = ctx->flow;
+    if (!cluster_enabled()) return cudaErrorNotSupported;
+    return flow_launch_cluster(F.p.nd, F.p.precision, F.f.p, F.fm, F.g, F.kc, F.ctrl.as<FlowCtrl>(),
+                               F.partials.as<double>(), F.nb, ctx->stream);
+}
+
 // Enqueues the whole flow loop of the set-up solve on the context's stream
 // without waiting (ev[0] / ev[1] bracket it): one launch of the WHILE graph,
 // or every chunk of the plain graph where conditional nodes are missing
@@ -310,6 +325,12 @@ int prt::flow_loop_async(prt_ctx* ctx) {
     cudaStream_t s = ctx->stream;
     CK(cudaEventRecord(ctx->ev[0], s));
     if (F.p.nit > 0) {
+        const cudaError_t e = flow_cluster(ctx);
+        if (e != cudaErrorNotSupported) {
+            CK(e);
+            CK(cudaEventRecord(ctx->ev[1], s));
+            return PRT_OK;
+        }
         int rc = flow_graph(ctx);
         if (rc != PRT_OK) return rc;
         const long long chunks = F.graph.conditional ? 1 : (F.p.nit + F.p.every - 1) / F.p.every;
@@ -338,6 +359,9 @@ extern "C" int prt_flow_dev(prt_ctx* ctx, const uint8_t* d_mat, const prt_flow_p
                 CK(cudaMemcpyAsync(&hc2, dctrl, sizeof(hc2), cudaMemcpyDeviceToHost, s));
                 CK(cudaStreamSynchronize(s));
             }
+        } else if (const cudaError_t e = flow_cluster(ctx); e != cudaErrorNotSupported) {
+            CK(e);
+            ctx->launches += 1;
         } else {
             rc = flow_graph(ctx);
             if (rc != PRT_OK) return rc;

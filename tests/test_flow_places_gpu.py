@@ -49,6 +49,12 @@ def grid(name):
     return g
 
 
+# voxels around what one cluster takes: one block, all 16, the most and one more
+EDGES = [("fp64", (1, 1, 128)), ("fp64", (8, 16, 16)), ("fp64", (16, 16, 24)), ("fp64", (16, 16, 25)),
+         ("fp32", (16, 16, 24)), ("fp32f", (16, 32, 20)), ("fp16", (10, 32, 32)), ("fp64", (128, 128)),
+         ("fp32f", (129, 127)), ("fp64", (128, 129))]
+
+
 GRIDS = ["no_rock", "one_voxel", "isolated", "row_of_33", "thin_y", "two_by_three", "wide_gap",
          "long_rows", "site3d", "line2d", "site2d"]
 
@@ -80,13 +86,39 @@ def without_allocation(g, precision, nit):
 def test_places_from_tables_and_maps_are_the_same(monkeypatch, name, precision):
     g = grid(name)
     nit = 53
+    monkeypatch.setenv("PRT_CLUSTER", "0")
     monkeypatch.setenv("PRT_NBR_TABLE", "1")
     plain = solve(g, precision, nit)
     monkeypatch.setenv("PRT_NBR_TABLE", "0")
     packed = solve(g, precision, nit)
     assert np.array_equal(plain, packed)
     assert np.array_equal(plain, without_allocation(g, precision, nit))
+    # the loop inside one cluster, whose blocks' places lie in one another's
+    # shared memory
+    monkeypatch.setenv("PRT_CLUSTER", "1")
+    assert np.array_equal(plain, solve(g, precision, nit))
     if precision == "fp64":
         from oracle.prtlb_oracle import stokes
         ref = stokes(g, nit=nit, tol=0.0)
         assert np.abs(plain - ref).max() <= 1e-6 * np.abs(ref).max()
+
+
+@pytest.mark.parametrize("tol", [0.0, 1e-3])
+@pytest.mark.parametrize("precision,shape", EDGES)
+def test_cluster_loop_is_the_launches(monkeypatch, precision, shape, tol):
+    """Fields and iteration counts of the loop inside one cluster against the
+    launches, at a count that is no multiple of the check interval and with
+    the stop rule."""
+    from prtlb_gpu import stokes_d2q9, stokes_d3q19
+    g = np.full(shape, 2, np.uint8)
+    g.reshape(-1)[5::97] = 0
+    found = []
+    for on in ("0", "1"):
+        monkeypatch.setenv("PRT_CLUSTER", on)
+        info = {}
+        with contextlib.redirect_stdout(io.StringIO()):
+            v = (stokes_d3q19 if g.ndim == 3 else stokes_d2q9)(g, nit=333, tol=tol, info=info,
+                                                               precision=precision)
+        found.append((v, info["flow_iters"], info["flow_change"], info["permeability"]))
+    assert np.array_equal(found[0][0], found[1][0])
+    assert found[0][1:] == found[1][1:]

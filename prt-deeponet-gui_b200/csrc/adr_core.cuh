@@ -152,33 +152,27 @@ __device__ __forceinline__ VoxelSetup<ND> voxel_setup(const AdrDev& d, const prt
 // near one for a far neighbour), so their differences vanish as the
 // reference's replaced values do.  BF: the run has biofilm; without it every
 // face takes the pore diffusivity.  Every transport kernel calls this, so
-// they compute the same function bit for bit.
+// they compute the same function bit for bit.  m2 is read only where the low
+// face velocity is >= 0, p2 only where the high one is not.
 template <int ND, bool BF>
-__device__ __forceinline__ float transport_one(const float* __restrict__ Ck,
-                                               const VoxelSetup<ND>& s, float Cc,
-                                               const float (&dj)[3]) {
-    float m2[ND], m1[ND], p1[ND], p2[ND];
-#pragma unroll
-    for (int i = 0; i < ND; ++i) {
-        m1[i] = ld_early(apart<-4>(Ck, s.nb[i].y));
-        p1[i] = ld_early(apart<4>(Ck, s.nb[i].z));
-        m2[i] = ld_if_up(apart<-4>(Ck, s.nb[i].x), s.fc[i].x);
-        p2[i] = ld_if_down(apart<4>(Ck, s.nb[i].w), s.fc[i].y);
-    }
+__device__ __forceinline__ float transport_terms(const float (&m2)[ND], const float (&m1)[ND],
+                                                 const float (&p1)[ND], const float (&p2)[ND],
+                                                 const float2 (&fc)[ND], uint32_t fl, float Cc,
+                                                 const float (&dj)[3]) {
     float out = 0.f;
     float divu = 0.f;
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
-        const float uL = s.fc[i].x, uH = s.fc[i].y;
+        const float uL = fc[i].x, uH = fc[i].y;
         float DL = dj[0], DH = dj[0];
         if constexpr (BF) {
             // face diffusivity by the biofilm count of its two voxels (0, 1,
             // 2); selected, not indexed, so the table stays in registers
             const int a = Axes<ND>::ax(i);
-            const bool bf = s.fl & F_BF;
+            const bool bf = fl & F_BF;
             const float pore = bf ? dj[1] : dj[0], film = bf ? dj[2] : dj[1];
-            DL = (s.fl & f_nbf_lo(a)) ? film : pore;
-            DH = (s.fl & f_nbf_hi(a)) ? film : pore;
+            DL = (fl & f_nbf_lo(a)) ? film : pore;
+            DH = (fl & f_nbf_hi(a)) ? film : pore;
         }
         // differences upwards along the axis
         const float below = Cc - m1[i], above = p1[i] - Cc;
@@ -194,6 +188,22 @@ __device__ __forceinline__ float transport_one(const float* __restrict__ Ck,
         divu = divu + (uH - uL);
     }
     return out + Cc * divu;
+}
+
+// The same with the neighbours read from the row whose voxel k is at Ck.
+template <int ND, bool BF>
+__device__ __forceinline__ float transport_one(const float* __restrict__ Ck,
+                                               const VoxelSetup<ND>& s, float Cc,
+                                               const float (&dj)[3]) {
+    float m2[ND], m1[ND], p1[ND], p2[ND];
+#pragma unroll
+    for (int i = 0; i < ND; ++i) {
+        m1[i] = ld_early(apart<-4>(Ck, s.nb[i].y));
+        p1[i] = ld_early(apart<4>(Ck, s.nb[i].z));
+        m2[i] = ld_if_up(apart<-4>(Ck, s.nb[i].x), s.fc[i].x);
+        p2[i] = ld_if_down(apart<4>(Ck, s.nb[i].w), s.fc[i].y);
+    }
+    return transport_terms<ND, BF>(m2, m1, p1, p2, s.fc, s.fl, Cc, dj);
 }
 
 // Whether r <= 1/2 (c / t) rounded as the reference rounds it is certain without

@@ -80,11 +80,13 @@ inline int cluster_span(long long n, int blocks) {
 }
 
 // Launches `kern` as one cluster, or returns cudaErrorNotSupported where the
-// device cannot place it (asked once per kernel and size).
+// device cannot place it.
 template <class K, class... A>
 inline cudaError_t launch_cluster(K kern, int blocks, int threads, size_t smem, cudaStream_t s,
                                   A... args) {
-    cudaError_t e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    cudaError_t e = cudaSuccess;
+    if (smem)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
     if (e == cudaSuccess && blocks > 8)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg = {};

@@ -372,6 +372,10 @@ cudaError_t adr_launch_setup(const float* vel, const prt_adr_params& p, const Ad
 cudaError_t adr_launch_expand(const AdrDev& d, const float* rows, float* out, cudaStream_t s);
 cudaError_t adr_launch_step(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl,
                             int kstep, cudaStream_t s);
+// The loop of the set-up run as one cluster's kernel (cluster_adr.cu) up to its
+// pause, stop or limit, or cudaErrorNotSupported (nothing launched).
+cudaError_t adr_launch_cluster(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl,
+                               float* means, cudaStream_t s);
 cudaError_t adr_launch_means(const AdrDev& d, int slot, float* means_out, cudaStream_t s);
 // Ladder rows (ns x nm) from the state in buffer `buf`.
 cudaError_t adr_launch_rows(const AdrDev& d, const float* buf, float* rows, cudaStream_t s);

@@ -806,6 +806,13 @@ static cudaError_t adr_graph(prt_ctx* ctx) {
     return e;
 }
 
+// The started run's loop as one cluster's kernel, or cudaErrorNotSupported.
+static cudaError_t adr_cluster(prt_ctx* ctx) {
+    AdrState& A = ctx->adr;
+    if (!cluster_enabled()) return cudaErrorNotSupported;
+    return adr_launch_cluster(A.d, A.p, A.ctrl.as<AdrCtrl>(), A.means.as<float>(), ctx->stream);
+}
+
 // Enqueues the whole transport loop of a started run (adr_run_setup with no
 // pause) without waiting (ev[2] / ev[3] bracket it), as flow_loop_async.
 int prt::adr_loop_async(prt_ctx* ctx) {
@@ -813,6 +820,12 @@ int prt::adr_loop_async(prt_ctx* ctx) {
     cudaStream_t s = ctx->stream;
     CK(cudaEventRecord(ctx->ev[2], s));
     if (A.rp.limit > 0) {
+        const cudaError_t e = adr_cluster(ctx);
+        if (e != cudaErrorNotSupported) {
+            CK(e);
+            CK(cudaEventRecord(ctx->ev[3], s));
+            return PRT_OK;
+        }
         CK(adr_graph(ctx));
         const long long chunks =
             A.graph.conditional ? 1 : (A.rp.limit + A.rp.check - 1) / A.rp.check;
@@ -846,10 +859,22 @@ extern "C" int prt_adr_run(prt_ctx* ctx, const prt_adr_run_params* rp, prt_progr
     CK(cudaMemcpyAsync(&cur, dctrl, sizeof(cur), cudaMemcpyDeviceToHost, s));
     CK(cudaStreamSynchronize(s));
     bool use_graph = !graphs_disabled();
-    if (use_graph && !cur.done) CK(adr_graph(ctx));
+    bool cluster = use_graph;  // until it turns out not to fit
     CK(cudaEventRecord(ctx->ev[2], s));
     while (!cur.done) {
-        if (!use_graph) {
+        if (cluster) {
+            const cudaError_t e = adr_cluster(ctx);
+            cluster = e != cudaErrorNotSupported;
+            if (cluster) {
+                CK(e);
+            } else {
+                CK(adr_graph(ctx));
+                CK(cudaEventRecord(ctx->ev[2], s));  // the loop starts here
+            }
+        }
+        if (cluster) {
+            ctx->launches += 1;
+        } else if (!use_graph) {
             CK(emit(cudaGraphConditionalHandle(0), 0));
             ctx->launches += per_chunk;
         } else if (A.graph.conditional) {
@@ -863,7 +888,7 @@ extern "C" int prt_adr_run(prt_ctx* ctx, const prt_adr_run_params* rp, prt_progr
         const long long before = cur.n_base;
         CK(cudaMemcpyAsync(&cur, dctrl, sizeof(cur), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
-        if (use_graph && A.graph.conditional)
+        if (!cluster && use_graph && A.graph.conditional)
             ctx->launches += (cur.n_base - before + check - 1) / check * per_chunk;
         if (cb && cur.nlog > delivered) {
             const int nrec = std::min(cur.nlog, log_cap) - delivered;

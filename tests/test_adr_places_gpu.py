@@ -2,8 +2,8 @@
 tables can go wrong: axes of 1, 2 and 3 voxels, rock on and off the inlet
 plane, an all-pore grid, one voxel, warps and blocks that end mid-row, fed,
 unfed and immobile chemicals on the inlet plane, a surface reaction -- with
-16-bit neighbour distances and with neighbour places (PRT_ADR_WIDE=1), alone
-and in a batch; and the same fields on a grid whose distances exceed 16 bits
+16-bit neighbour distances and with neighbour places (PRT_ADR_WIDE=1), by
+launches and inside one cluster (PRT_CLUSTER), alone and in a batch; and the same fields on a grid whose distances exceed 16 bits
 (so that only the places can hold them) as on two halves of it."""
 
 import contextlib
@@ -73,10 +73,11 @@ def test_steps_equal_the_oracle(monkeypatch, name, kind):
     with contextlib.redirect_stdout(io.StringIO()):
         want, _ = reference(g, v, kw["pe"], kw["da"], kw["n_t"], n_species=kw["n_species"],
                             steps=kw["steps"], chem=kw["chem"], da_abio=kw["da_abio"])
-    for wide in ("0", "1"):
+    for wide, cluster in (("0", "0"), ("1", "0"), ("0", "1"), ("1", "1")):
         monkeypatch.setenv("PRT_ADR_WIDE", wide)
+        monkeypatch.setenv("PRT_CLUSTER", cluster)
         out, _ = solve(g, v, kw)
-        assert np.array_equal(out, want), (wide, float(np.abs(out - want).max()))
+        assert np.array_equal(out, want), (wide, cluster, float(np.abs(out - want).max()))
 
 
 def test_wide_neighbours_in_a_batch(monkeypatch):
@@ -112,3 +113,28 @@ def test_distances_beyond_16_bits():
     a, _ = solve(half, v1, kw)
     b, _ = solve(both, v2, kw)
     assert np.array_equal(b[:, :, :, :128], a) and np.array_equal(b[:, :, :, 128:], a)
+
+
+# solute voxels around what one cluster takes: one block, all 16, the most and more
+@pytest.mark.parametrize("kind", ["monod", "default4", "surface3"])
+@pytest.mark.parametrize("shape", [(4, 4, 8), (16, 16, 9), (20, 16, 32), (20, 16, 33), (80, 128)])
+def test_cluster_loop_is_the_launches(monkeypatch, shape, kind):
+    """Snapshots, times, stop step and progress records of the loop inside one
+    cluster against the launches, under the stop rule with its pauses for the
+    callback, and for a step count that is no multiple of the check interval."""
+    g = np.full(shape, 2, np.uint8)
+    g.reshape(-1)[37::61] = 0
+    g[0, 0] = 2
+    v = integer_velocity(g)
+    for steps, most in ((None, 2500), (271, 0)):
+        found = []
+        for cluster in ("0", "1"):
+            monkeypatch.setenv("PRT_CLUSTER", cluster)
+            seen, info = [], {}
+            kw = arguments(g, kind, steps)
+            out, t = solve(g, v, dict(kw, max_steps=most or 100000, info=info,
+                                      on_progress=lambda *a: seen.append(a)))
+            found.append((out, t, info["steps"], info["ladder"], seen))
+        assert np.array_equal(found[0][0], found[1][0])
+        assert np.array_equal(found[0][1], found[1][1])
+        assert found[0][2:] == found[1][2:]

@@ -17,15 +17,23 @@
 // build_dataset_2d.py:290-294, build_geometry_3d.py:201-221): a component
 // touches planes p and q exactly when the walk from p reaches plane q.
 //
-// Here the walk is level-synchronous and pulls: launch L visits every voxel
+// Here the walk is level-synchronous and pulls.  A grid whose voxels, as bits,
+// fit in the shared memory of one thread-block cluster (up to about 8.4
+// million voxels in whole words of 32 along z) walks inside one kernel: the
+// pore not reached yet and the last levels are bit masks, and a level ends
+// with the cluster barrier: 2.4 us a level at 128^3, bound by the barrier
+// behind the scattered stores of the steps, against 9 us for a launch that
+// reads every voxel's step number (the whole call 2.58 -> 1.05 ms).
+// A larger grid takes a launch per level, which visits every voxel
 // once; a pore voxel not reached yet takes L + 1 if a face neighbour holds
-// L.  A voxel is written only by its own thread, and during launch L the
+// L.  There a voxel is written only by its own thread, and during launch L the
 // values change only from "unreached" to L + 1, neither of which is L, so
 // the result does not depend on the order threads run in.  The host enqueues
 // a chunk of levels and stops after the first chunk whose last level reached
 // nothing new (no level can reach anything after one that reached nothing).
 #include <vector>
 
+#include "cluster.cuh"
 #include "runtime_internal.h"
 
 namespace prt {
@@ -108,6 +116,179 @@ __global__ void __launch_bounds__(kWalkThreads)
     if (threadIdx.x == 0 && nb) atomicAdd(counts + 1, (unsigned long long)nb);
 }
 
+// ---------------------------------------------------------------------------
+// the walk on bit masks inside one cluster
+// ---------------------------------------------------------------------------
+// A row is a line of nz voxels along z, in wpr words of 32.  A walk's front is
+// much of a plane at a time, so the rows are dealt out to the 16 blocks
+// diagonally, (x + y) mod 16 (by the row number when ny < 16), and a front
+// across any axis is spread over all of them: with whole planes to a block a
+// level took 6.1 us at 128^3.
+struct BitWalk {
+    int nx, ny, nz, wpr;
+    int nyc;   // rows of one x in a block (diagonal dealing), 0: by row number
+    int rows;  // rows of a block
+    FastDiv by_word, by_nyc, by_ny;
+};
+constexpr int kBitThreads = 512;
+constexpr int kBitWords = 16384;  // words of a block: three masks and a queue in 224 KB
+constexpr int kLevelsPerVote = 16;
+
+inline BitWalk make_bit_walk(const Grid& g) {
+    BitWalk b;
+    b.nx = g.nx;
+    b.ny = g.ny;
+    b.nz = g.nz;
+    b.wpr = (g.nz + 31) / 32;
+    b.nyc = g.ny >= kClusterMax ? (g.ny + kClusterMax - 1) / kClusterMax : 0;
+    const long long rows = b.nyc ? (long long)g.nx * b.nyc
+                                 : ((long long)g.nx * g.ny + kClusterMax - 1) / kClusterMax;
+    b.rows = (int)std::min<long long>(rows, kBitWords + 1);  // more is refused below
+    b.by_word = make_fastdiv((unsigned)b.wpr);
+    b.by_nyc = make_fastdiv((unsigned)std::max(b.nyc, 1));
+    b.by_ny = make_fastdiv((unsigned)g.ny);
+    return b;
+}
+
+// Row (x, y): its block and its number there; and back.
+__device__ __forceinline__ void row_place(const BitWalk& b, int x, int y, int& blk, int& lr) {
+    const int row = x * b.ny + y;
+    blk = (b.nyc ? x + y : row) & (kClusterMax - 1);
+    lr = b.nyc ? x * b.nyc + y / kClusterMax : row / kClusterMax;
+}
+__device__ __forceinline__ void place_row(const BitWalk& b, int blk, int lr, int& x, int& y) {
+    if (b.nyc) {
+        x = (int)fast_div((unsigned)lr, b.by_nyc);
+        y = (lr - x * b.nyc) * kClusterMax + ((blk - x) & (kClusterMax - 1));
+    } else {
+        const int row = lr * kClusterMax + blk;
+        x = (int)fast_div((unsigned)row, b.by_ny);
+        y = row - x * b.ny;
+    }
+}
+
+// One warp per word: steps = 0 on the pore of the seed plane, -2 on the other
+// pore, -1 elsewhere; seed and rest (zeroed before): the bits of the first
+// two, block by block; counts[0] += pore voxels.
+__global__ void __launch_bounds__(kWalkThreads)
+    bit_init_kernel(const uint8_t* __restrict__ mat, WalkGrid w, BitWalk b, int code,
+                    int* __restrict__ steps, unsigned* __restrict__ seed,
+                    unsigned* __restrict__ rest, unsigned long long* __restrict__ counts) {
+    const unsigned word = blockIdx.x * (kWalkThreads / 32) + (threadIdx.x >> 5);
+    int pore = 0;
+    if (word < (unsigned)(b.nx * b.ny * b.wpr)) {  // whole warps
+        const unsigned row = fast_div(word, b.by_word);
+        const int q = (int)(word - row * b.wpr), z = q * 32 + (threadIdx.x & 31);
+        const int x = (int)fast_div(row, b.by_ny), y = (int)row - x * b.ny;
+        bool start = false;
+        if (z < b.nz) {
+            const long long c = (long long)row * b.nz + z;
+            pore = mat[c] == code;
+            start = pore && (w.axis == 0 ? x : (w.axis == 1 ? y : z)) == w.plane;
+            steps[c] = pore ? (start ? 0 : -2) : -1;
+        }
+        const unsigned s = __ballot_sync(0xffffffffu, start);
+        const unsigned r = __ballot_sync(0xffffffffu, pore && !start);
+        if ((threadIdx.x & 31) == 0) {
+            int blk, lr;
+            row_place(b, x, y, blk, lr);
+            const long long at = ((long long)blk * b.rows + lr) * b.wpr + q;
+            seed[at] = s;
+            rest[at] = r;
+        }
+    }
+    const int n = __syncthreads_count(pore);
+    if (threadIdx.x == 0 && n) atomicAdd(counts, (unsigned long long)n);
+}
+
+// The whole walk from the masks; steps of the reached voxels, counts[1] +=
+// reached pore voxels.  A level: every thread looks through its words for bits
+// that the level before sent (few have any), what of them is still open is
+// the level's pore and its words are queued; then the queued words' bits are
+// sent on, to their own word shifted by one voxel, and to the words of the
+// neighbouring rows in their blocks.
+__global__ void __launch_bounds__(kBitThreads, 1)
+    bit_walk_kernel(BitWalk b, const unsigned* __restrict__ seed, const unsigned* __restrict__ rest,
+                    int* __restrict__ steps, unsigned long long* __restrict__ counts) {
+    extern __shared__ unsigned masks[];  // open, sent to even and to odd levels, queue
+    __shared__ int votes[kClusterMax];
+    __shared__ int queued[2];
+    const int t = threadIdx.x;
+    const int rank = (int)cluster_rank();
+    const int mine = b.rows * b.wpr;
+    unsigned* open = masks;
+    unsigned* sent[2] = {masks + mine, masks + 2 * mine};
+    unsigned short* queue = reinterpret_cast<unsigned short*>(masks + 3 * mine);
+    const uint32_t sent_at[2] = {shared_address(sent[0]), shared_address(sent[1])};
+    for (int i = t; i < mine; i += kBitThreads) {
+        const long long at = (long long)rank * mine + i;
+        const unsigned s = seed[at];
+        open[i] = rest[at] | s;
+        sent[0][i] = s;
+        sent[1][i] = 0u;
+    }
+    if (t < 2) queued[t] = 0;
+    unsigned long long reached = 0;
+    cluster_sync();
+    for (int lv = 0;; ++lv) {
+        unsigned* now = sent[lv & 1];
+        unsigned* next = sent[(lv & 1) ^ 1];
+        int* n = queued + (lv & 1);
+        for (int i = t; i < mine; i += kBitThreads) {
+            if (now[i] == 0u) continue;
+            const unsigned o = open[i], f = now[i] & o;
+            now[i] = f;
+            if (f == 0u) continue;
+            open[i] = o ^ f;
+            reached += __popc(f);
+            queue[atomicAdd(n, 1)] = (unsigned short)i;
+        }
+        __syncthreads();
+        const int nq = *n;
+        if (t == 0) queued[(lv & 1) ^ 1] = 0;
+        for (int e = t; e < nq; e += kBitThreads) {
+            const int i = queue[e];
+            const unsigned f = now[i];
+            now[i] = 0u;
+            const int lr = (int)fast_div((unsigned)i, b.by_word), q = i - lr * b.wpr;
+            int x, y;
+            place_row(b, rank, lr, x, y);
+            auto send = [&](int xn, int yn) {  // f to the same word of row (xn, yn)
+                int blk, r;
+                row_place(b, xn, yn, blk, r);
+                const uint32_t a =
+                    in_block(sent_at[(lv & 1) ^ 1] + (r * b.wpr + q) * 4, (unsigned)blk);
+                asm volatile("red.relaxed.cluster.shared::cluster.or.b32 [%0], %1;" ::"r"(a), "r"(f)
+                             : "memory");
+            };
+            if (y > 0) send(x, y - 1);
+            if (y < b.ny - 1) send(x, y + 1);
+            if (x > 0) send(x - 1, y);
+            if (x < b.nx - 1) send(x + 1, y);
+            atomicOr(next + i, (f << 1) | (f >> 1));
+            if (q > 0 && (f & 1u)) atomicOr(next + (i - 1), 1u << 31);
+            if (q < b.wpr - 1 && (f >> 31)) atomicOr(next + (i + 1), 1u);
+            int* out = steps + ((long long)(x * b.ny + y) * b.nz + q * 32);
+            for (unsigned m = f; m; m &= m - 1) out[__ffs(m) - 1] = lv;
+        }
+        // no level can reach anything after one that reached nothing
+        const bool vote = lv % kLevelsPerVote == kLevelsPerVote - 1;
+        if (vote && t == 0) {
+            const uint32_t a = in_block(shared_address(votes + rank), 0);
+            asm volatile("st.shared::cluster.s32 [%0], %1;" ::"r"(a), "r"(nq) : "memory");
+        }
+        cluster_sync();
+        if (vote) {
+            int v = 0;
+            if (t < kClusterMax) ld_cluster(in_block(shared_address(votes + t), 0), v);
+            if (!__syncthreads_or(v)) break;
+        }
+    }
+    for (int o = 16; o > 0; o >>= 1) reached += __shfl_down_sync(0xffffffffu, reached, o);
+    if ((t & 31) == 0 && reached) atomicAdd(counts + 1, reached);
+    cluster_sync();  // no block leaves while another may read its votes or words
+}
+
 // label_materials (build_geometry_3d.py:224-239): pore 2, solid with a
 // pore face neighbour 1, other solid 0; positions beyond the grid's faces
 // count as solid (no wrap).  One thread per voxel, six neighbour reads
@@ -172,6 +353,12 @@ extern "C" int prt_label_materials(prt_ctx* ctx, const uint8_t* solid, int32_t n
     return PRT_OK;
 }
 
+// PRT_CLUSTER=0: a launch per level whatever the size (the same steps).
+static bool bit_walk_enabled() {
+    const char* v = std::getenv("PRT_CLUSTER");
+    return !(v && v[0] == '0');
+}
+
 extern "C" int prt_walk_from_plane(prt_ctx* ctx, const uint8_t* mat, int32_t nd,
                                    const int32_t* dims, int32_t pore_code, int32_t axis,
                                    int32_t plane, int32_t* steps_out, int64_t* n_reached,
@@ -209,25 +396,48 @@ extern "C" int prt_walk_from_plane(prt_ctx* ctx, const uint8_t* mat, int32_t nd,
     int* steps = P.steps.as<int>();
     int* flags = P.flags.as<int>();
     unsigned long long* counts = P.counts.as<unsigned long long>();
-    walk_init_kernel<<<nb, kWalkThreads, 0, s>>>(P.mat.as<uint8_t>(), w, pore_code, steps, counts);
-    CK(cudaGetLastError());
-    ctx->launches += 1;
-    // at most one level per pore voxel, so the loop ends; in practice after
-    // the longest shortest path
-    std::vector<int> h(kLevelsPerChunk);
-    for (long long base = 0; base <= g.n; base += kLevelsPerChunk) {
-        CK(cudaMemsetAsync(flags, 0, kLevelsPerChunk * sizeof(int), s));
-        for (int i = 0; i < kLevelsPerChunk; ++i)
-            walk_level_kernel<<<nb, kWalkThreads, 0, s>>>(steps, w, (int)(base + i), flags + i);
+    bool walked = false;
+    const BitWalk b = make_bit_walk(g);
+    if (bit_walk_enabled() && (long long)b.rows * b.wpr <= kBitWords) {
+        const size_t words = (size_t)kClusterMax * b.rows * b.wpr;
+        CK(P.bits.ensure(words * 2 * sizeof(unsigned)));
+        CK(cudaMemsetAsync(P.bits.p, 0, words * 2 * sizeof(unsigned), s));
+        unsigned* seed = P.bits.as<unsigned>();
+        unsigned* rest = seed + words;
+        const unsigned used = (unsigned)(b.nx * b.ny * b.wpr);
+        bit_init_kernel<<<(used + kWalkThreads / 32 - 1) / (kWalkThreads / 32), kWalkThreads, 0,
+                          s>>>(P.mat.as<uint8_t>(), w, b, pore_code, steps, seed, rest, counts);
         CK(cudaGetLastError());
-        ctx->launches += kLevelsPerChunk;
-        CK(cudaMemcpyAsync(h.data(), flags, kLevelsPerChunk * sizeof(int), cudaMemcpyDeviceToHost, s));
-        CK(cudaStreamSynchronize(s));
-        if (h[kLevelsPerChunk - 1] == 0) break;
+        const size_t smem = (size_t)b.rows * b.wpr * (3 * sizeof(unsigned) + sizeof(unsigned short));
+        const cudaError_t e = launch_cluster(bit_walk_kernel, kClusterMax, kBitThreads, smem, s, b,
+                                             (const unsigned*)seed, (const unsigned*)rest, steps,
+                                             counts);
+        walked = e != cudaErrorNotSupported;
+        if (walked) CK(e);
+        ctx->launches += 1 + walked;
+        if (!walked) CK(cudaMemsetAsync(P.counts.p, 0, 2 * sizeof(unsigned long long), s));
     }
-    walk_final_kernel<<<nb, kWalkThreads, 0, s>>>(steps, g.n, counts);
-    CK(cudaGetLastError());
-    ctx->launches += 1;
+    if (!walked) {
+        walk_init_kernel<<<nb, kWalkThreads, 0, s>>>(P.mat.as<uint8_t>(), w, pore_code, steps, counts);
+        CK(cudaGetLastError());
+        ctx->launches += 1;
+        // at most one level per pore voxel, so the loop ends; in practice after
+        // the longest shortest path
+        std::vector<int> h(kLevelsPerChunk);
+        for (long long base = 0; base <= g.n; base += kLevelsPerChunk) {
+            CK(cudaMemsetAsync(flags, 0, kLevelsPerChunk * sizeof(int), s));
+            for (int i = 0; i < kLevelsPerChunk; ++i)
+                walk_level_kernel<<<nb, kWalkThreads, 0, s>>>(steps, w, (int)(base + i), flags + i);
+            CK(cudaGetLastError());
+            ctx->launches += kLevelsPerChunk;
+            CK(cudaMemcpyAsync(h.data(), flags, kLevelsPerChunk * sizeof(int), cudaMemcpyDeviceToHost, s));
+            CK(cudaStreamSynchronize(s));
+            if (h[kLevelsPerChunk - 1] == 0) break;
+        }
+        walk_final_kernel<<<nb, kWalkThreads, 0, s>>>(steps, g.n, counts);
+        CK(cudaGetLastError());
+        ctx->launches += 1;
+    }
     unsigned long long hc[2];
     CK(cudaMemcpyAsync(hc, counts, sizeof(hc), cudaMemcpyDeviceToHost, s));
     CK(copy_out(ctx, steps_out, steps, (size_t)g.n * 4));  // waits for both

@@ -37,11 +37,11 @@ constexpr int kAdrThreads = 128;
 template <int ND, int NS, bool BF, bool WIDE>
 __global__ void __launch_bounds__(kAdrThreads) adr_step_kernel(AdrDev d, prt_adr_params p,
                                                                const AdrCtrl* __restrict__ ctrl,
-                                                               int kstep, int late) {
+                                                               int kstep, int late, int turn) {
     if (!late) griddep_launch_dependents();
-    // every other step walks the voxels downwards: it starts on what the step
-    // before left in the L2
-    const unsigned b = (kstep & 1) ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    // turn (a grid of more than half a wave): every other step walks the voxels
+    // downwards, so it starts on what the step before left in the L2
+    const unsigned b = (kstep & 1) && turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const unsigned k = b * kAdrThreads + threadIdx.x;
     const bool live = k < (unsigned)d.nm;
     VoxelSetup<ND> s;
@@ -383,7 +383,7 @@ static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctr
     const long long resident = resident_blocks(kern);
     const int late = pdl_late(nb <= resident && 2 * nb > resident) ? 1 : 0;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    return cudaLaunchKernelEx(&cfg, kern, d, p, ctrl, k, late);
+    return cudaLaunchKernelEx(&cfg, kern, d, p, ctrl, k, late, 2 * nb > resident ? 1 : 0);
 }
 
 template <int ND>

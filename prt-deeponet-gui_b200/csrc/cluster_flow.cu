@@ -76,8 +76,8 @@ __device__ __forceinline__ double cluster_cell(uint32_t own, const uint32_t (&fa
 #pragma unroll
     for (int p = 0; p < L::NP; ++p)
         h[L::pa(p)] = Pop<S>::dec(ld_own<S>(own + L::pa(p) * ROW + o), kc.inv_scale);
-    const Moments<R, RA> m = moments<L, R, RA>(h, kc.half_g);
-    collide<L, R, RA>(h, m, kc, [&](int i, int p, R v) {
+    const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(kc));
+    collide_mode<L, M>(h, m, kc, [&](int i, int p, R v) {
         const S q = Pop<S>::enc(v, kc.scale);
         if (p < 0) st_own(own, q);
         else if (i == L::pa(p)) st_cluster(far[p] + i * ROW + f, q);

@@ -99,23 +99,28 @@ struct Pop<__half> {
 // base: again from the lattice's address.  Measured on 128^3 / 64^3 packs (us
 // an iteration, none / index / base): float64 72.8 / 57.3 / 56.9 and 8.3 /
 // 6.6 / 6.1, float32 with float64 momentum 32.1 / 28.6 / 29.3 and 4.8 / 4.7 /
-// 4.9, float16 22.4 / 20.1 / 20.8 and - / 3.8 / 4.3; float32 alone fits its
-// registers either way (4.18 / 4.42 / - at 64^3).
+// 4.9, float16 22.4 / 20.1 / 20.8 and - / 3.8 / 4.3; float32 alone without it
+// spills 88 bytes (4.97 against 3.91 at 64^3).
 enum class Fresh { none, index, base };
 
 // Precision modes: storage type S, arithmetic R for the symmetric part and
 // RA for the momentum and the antisymmetric non-equilibrium part (a small
 // difference of two O(u) numbers), and the resident blocks of kFlowThreads
 // per SM the register budget is cut for (single-solve and batched steps).
-// `fresh`: see Fresh.
-// `staged`: the arrived populations go to shared memory by cp.async, so no
-// register waits on a gather load (4- and 8-byte populations only).
+// `fresh`: see Fresh; `regrouped`: see collide_regrouped.
+// `staged`: D3Q19's arrived populations go to shared memory by cp.async, so no
+// register waits on a gather load.  Only float64 gains by it (80^3 9.8 against
+// 12.1 us in registers, which spill); in float32 the 57 shared-memory accesses
+// a voxel cost more than they save: us an iteration, staged -> in registers,
+// 64^3 4.27 -> 3.91 (float64 momentum 4.73 -> 4.35), 128^3 23.8 -> 23.2 (26.5
+// -> 25.6), 192^3 104 -> 93 (106 -> 100); D2Q9 256^2 float64 2.34 -> 2.14.
 struct ModeF64 {  // the reference's arithmetic
     using S = double;
     using R = double;
     using RA = double;
     static constexpr int min_blocks = 7;
     static constexpr Fresh fresh = Fresh::base;
+    static constexpr bool regrouped = true;
     static constexpr int batch_min_blocks = 6;
     static constexpr bool staged = true;
 };
@@ -123,12 +128,12 @@ struct ModeF32 {  // float32 populations, float32 collision
     using S = float;
     using R = float;
     using RA = float;
-    // 64 registers (8 blocks per SM): at 48 (10 blocks) an iteration took
-    // 5.46 us at 64^3 and 4.73 at 48^3, at 64 it takes 4.58 and 3.17
+    // 64 registers (8 blocks per SM)
     static constexpr int min_blocks = 8;
-    static constexpr Fresh fresh = Fresh::none;
+    static constexpr Fresh fresh = Fresh::index;
+    static constexpr bool regrouped = true;
     static constexpr int batch_min_blocks = 8;
-    static constexpr bool staged = true;
+    static constexpr bool staged = false;
 };
 struct ModeF32D {  // float32 populations, float64 momentum
     using S = float;
@@ -139,8 +144,9 @@ struct ModeF32D {  // float32 populations, float64 momentum
     // per iteration; 128^3 unchanged)
     static constexpr int min_blocks = 8;
     static constexpr Fresh fresh = Fresh::index;
+    static constexpr bool regrouped = false;
     static constexpr int batch_min_blocks = 8;
-    static constexpr bool staged = true;
+    static constexpr bool staged = false;
 };
 struct ModeF16 {  // scaled float16 populations, float32 collision
     using S = __half;
@@ -148,6 +154,7 @@ struct ModeF16 {  // scaled float16 populations, float32 collision
     using RA = float;
     static constexpr int min_blocks = 6;
     static constexpr Fresh fresh = Fresh::index;
+    static constexpr bool regrouped = false;
     static constexpr int batch_min_blocks = 6;
     static constexpr bool staged = false;
 };
@@ -271,7 +278,7 @@ __device__ __forceinline__ void far_slots_packed(const FlowMap& fm, const Grid& 
 // the lattice stay in the L2 (flow_use_nbr): us an iteration, plain / packed
 // / maps alone, 64^3 float32 4.2 / 4.6 / 5.0, 96^3 float64 16.2 / 17.6 / 23.6,
 // 128^3 float16 20.3 / 21.7 / 26.2; beyond it the bytes decide: 128^3 float32
-// 26.7 / 24.9 / 30.7, 192^3 112 / 104 / 126.
+// 26.7 / 24.9 / 30.7, 192^3 112 / 104 / 126 (populations staged, see below).
 enum class Far { table, packed };
 
 template <class L, Far F>
@@ -343,6 +350,12 @@ __device__ __forceinline__ void gather_staged(const Lat<S>& lat, int k, const in
     cp_async_commit();
 }
 
+template <class RA>
+__device__ __forceinline__ RA half_force(const LbParams& kc) {
+    if constexpr (sizeof(RA) == 8) return kc.half_g;
+    else return kc.half_g_f;
+}
+
 template <class R, class RA>
 struct Moments {
     R drho, jsq;    // density deviation, rho u^2
@@ -353,7 +366,7 @@ struct Moments {
 // Moments of the arrived (shifted) populations (prtlb_3d.py:428-433):
 // drho = sum h, J = rho u = sum e h + g/2 x.
 template <class L, class R, class RA, class HA>
-__device__ __forceinline__ Moments<R, RA> moments(const HA& h, double half_g) {
+__device__ __forceinline__ Moments<R, RA> moments(const HA& h, RA half_g) {
     Moments<R, RA> m;
     RA s = RA(h[0]);
     RA jx = RA(0), jy = RA(0), jz = RA(0);
@@ -369,7 +382,7 @@ __device__ __forceinline__ Moments<R, RA> moments(const HA& h, double half_g) {
         if (L::c(a, 2) == 1) jz += d;
         if (L::c(a, 2) == -1) jz -= d;
     }
-    jx += RA(half_g);
+    jx += half_g;
     m.jx = jx;
     m.jy = jy;
     m.jz = jz;
@@ -416,12 +429,63 @@ __device__ __forceinline__ void collide(const HA& h, const Moments<R, RA>& m, co
     }
 }
 
+// The same collision with its constants folded and the pair's symmetric and
+// antisymmetric changes formed as one fused sum each, the two members as h +
+// (A - B) and h + (A + B): 12 operations a pair where collide takes 18, and
+// no conversion of constants.  Its rounding errors are of the same size (a
+// sum of the same terms, fewer roundings); the modes whose collision has one
+// arithmetic type and whose results are not tied to another rounding take it.
+template <class L, class R, class HA, class Put>
+__device__ __forceinline__ void collide_regrouped(const HA& h, const Moments<R, R>& m,
+                                                  const Regrouped<R>& kc, Put put) {
+    const R base = m.drho - R(1.5) * m.jsq;
+    const R h0 = R(h[0]);
+    put(0, -1, h0 + (kc.w0 * base - kc.omp * h0));
+    const R b[2] = {kc.wp[0] * base, kc.wp[1] * base};
+    const R q[2] = {kc.w45[0] * m.inv_rho, kc.w45[1] * m.inv_rho};
+#pragma unroll
+    for (int p = 0; p < L::NP; ++p) {
+        const int a = L::pa(p), bb = L::pb(p);
+        constexpr int axis_pairs = L::Q == 19 ? 3 : 2;
+        const int c = p < axis_pairs ? 0 : 1;
+        R eJ = R(0);
+        if (L::c(a, 0) == 1) eJ += m.jx;
+        if (L::c(a, 0) == -1) eJ -= m.jx;
+        if (L::c(a, 1) == 1) eJ += m.jy;
+        if (L::c(a, 1) == -1) eJ -= m.jy;
+        if (L::c(a, 2) == 1) eJ += m.jz;
+        if (L::c(a, 2) == -1) eJ -= m.jz;
+        const R ha = R(h[a]), hb = R(h[bb]);
+        const R A = (q[c] * eJ * eJ + b[c]) - kc.half_omp * (ha + hb);
+        R B = kc.half_omm * (ha - hb) - kc.wm[c] * eJ;
+        if (L::c(a, 0) != 0) B -= kc.guo[p];
+        put(a, p, ha + (A - B));
+        put(bb, p, hb + (A + B));
+    }
+}
+
+// The mode's collision.
+template <class L, class M, class HA, class Put>
+__device__ __forceinline__ void collide_mode(const HA& h,
+                                             const Moments<typename M::R, typename M::RA>& m,
+                                             const LbParams& kc, Put put) {
+    if constexpr (M::regrouped) {
+        if constexpr (sizeof(typename M::R) == 8) collide_regrouped<L>(h, m, kc.d, put);
+        else collide_regrouped<L>(h, m, kc.f, put);
+    } else {
+        collide<L, typename M::R, typename M::RA>(h, m, kc, put);
+    }
+}
+
 // The collision of slot k with its results stored in the lattice: f_a to the
 // pair's far place and f_b to its own (see Lat).
-template <class L, Fresh F, class S, class R, class RA, class HA>
-__device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const int (&far)[L::NP],
-                                              const HA& h, const Moments<R, RA>& m,
+template <class L, class M, class HA>
+__device__ __forceinline__ void collide_store(const Lat<typename M::S>& lat0, int k,
+                                              const int (&far)[L::NP], const HA& h,
+                                              const Moments<typename M::R, typename M::RA>& m,
                                               const LbParams& kc) {
+    using S = typename M::S;
+    constexpr Fresh F = L::Q == 19 ? M::fresh : Fresh::none;
     Lat<S> lat = lat0;
     int to[L::NP];
     if (F == Fresh::base) asm volatile("" : "+l"(lat.f));
@@ -431,7 +495,7 @@ __device__ __forceinline__ void collide_store(const Lat<S>& lat0, int k, const i
         to[p] = far[p];
         if (F == Fresh::index) asm volatile("" : "+r"(to[p]));
     }
-    collide<L, R, RA>(h, m, kc, [&](int i, int p, R v) {
+    collide_mode<L, M>(h, m, kc, [&](int i, int p, typename M::R v) {
         const S q = Pop<S>::enc(v, kc.scale);
         if (p < 0) lat.f[k] = q;
         else if (i == L::pa(p)) *lat.at_far(i, to[p]) = q;
@@ -447,20 +511,20 @@ __device__ __forceinline__ double lb_cell(const Lat<typename M::S>& lat, const L
     using S = typename M::S;
     using R = typename M::R;
     using RA = typename M::RA;
-    if constexpr (M::staged) {
+    if constexpr (M::staged && L::Q == 19) {
         __shared__ S stage[L::Q * kFlowThreads];
         S* col = stage + threadIdx.x;
         gather_staged<L, S>(lat, k, far, col);
         cp_async_wait<0>();
         const Staged<S> h{col};
-        const Moments<R, RA> m = moments<L, R, RA>(h, kc.half_g);
-        collide_store<L, L::Q == 19 ? M::fresh : Fresh::none, S, R, RA>(lat, k, far, h, m, kc);
+        const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(kc));
+        collide_store<L, M>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     } else {
         typename Pop<S>::H h[L::Q];
         gather<L, S>(lat, k, far, kc.inv_scale, h);
-        const Moments<R, RA> m = moments<L, R, RA>(h, kc.half_g);
-        collide_store<L, L::Q == 19 ? M::fresh : Fresh::none, S, R, RA>(lat, k, far, h, m, kc);
+        const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(kc));
+        collide_store<L, M>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     }
 }

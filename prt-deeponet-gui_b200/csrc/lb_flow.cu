@@ -33,12 +33,13 @@
 namespace prt {
 
 // One whole LB iteration t (ODD = t & 1); solid voxels do nothing.  late: the
-// next iteration is let in after this one's stores (see pdl_late).
+// next iteration is let in after this one's stores (see pdl_late).  turn: odd
+// iterations walk the slots downwards (a grid of several waves).
 //
 // Bound by the L2 and DRAM traffic where the lattice exceeds the L2 (192^3),
 // by latency below; in place it reads and writes each population once and
-// finds 9 places instead of 18.  Odd iterations walk the slots downwards, so
-// an iteration starts on what the one before left in the L2: 128^3 float32
+// finds 9 places instead of 18.  Odd iterations walk the slots downwards when
+// there are several waves, so an iteration starts on what the one before left in the L2: 128^3 float32
 // 28.4 -> 26.8 us, float64 57.3 -> 48.3, 192^3 115 -> 105 and 174 -> 167.
 // From one lattice into another (the form before): 40.3, 65.1, 126.6, 206.5;
 // 96^3 float64 27.1 -> 16.2, float32 11.8 -> 10.7, 64^3 unchanged within 5 %.
@@ -48,9 +49,9 @@ template <class L, class M, Far F, bool ODD, bool CHECK>
 __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
     lb_step_kernel(typename M::S* __restrict__ f, FlowMap fm, Grid g, LbParams kc,
                    const FlowCtrl* __restrict__ ctrl, int kstep, double* __restrict__ partials,
-                   int late) {
+                   int late, int turn) {
     if (!late) griddep_launch_dependents();
-    const int b = ODD ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
+    const int b = ODD && turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
     const int k = b * kFlowThreads + threadIdx.x;
     const Lat<typename M::S> lat = lattice<L>(f, fm.rs, ODD);
     // the pore maps never change during a solve: the far places are looked
@@ -117,7 +118,7 @@ __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
         {
             typename Pop<S>::H h[L::Q];
             gather<L, S>(lat, kk, far, k.inv_scale, h);
-            const Moments<R, RA> m = moments<L, R, RA>(h, k.half_g);
+            const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(k));
             const RA ux = m.jx * m.inv_rho, uy = m.jy * m.inv_rho, uz = m.jz * m.inv_rho;
             vx = (float)ux;
             vy = (float)uy;
@@ -364,8 +365,9 @@ static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Gr
                        : lb_step_kernel<L, M, Far::packed, ODD, CHECK>;
     // both forms are held to the same register budget
     static const long long resident = resident_blocks(kern);
+    const bool one_wave = nb <= resident;
     return cudaLaunchKernelEx(&cfg, kern, f, fm, g, k, ctrl, kstep, partials,
-                              pdl_late(nb <= resident) ? 1 : 0);
+                              pdl_late(one_wave) ? 1 : 0, one_wave ? 0 : 1);
 }
 
 template <class L, class M>

@@ -104,6 +104,19 @@ struct FlowCtrl {
     int pad;
 };
 
+// The constants of the regrouped collision (lb_core.cuh), formed in float64 and
+// rounded once to its arithmetic type: the index is 0 for the pairs along an
+// axis, 1 for the diagonal ones.
+template <class R>
+struct Regrouped {
+    R omp, half_omp, half_omm;
+    R w0;       // w_0 omega+
+    R wp[2];    // w omega+
+    R w45[2];   // 4.5 w omega+
+    R wm[2];    // 3 w omega-
+    R guo[9];
+};
+
 // Constants of one flow solve, in float64; kernels round them to their
 // arithmetic type.
 struct LbParams {
@@ -112,7 +125,29 @@ struct LbParams {
     double guo[9];    // w_a (1 - omega-/2) 3 g c_ax for the first member of each pair
     float scale;      // FP16 storage scale (2^k) and its inverse
     float inv_scale;
+    Regrouped<double> d;
+    Regrouped<float> f;
+    float half_g_f;
 };
+
+// (batches compare constants as bytes)
+static_assert(sizeof(LbParams) == 12 * 8 + 2 * 4 + 19 * 8 + 19 * 4 + 4, "no padding in LbParams");
+
+template <class R>
+inline void fill_regrouped(Regrouped<R>& r, const LbParams& k, int nd) {
+    const double w0 = nd == 3 ? 1.0 / 3.0 : 4.0 / 9.0;
+    const double w[2] = {nd == 3 ? 1.0 / 18.0 : 1.0 / 9.0, 1.0 / 36.0};
+    r.omp = (R)k.omp;
+    r.half_omp = (R)(0.5 * k.omp);
+    r.half_omm = (R)(0.5 * k.omm);
+    r.w0 = (R)(w0 * k.omp);
+    for (int c = 0; c < 2; ++c) {
+        r.wp[c] = (R)(w[c] * k.omp);
+        r.w45[c] = (R)(4.5 * w[c] * k.omp);
+        r.wm[c] = (R)(3.0 * w[c] * k.omm);
+    }
+    for (int p = 0; p < 9; ++p) r.guo[p] = (R)k.guo[p];
+}
 
 // Control block of one transport solve (the while loop of prtlb_3d.py:1493).
 struct AdrCtrl {
@@ -260,6 +295,9 @@ inline void fill_lbconst(LbParams& k, int nd, double force, double tau, double m
     }
     k.scale = scale;
     k.inv_scale = 1.0f / scale;
+    fill_regrouped(k.d, k, nd);
+    fill_regrouped(k.f, k, nd);
+    k.half_g_f = (float)k.half_g;
 }
 
 // Bits that hold the values 0 .. n-1.

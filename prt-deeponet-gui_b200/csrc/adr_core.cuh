@@ -368,12 +368,6 @@ __device__ __forceinline__ void adr_voxel_step(const AdrDev& d, const prt_adr_pa
     for (int j = 0; j < NS; ++j) Cout[j * ms + k] = cn[j];
 }
 
-template <int ND, int NS, bool BF, bool WIDE>
-__device__ __forceinline__ void adr_voxel(const AdrDev& d, const prt_adr_params& p, long long n,
-                                          unsigned k) {
-    adr_voxel_step<ND, NS, BF>(d, p, n, k, voxel_setup<ND, BF, WIDE>(d, p, k));
-}
-
 // The check of the time loop at step `end` (prtlb_3d.py:1499-1543), in
 // float64 like the reference's arrays of Python floats: running scale,
 // per-check change, geometric-tail remainder `rest`, the progress record,

@@ -31,8 +31,23 @@ __device__ __forceinline__ const LbParams& job_constants(const LbParams& kcu, co
     else return own;
 }
 
-template <class L, class M, bool UNI>
-__global__ void __launch_bounds__(kFlowThreads, M::batch_min_blocks)
+// F: where the far places come from.  With plain tables (small batches, in the
+// L2) float32 gathers into registers, six blocks an SM; with packed ones
+// staged through shared memory like float64.  us a step of 16 / 48 float32
+// solves of edges 24-48: table 14.7 / 51.1, packed 17.6 / 51.3; 12 of edges
+// 60-90: 102.4 and 100.4 (from one lattice into another before: 17.5 / 58.9
+// and 111.6); 48 in float64 88.7 -> 81.8.
+template <class M, Far F>
+__host__ __device__ constexpr int batch_blocks() {
+    return F == Far::table && sizeof(typename M::S) == 4 ? 6 : M::batch_min_blocks;
+}
+template <class L, class M, Far F>
+__host__ __device__ constexpr bool batch_staged() {
+    return L::Q == 19 && (F == Far::packed ? sizeof(typename M::S) >= 4 : M::staged);
+}
+
+template <class L, class M, bool UNI, Far F>
+__global__ void __launch_bounds__(kFlowThreads, batch_blocks<M, F>())
     batch_flow_kernel(const FlowJob* __restrict__ jobs, const BatchTile* __restrict__ tiles,
                       const int* __restrict__ ntiles_p, const long long* __restrict__ gstep,
                       int k, LbParams kcu, int late) {
@@ -65,7 +80,7 @@ __global__ void __launch_bounds__(kFlowThreads, M::batch_min_blocks)
         const long long it = done_steps - sj.g0;  // iterations done before this one
         const long long nit = __ldcg(&ctrl->nit);
         const bool run = !__ldcg(&ctrl->done) && it < nit;
-        const bool check = ((it + 1) % __ldcg(&ctrl->every)) == 0;  // the sampled iterations
+        const bool check = divides(__ldcg(&ctrl->every), it + 1);  // the sampled iterations
         const bool advance = check || it + 1 >= nit;
         if (!run) {  // uniform over the block
             __syncthreads();  // every thread has read ctrl before sj may change
@@ -78,8 +93,8 @@ __global__ void __launch_bounds__(kFlowThreads, M::batch_min_blocks)
             const int slot = b * kFlowThreads + threadIdx.x;
             double acc = 0.0;
             int far[L::NP];
-            far_slots<L, Far::packed>(sj.fm, sj.g, slot, far);
-            if (slot < nf) acc = lb_cell<L, M>(lat, job_constants<UNI>(kcu, sj.kc), slot, far);
+            far_slots<L, F>(sj.fm, sj.g, slot, far);
+            if (slot < nf) acc = lb_cell<L, M, batch_staged<L, M, F>()>(lat, job_constants<UNI>(kcu, sj.kc), slot, far);
             if (check) block_sum_store(acc, sj.partials + b);
         }
         if (!advance) {  // uniform over the block
@@ -110,10 +125,11 @@ __global__ void __launch_bounds__(kFlowThreads, M::batch_min_blocks)
 }
 
 template <class L, class M>
-static int occupancy_t() {
+static int occupancy_t(bool table) {
     int nb = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, batch_flow_kernel<L, M, false>,
-                                                      kFlowThreads, 0) != cudaSuccess) {
+    auto kern = table ? batch_flow_kernel<L, M, false, Far::table>
+                      : batch_flow_kernel<L, M, false, Far::packed>;
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&nb, kern, kFlowThreads, 0) != cudaSuccess) {
         cudaGetLastError();
         return 1;
     }
@@ -123,7 +139,7 @@ static int occupancy_t() {
 template <class L, class M>
 static cudaError_t launch_batch_t(const FlowJob* jobs, const BatchTile* tiles, const int* ntiles,
                                   const long long* gstep, int k, const LbParams* uniform,
-                                  int grid, cudaStream_t s) {
+                                  bool table, int grid, cudaStream_t s) {
     cudaLaunchConfig_t cfg = {};
     cfg.gridDim = dim3(grid);
     cfg.blockDim = dim3(kFlowThreads);
@@ -138,11 +154,12 @@ static cudaError_t launch_batch_t(const FlowJob* jobs, const BatchTile* tiles, c
     // solves ran 56.9k solves/h with it against 52.3k with the release at
     // the start (one run each)
     const int late = pdl_late(true) ? 1 : 0;
-    if (uniform)
-        return cudaLaunchKernelEx(&cfg, batch_flow_kernel<L, M, true>, jobs, tiles, ntiles, gstep,
-                                  k, *uniform, late);
-    return cudaLaunchKernelEx(&cfg, batch_flow_kernel<L, M, false>, jobs, tiles, ntiles, gstep, k,
-                              LbParams{}, late);
+    auto kern = uniform ? (table ? batch_flow_kernel<L, M, true, Far::table>
+                                 : batch_flow_kernel<L, M, true, Far::packed>)
+                        : (table ? batch_flow_kernel<L, M, false, Far::table>
+                                 : batch_flow_kernel<L, M, false, Far::packed>);
+    return cudaLaunchKernelEx(&cfg, kern, jobs, tiles, ntiles, gstep, k,
+                              uniform ? *uniform : LbParams{}, late);
 }
 
 
@@ -160,8 +177,8 @@ static cudaError_t launch_batch_t(const FlowJob* jobs, const BatchTile* tiles, c
 
 cudaError_t batch_launch_flow(int nd, int precision, const FlowJob* jobs, const BatchTile* tiles,
                               const int* ntiles, const long long* gstep, int k,
-                              const LbParams* uniform, int grid, cudaStream_t s) {
-    PRT_BATCH_DISPATCH(launch_batch_t, jobs, tiles, ntiles, gstep, k, uniform, grid, s)
+                              const LbParams* uniform, bool table, int grid, cudaStream_t s) {
+    PRT_BATCH_DISPATCH(launch_batch_t, jobs, tiles, ntiles, gstep, k, uniform, table, grid, s)
 }
 
 __global__ void batch_gstep_kernel(long long* gstep, int k) { *gstep += k; }
@@ -171,7 +188,9 @@ cudaError_t batch_launch_gstep(long long* gstep, int k, cudaStream_t s) {
     return cudaGetLastError();
 }
 
-int batch_flow_occupancy(int nd, int precision) { PRT_BATCH_DISPATCH(occupancy_t) }
+int batch_flow_occupancy(int nd, int precision, bool table) {
+    PRT_BATCH_DISPATCH(occupancy_t, table)
+}
 
 // out[i] = *done_ptrs[i]: the done flags of every job of a batch in one copy.
 __global__ void batch_status_kernel(const int* const* __restrict__ done_ptrs, int n,

@@ -22,10 +22,12 @@ namespace prt {
 namespace {
 constexpr int kBatchAdrThreads = kBatchAdrBlock;
 constexpr int kWarps = kBatchAdrThreads / 32;
-// four resident blocks (64 registers): measured against 5, 6 and 8, which
-// spill in the voxel step (32.1 against 33.8, 35.1 and 41.8 us a step for
-// 48 small transport runs); without a bound the step takes 80-95 registers
-constexpr int kBatchAdrMinBlocks = 4;
+// Resident blocks: four (64 registers) while the voxel step spills little; with
+// three chemicals or more it takes 80 (16 four-chemical runs of edges 24-48:
+// 21.3 -> 17.5 us a step; two chemicals 12 runs of edges 60-90: 67 at four
+// blocks, 72 at three).
+template <int NS>
+__host__ __device__ constexpr int adr_blocks() { return NS < 3 ? 4 : 3; }
 }
 
 // The leaves of block b of job J on a check step n, after the block's
@@ -111,8 +113,16 @@ __device__ __noinline__ void job_step_end(const AdrJob& J, long long n, long lon
     }
 }
 
+// voxel_setup in the form of job J.
+template <int ND>
+__device__ __forceinline__ VoxelSetup<ND> job_setup(const AdrJob& J, bool bf, unsigned k) {
+    if (J.d.near == nullptr) return voxel_setup<ND, true, true>(J.d, J.p, k);
+    if (bf) return voxel_setup<ND, true, false>(J.d, J.p, k);
+    return voxel_setup<ND, false, false>(J.d, J.p, k);
+}
+
 template <int ND, int NS>
-__global__ void __launch_bounds__(kBatchAdrThreads, kBatchAdrMinBlocks)
+__global__ void __launch_bounds__(kBatchAdrThreads, adr_blocks<NS>())
     batch_adr_kernel(const AdrJob* __restrict__ jobs, const BatchTile* __restrict__ tiles,
                      const int* __restrict__ ntiles_p, const long long* __restrict__ gstep, int k,
                      int late) {
@@ -148,7 +158,7 @@ __global__ void __launch_bounds__(kBatchAdrThreads, kBatchAdrMinBlocks)
         const int done = __ldcg(&ctrl->done);
         const long long n = done_steps - J.g0 + 1;  // the step this launch takes
         const long long limit = __ldcg(&ctrl->limit);
-        const bool due = n % __ldcg(&ctrl->check) == 0;
+        const bool due = divides(__ldcg(&ctrl->check), n);
         const bool advance = due || n >= limit;
         __syncthreads();  // every thread has read the control block
         if (done) continue;
@@ -162,9 +172,9 @@ __global__ void __launch_bounds__(kBatchAdrThreads, kBatchAdrMinBlocks)
         for (int b = tl.b0; b < tl.b0 + tl.nb; ++b) {
             const unsigned k = (unsigned)b * kBatchAdrThreads + threadIdx.x;
             if (k < (unsigned)J.d.nm) {
-                if (J.d.near == nullptr) adr_voxel<ND, NS, true, true>(J.d, J.p, n, k);
-                else if (bf) adr_voxel<ND, NS, true, false>(J.d, J.p, n, k);
-                else adr_voxel<ND, NS, false, false>(J.d, J.p, n, k);
+                const VoxelSetup<ND> v = job_setup<ND>(J, bf, k);
+                if (bf) adr_voxel_step<ND, NS, true>(J.d, J.p, n, k, v);
+                else adr_voxel_step<ND, NS, false>(J.d, J.p, n, k, v);
             }
             if (due) {
                 __syncthreads();  // the block's voxels of step n are stored

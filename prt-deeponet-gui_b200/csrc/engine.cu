@@ -91,6 +91,8 @@ struct prt_batch {
     // flow classes whose jobs all share their constants (passed as a parameter)
     bool flow_uni[kFlowClasses] = {};
     LbParams flow_kc[kFlowClasses] = {};
+    // flow classes whose steps read the plain tables of far places
+    bool flow_table[kFlowClasses] = {};
     GrowBuf d_flow, d_adr, d_done, d_status, d_arrive, d_adr_cnt, d_counts;
     GrowBuf d_gstep;  // batch steps done (one long long), advanced by each replay
     GrowBuf d_tiles[kClasses];
@@ -233,6 +235,25 @@ int rebuild(prt_batch* b) {
         }
         for (int c = 0; c < kFlowClasses; ++c) b->flow_uni[c] = seen[c] && !differ[c];
     }
+    // plain tables of far places: each solve chose them against the whole L2;
+    // in a batch a class reads them while all its jobs have one and all the
+    // flow jobs' lattices and tables together fit in three quarters of it, else
+    // the packed ones (the same places, so the fields do not change)
+    {
+        long long ws = 0, l2 = 0;
+        for (int c = 0; c < kFlowClasses; ++c) b->flow_table[c] = true;
+        for (int i = 0; i < b->nflow; ++i) {
+            const prt_ctx* ctx = b->order[i];
+            const FlowState& F = ctx->flow;
+            const int q = F.p.nd == 3 ? 19 : 9;
+            const long long es = F.p.precision == PRT_FP64 ? 8 : F.p.precision == PRT_FP16 ? 2 : 4;
+            ws += (long long)q * F.fm.rs * es + flow_nbr_bytes(q, F.fm.nf);
+            l2 = ctx->l2_bytes;
+            if (!F.fm.nbr && F.fm.nf > 0) b->flow_table[flow_class(F.p.nd, F.p.precision)] = false;
+        }
+        if (ws > l2 / 4 * 3)
+            for (int c = 0; c < kFlowClasses; ++c) b->flow_table[c] = false;
+    }
     const int njobs = (int)b->order.size();
     BK(b->d_arrive.fit((size_t)std::max(b->nflow, 1) * sizeof(unsigned)));
     for (int i = 0; i < b->nflow; ++i) b->h_flow[i].arrive = b->d_arrive.b.as<unsigned>() + i;
@@ -286,7 +307,7 @@ int rebuild(prt_batch* b) {
             continue;
         }
         int occ = 1;
-        if (c < kFlowClasses) occ = batch_flow_occupancy(c >= 4 ? 3 : 2, c % 4);
+        if (c < kFlowClasses) occ = batch_flow_occupancy(c >= 4 ? 3 : 2, c % 4, b->flow_table[c]);
         else occ = batch_adr_occupancy(c >= kFlowClasses + 8 ? 3 : 2, (c - kFlowClasses) % 8 + 1);
         b->grid[c] = b->grid_mult == 0 ? nt
                                        : std::max(1, std::min(nt, b->grid_mult * occ * b->nsm));
@@ -310,7 +331,8 @@ cudaError_t emit_step(prt_batch* b, cudaStream_t s, const cudaStream_t* streams,
             e = batch_launch_flow(c >= 4 ? 3 : 2, c % 4, b->d_flow.b.as<FlowJob>(),
                                   b->d_tiles[c].b.as<BatchTile>(), counts + c,
                                   b->d_gstep.b.as<long long>(), k,
-                                  b->flow_uni[c] ? &b->flow_kc[c] : nullptr, b->grid[c], sc);
+                                  b->flow_uni[c] ? &b->flow_kc[c] : nullptr, b->flow_table[c],
+                                  b->grid[c], sc);
         } else {
             const int a = c - kFlowClasses;
             e = batch_launch_adr(a >= 8 ? 3 : 2, a % 8 + 1, b->d_adr.b.as<AdrJob>(),
@@ -336,6 +358,7 @@ int ensure_graph(prt_batch* b) {
     for (int c = 0; c < kClasses; ++c) key.push_back(b->grid[c]);
     for (int c = 0; c < kFlowClasses; ++c) {  // constants baked into the launches
         key.push_back(b->flow_uni[c]);
+        key.push_back(b->flow_table[c]);
         if (!b->flow_uni[c]) continue;
         long long w[(sizeof(LbParams) + 7) / 8] = {};
         std::memcpy(w, &b->flow_kc[c], sizeof(LbParams));

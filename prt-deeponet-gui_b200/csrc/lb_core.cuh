@@ -505,13 +505,13 @@ __device__ __forceinline__ void collide_store(const Lat<typename M::S>& lat0, in
 
 // One pore voxel (slot k) of one LB iteration, its far places already found:
 // gather, moments, collision, store; returns |u_x| for the convergence mean.
-template <class L, class M>
+template <class L, class M, bool STAGED = M::staged && L::Q == 19>
 __device__ __forceinline__ double lb_cell(const Lat<typename M::S>& lat, const LbParams& kc, int k,
                                           const int (&far)[L::NP]) {
     using S = typename M::S;
     using R = typename M::R;
     using RA = typename M::RA;
-    if constexpr (M::staged && L::Q == 19) {
+    if constexpr (STAGED) {
         __shared__ S stage[L::Q * kFlowThreads];
         S* col = stage + threadIdx.x;
         gather_staged<L, S>(lat, k, far, col);

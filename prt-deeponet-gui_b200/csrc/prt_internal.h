@@ -481,6 +481,11 @@ __device__ __forceinline__ void block_copy(T* dst, const T* src) {
     for (int i = threadIdx.x; i < (int)(sizeof(T) / 8); i += blockDim.x) d[i] = s[i];
 }
 
+// Whether c divides n >= 0 (64-bit division only where n needs it).
+__device__ __forceinline__ bool divides(int c, long long n) {
+    return (n >> 32) == 0 ? (unsigned)n % (unsigned)c == 0u : n % c == 0;
+}
+
 // The contiguous range of work-list entries block b of g handles, so that
 // consecutive tiles of a block mostly belong to one job.
 __device__ __forceinline__ void tile_range(int n, int& t0, int& t1) {
@@ -496,11 +501,12 @@ __device__ __forceinline__ void tile_range(int n, int& t0, int& t1) {
 // the current graph replay) and their step's place k in the replay; a job's
 // own count is that plus k minus its g0, so its control block is written
 // only on the steps that sample, check or end it.
-// uniform: the constants every job of the launch shares, or null.
+// uniform: the constants every job of the launch shares, or null; table: every
+// job has the plain table of far places.
 cudaError_t batch_launch_flow(int nd, int precision, const FlowJob* jobs, const BatchTile* tiles,
                               const int* ntiles, const long long* gstep, int k,
-                              const LbParams* uniform, int grid, cudaStream_t s);
-int batch_flow_occupancy(int nd, int precision);
+                              const LbParams* uniform, bool table, int grid, cudaStream_t s);
+int batch_flow_occupancy(int nd, int precision, bool table);
 cudaError_t batch_launch_adr(int nd, int ns, const AdrJob* jobs, const BatchTile* tiles,
                              const int* ntiles, const long long* gstep, int k, int grid,
                              cudaStream_t s);

@@ -48,7 +48,7 @@ __global__ void __launch_bounds__(kAdrThreads) adr_step_kernel(AdrDev d, prt_adr
     if (live) s = voxel_setup<ND, BF, WIDE>(d, p, k);
     griddep_wait();
     const long long n = ctrl->n_base + kstep + 1;
-    if (ctrl->done || n > ctrl->limit) return;  // uniform over the grid
+    if (ctrl->done || n > ctrl->n_stop) return;  // uniform over the grid
     if (!live) return;
     adr_voxel_step<ND, NS, BF>(d, p, n, k, s);
     if (late) griddep_launch_dependents();
@@ -306,12 +306,12 @@ __global__ void __launch_bounds__(kTreeThreads)
     tree_means(t, nm, ns, vals, means);
 }
 
-// The leaves of the state at the end of the current chunk, when its means are
-// due.
+// The leaves of the state at the end of the current segment, when its means
+// are due.
 __global__ void __launch_bounds__(kLeafThreads)
     chunk_leaf_kernel(const AdrCtrl* __restrict__ ctrl, AdrDev d) {
     if (ctrl->done) return;
-    const long long end = min(ctrl->n_base + (long long)ctrl->check, ctrl->limit);
+    const long long end = ctrl->n_stop;
     if (end % ctrl->check != 0) return;
     block_of_leaves(d.buf[end & 1], d.ms, (unsigned)d.n0, (unsigned)d.nm, d.tree, d.ns, d.tree_vals);
 }
@@ -325,14 +325,14 @@ __global__ void __launch_bounds__(kTreeThreads)
         if (use_handle && threadIdx.x == 0) cudaGraphSetConditional(h, 0);
         return;
     }
-    const long long base = ctrl->n_base;
-    const long long end = min(base + (long long)ctrl->check, ctrl->limit);
-    const bool due = end > base && end % ctrl->check == 0;
+    const long long end = ctrl->n_stop;
+    const bool due = end > ctrl->n_base && end % ctrl->check == 0;
     if (due) tree_means(d.tree, d.nm, d.ns, d.tree_vals, means);
     __syncthreads();  // the means are written, and every thread has read ctrl
     if (threadIdx.x != 0) return;
     if (due) adr_check(ctrl, means, end, d.log, d.log_cap);
     ctrl->n_base = end;
+    ctrl->n_stop = segment_end(end, ctrl->segment, ctrl->check, ctrl->limit);
     if (end >= ctrl->limit) ctrl->done = 1;
     const int go = (!ctrl->done && end < ctrl->n_pause) ? 1 : 0;
     if (use_handle) cudaGraphSetConditional(h, go);

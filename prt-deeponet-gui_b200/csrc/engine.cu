@@ -687,6 +687,7 @@ extern "C" int prt_batch_remove(prt_batch* b, prt_ctx* job) {
             BK(cudaStreamSynchronize(s));
             if (!ac.done) {
                 ac.n_base = count;
+                ac.n_stop = segment_end(count, ac.segment, ac.check, ac.limit);
                 BK(cudaMemcpyAsync(job->adr.ctrl.p, &ac, sizeof(ac), cudaMemcpyHostToDevice, s));
                 BK(cudaStreamSynchronize(s));
             }

@@ -154,6 +154,7 @@ struct AdrCtrl {
     long long n_base;  // steps completed before the current chunk
     long long limit;
     long long n_pause;  // host asked to regain control at this step
+    long long n_stop;   // the current segment of the loop ends at this step
     long long checks;
     int check;
     int until_conv;
@@ -161,12 +162,23 @@ struct AdrCtrl {
     int converged;
     int ns;
     int nlog;
+    int segment;  // steps of a loop segment at most
+    int pad;
     double tol;
     double last_rest;
     double prev[PRT_MAX_SPECIES];
     double prev_change[PRT_MAX_SPECIES];
     double scale[PRT_MAX_SPECIES];
 };
+
+// Where the segment after `base` steps ends: a full segment on, the next check
+// or the limit.
+__host__ __device__ inline long long segment_end(long long base, int segment, int check,
+                                                 long long limit) {
+    long long end = (base / check + 1) * check;
+    if (end > base + segment) end = base + segment;
+    return end < limit ? end : limit;
+}
 
 struct ProgressRec {
     long long n;

@@ -662,6 +662,16 @@ static cudaError_t copy_rows(const AdrState& A, const DevBuf& buf, int slot, cud
                            A.ladder.as<float>() + (size_t)A.d.nm * A.p.ns * slot, s);
 }
 
+// Steps of the transport loop's graph body: the steps between two checks in
+// equal parts of at most kSegment.  The check interval grows as 1 / Pe (7000
+// steps at Pe 1 on 700 voxels) and a graph costs about 8 us a node to build,
+// which had been more than the run itself; a segment end costs about 4 us.
+constexpr int kSegment = 128;
+static int loop_segment(int check) {
+    const int parts = (check + kSegment - 1) / kSegment;
+    return (check + parts - 1) / parts;
+}
+
 // Transport time loop in three parts (see flow_setup): the ladder and the
 // control block, the loop, and the kept snapshots.
 int prt::adr_run_setup(prt_ctx* ctx, const prt_adr_run_params* rp, long long pause_every) {
@@ -715,6 +725,8 @@ int prt::adr_run_setup(prt_ctx* ctx, const prt_adr_run_params* rp, long long pau
         hc.scale[j] = 1e-6;
     }
     hc.n_pause = std::min(limit, pause_every);
+    hc.segment = A.segment = loop_segment(rp->check);
+    hc.n_stop = segment_end(0, hc.segment, hc.check, limit);
     hc.done = limit == 0 ? 1 : 0;
     CK(cudaMemcpyAsync(A.ctrl.p, &hc, sizeof(hc), cudaMemcpyHostToDevice, s));
     CK(cudaStreamSynchronize(s));  // the host vector above goes out of scope
@@ -757,14 +769,14 @@ int prt::adr_run_finish(prt_ctx* ctx, prt_adr_result* res) {
     return PRT_OK;
 }
 
-// The transport loop's graph body: `check` step kernels, the numpy-order
-// means of the chunk's last step and the stop rule (which sets the WHILE
-// condition when h is used).
+// The transport loop's graph body: a segment of step kernels, then, where its
+// end is due for a check, the numpy-order means and the stop rule (which sets
+// the WHILE condition when h is used).
 static cudaError_t adr_emit(prt_ctx* ctx, cudaGraphConditionalHandle h, int use) {
     AdrState& A = ctx->adr;
     AdrCtrl* dctrl = A.ctrl.as<AdrCtrl>();
     float* dmeans = A.means.as<float>();
-    for (int k = 0; k < A.rp.check; ++k) {
+    for (int k = 0; k < A.segment; ++k) {
         cudaError_t e = adr_launch_step(A.d, A.p, dctrl, k, ctx->stream);
         if (e != cudaSuccess) return e;
     }
@@ -777,7 +789,7 @@ static cudaError_t adr_emit(prt_ctx* ctx, cudaGraphConditionalHandle h, int use)
 static std::vector<unsigned char> adr_graph_key(prt_ctx* ctx) {
     AdrState& A = ctx->adr;
     const void* ptrs[2] = {A.means.p, A.ctrl.p};
-    const int ints[2] = {A.rp.check, pdl_key()};
+    const int ints[2] = {A.segment, pdl_key()};
     std::vector<unsigned char> k(sizeof(AdrDev) + sizeof(prt_adr_params) + sizeof(ptrs) +
                                  sizeof(ints));
     unsigned char* q = k.data();
@@ -827,8 +839,9 @@ int prt::adr_loop_async(prt_ctx* ctx) {
             return PRT_OK;
         }
         CK(adr_graph(ctx));
+        const long long per_check = (A.rp.check + A.segment - 1) / A.segment;
         const long long chunks =
-            A.graph.conditional ? 1 : (A.rp.limit + A.rp.check - 1) / A.rp.check;
+            A.graph.conditional ? 1 : (A.rp.limit + A.rp.check - 1) / A.rp.check * per_check;
         for (long long r = 0; r < chunks; ++r) CK(cudaGraphLaunch(A.graph.exec, s));
     }
     CK(cudaEventRecord(ctx->ev[3], s));
@@ -847,12 +860,12 @@ extern "C" int prt_adr_run(prt_ctx* ctx, const prt_adr_run_params* rp, prt_progr
     const long long limit = rp->limit;
     const int log_cap = A.d.log_cap;
     AdrCtrl* dctrl = A.ctrl.as<AdrCtrl>();
-    const int check = rp->check;
+    const int seg = A.segment;
     const AdrDev D = A.d;
     auto emit = [&](cudaGraphConditionalHandle h, int use) -> cudaError_t {
         return adr_emit(ctx, h, use);
     };
-    const int per_chunk = check + 1 + (D.tree.nleaf > 0 ? 1 : 0);
+    const int per_chunk = seg + 1 + (D.tree.nleaf > 0 ? 1 : 0);
     std::vector<ProgressRec> logbuf;
     int delivered = 0;
     AdrCtrl cur;
@@ -889,7 +902,7 @@ extern "C" int prt_adr_run(prt_ctx* ctx, const prt_adr_run_params* rp, prt_progr
         CK(cudaMemcpyAsync(&cur, dctrl, sizeof(cur), cudaMemcpyDeviceToHost, s));
         CK(cudaStreamSynchronize(s));
         if (!cluster && use_graph && A.graph.conditional)
-            ctx->launches += (cur.n_base - before + check - 1) / check * per_chunk;
+            ctx->launches += (cur.n_base - before + seg - 1) / seg * per_chunk;
         if (cb && cur.nlog > delivered) {
             const int nrec = std::min(cur.nlog, log_cap) - delivered;
             logbuf.resize(nrec);

@@ -136,6 +136,7 @@ struct AdrState {
     const uint8_t* d_mat = nullptr;  // staged inputs (borrowed until begin)
     const float* d_vel = nullptr;
     DevBuf tmp, vstats;
+    int segment = 1;                    // steps of the run's graph body
     std::vector<long long> sched;       // ladder step schedule of the run
     prt_adr_run_params rp{};
     std::vector<long long> keep_steps;  // ladder step numbers

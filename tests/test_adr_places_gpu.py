@@ -138,3 +138,27 @@ def test_cluster_loop_is_the_launches(monkeypatch, shape, kind):
         assert np.array_equal(found[0][0], found[1][0])
         assert np.array_equal(found[0][1], found[1][1])
         assert found[0][2:] == found[1][2:]
+
+
+def test_long_check_intervals_run_in_segments(monkeypatch):
+    """At a low Peclet number the check interval (here 1 500 steps) exceeds a
+    graph body, so a check follows several segments; the stop step, the
+    progress records and the fields are those of direct launches, of one
+    cluster, and of the oracle's step rule."""
+    from oracle.prtlb_oracle import solve_adr as reference
+    g = np.full((24, 20), 2, np.uint8)
+    g[5::7, ::3] = 0
+    v = integer_velocity(g)
+    kw = dict(pe=0.16, da=2.0, n_t=3, n_species=1, max_steps=3100, chem=chemistry("monod")[0])
+    with contextlib.redirect_stdout(io.StringIO()):
+        said = []
+        want, _ = reference(g, v, kw["pe"], kw["da"], 3, n_species=1, max_steps=3100,
+                            chem=kw["chem"], on_progress=lambda *a: said.append(a))
+    assert len(said) == 2 and said[0][0] > 1000
+    for cluster, graphs in (("0", "1"), ("0", "0"), ("1", "1")):
+        monkeypatch.setenv("PRT_CLUSTER", cluster)
+        monkeypatch.setenv("PRT_GRAPHS", graphs)
+        seen = []
+        out, _ = solve(g, v, dict(kw, on_progress=lambda *a: seen.append(a)))
+        assert np.array_equal(out, want)
+        assert [a[0] for a in seen] == [a[0] for a in said]

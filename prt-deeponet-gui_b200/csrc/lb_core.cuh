@@ -479,13 +479,13 @@ __device__ __forceinline__ void collide_mode(const HA& h,
 
 // The collision of slot k with its results stored in the lattice: f_a to the
 // pair's far place and f_b to its own (see Lat).
-template <class L, class M, class HA>
+template <class L, class M, bool INDEX, class HA>
 __device__ __forceinline__ void collide_store(const Lat<typename M::S>& lat0, int k,
                                               const int (&far)[L::NP], const HA& h,
                                               const Moments<typename M::R, typename M::RA>& m,
                                               const LbParams& kc) {
     using S = typename M::S;
-    constexpr Fresh F = L::Q == 19 ? M::fresh : Fresh::none;
+    constexpr Fresh F = INDEX ? Fresh::index : L::Q == 19 ? M::fresh : Fresh::none;
     Lat<S> lat = lat0;
     int to[L::NP];
     if (F == Fresh::base) asm volatile("" : "+l"(lat.f));
@@ -505,7 +505,8 @@ __device__ __forceinline__ void collide_store(const Lat<typename M::S>& lat0, in
 
 // One pore voxel (slot k) of one LB iteration, its far places already found:
 // gather, moments, collision, store; returns |u_x| for the convergence mean.
-template <class L, class M, bool STAGED = M::staged && L::Q == 19>
+// INDEX: the store addresses from the slot numbers whatever the mode's Fresh.
+template <class L, class M, bool STAGED = M::staged && L::Q == 19, bool INDEX = false>
 __device__ __forceinline__ double lb_cell(const Lat<typename M::S>& lat, const LbParams& kc, int k,
                                           const int (&far)[L::NP]) {
     using S = typename M::S;
@@ -518,13 +519,13 @@ __device__ __forceinline__ double lb_cell(const Lat<typename M::S>& lat, const L
         cp_async_wait<0>();
         const Staged<S> h{col};
         const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(kc));
-        collide_store<L, M>(lat, k, far, h, m, kc);
+        collide_store<L, M, INDEX>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     } else {
         typename Pop<S>::H h[L::Q];
         gather<L, S>(lat, k, far, kc.inv_scale, h);
         const Moments<R, RA> m = moments<L, R, RA>(h, half_force<RA>(kc));
-        collide_store<L, M>(lat, k, far, h, m, kc);
+        collide_store<L, M, INDEX>(lat, k, far, h, m, kc);
         return fabs((double)m.jx * (double)m.inv_rho);
     }
 }

@@ -45,8 +45,10 @@ namespace prt {
 // 96^3 float64 27.1 -> 16.2, float32 11.8 -> 10.7, 64^3 unchanged within 5 %.
 // A grid of one wave whose threads overlap the next voxel's loads with this
 // one's collision (two cp.async stages) was slower beyond the L2 (192^3 122).
-template <class L, class M, Far F, bool ODD, bool CHECK>
-__global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
+// REG: the form of a D3Q19 float64 step that gathers into registers, four
+// blocks an SM (see launch_step_one).
+template <class L, class M, Far F, bool ODD, bool CHECK, bool REG>
+__global__ void __launch_bounds__(kFlowThreads, REG ? 4 : M::min_blocks)
     lb_step_kernel(typename M::S* __restrict__ f, FlowMap fm, Grid g, LbParams kc,
                    const FlowCtrl* __restrict__ ctrl, int kstep, double* __restrict__ partials,
                    int late, int turn) {
@@ -63,7 +65,7 @@ __global__ void __launch_bounds__(kFlowThreads, M::min_blocks)
     if (ctrl->done || it >= ctrl->nit) return;  // uniform over the grid
     double acc = 0.0;
     if (k < fm.nf) {
-        const double ux = lb_cell<L, M>(lat, kc, k, far);
+        const double ux = lb_cell<L, M, M::staged && L::Q == 19 && !REG, REG>(lat, kc, k, far);
         if (CHECK) acc = ux;
     }
     if (CHECK) block_sum_store(acc, partials + b);
@@ -361,8 +363,19 @@ static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Gr
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() ? 1 : 0;
-    auto kern = fm.nbr ? lb_step_kernel<L, M, Far::table, ODD, CHECK>
-                       : lb_step_kernel<L, M, Far::packed, ODD, CHECK>;
+    // D3Q19 float64 stages its gather in shared memory, because in registers it
+    // takes 118 of them; a solve whose blocks all fit at four an SM has the
+    // registers (54^3: 4.16 -> 3.94 us an iteration, 44^3 3.23 -> 3.07; beyond
+    // one such wave it loses, 60^3 5.3 against 5.6).
+    if constexpr (M::staged && L::Q == 19) {
+        auto reg = lb_step_kernel<L, M, Far::table, ODD, CHECK, true>;
+        static const long long wave = resident_blocks(reg);
+        if (fm.nbr && nb <= wave)
+            return cudaLaunchKernelEx(&cfg, reg, f, fm, g, k, ctrl, kstep, partials,
+                                      pdl_late(true) ? 1 : 0, 0);
+    }
+    auto kern = fm.nbr ? lb_step_kernel<L, M, Far::table, ODD, CHECK, false>
+                       : lb_step_kernel<L, M, Far::packed, ODD, CHECK, false>;
     // both forms are held to the same register budget
     static const long long resident = resident_blocks(kern);
     const bool one_wave = nb <= resident;

@@ -21,7 +21,7 @@ e2e    the same through the public drop-in API (stokes_d3q19 + solve_adr on
        host numpy arrays), host<->device copies inside the timed region.
 roofline  the dominant kernel (the D3Q19 stream-collide) against the measured
        HBM copy bandwidth: algorithmic bytes = 152 B per pore voxel (19
-       float32 read + written) + 1 B mask per voxel, per iteration.
+       float32 read + written), per iteration.
 cpu_baseline  the NumPy oracle (a restatement of the reference's algorithm)
        on a bounded sample of the same workload, one core.
 
@@ -65,10 +65,10 @@ SEED = 0
 FORCE, TAU, FLOW_TOL, FLOW_NIT = 2e-6, 0.8, 1e-6, 30000
 ADR_STEPS = None  # None: run to the reference's stop rule
 # DRAM bytes (read + write) of one lb_step_kernel launch from an ncu capture
-# (cache flushed before the launch), by grid edge.  At 64^3 they include the
-# upstream-slot table (72 B per pore voxel, 8.4 MB), which the solve reads
-# instead of the voxel map because its working set fits in L2.
-TRAFFIC_PER_LAUNCH = {64: 25157632, 128: 176652032}
+# (cache flushed before the launch), by grid edge.  They include the table of
+# far places (36 B per pore voxel at 64^3, 14.3 B at 128^3); part of the
+# writes is still in the L2 when the kernel ends.
+TRAFFIC_PER_LAUNCH = {64: 13801472, 128: 112765184}
 PE, DA, KS, N_T = 10.0, 1.0, 0.5, 5
 # float32 populations collided in float32 (the "fp32" mode keeps the
 # momentum in float64); float64 only for the residual and the integrals
@@ -76,8 +76,8 @@ PRECISION = "fp32f"
 METRIC = "D3Q19 TRT+ADR GLUPS"
 UNIT = "GLUPS"
 LB_BYTES_PER_FLUID = 19 * 4 * 2  # float32 populations read + written
-# one solute: C read and written, three face velocities, flags, list index
-ADR_BYTES_PER_SOLUTE = 4 + 4 + 12 + 4 + 4
+# one solute: C read and written, three face velocities
+ADR_BYTES_PER_SOLUTE = 4 + 4 + 12
 WORKLOAD = ("plain-3d: 64^3 sphere pack (r U[4,7], porosity 0.45, seed 0), D3Q19 TRT fp32 "
             "to tol 1e-6 + Monod ADR (Ks 0.5) Pe 10 Da 1 to the stop rule")
 
@@ -308,21 +308,20 @@ def run_ours(args, rank, world, torch, dist):
     fl_ms = statistics.mean(flow_ms)
     ad_ms = statistics.mean(adr_ms)
     per_launch_ms = fl_ms / max(iters[0], 1)
-    lb_bytes = nfluid * LB_BYTES_PER_FLUID + 4 * ncell
+    lb_bytes = nfluid * LB_BYTES_PER_FLUID
     achieved = lb_bytes / (per_launch_ms * 1e-3) / 1e9
     peak, kind = peaks()
     roof = {"kernel": "lb_step_kernel<D3Q19,ModeF32>", "bound": "hbm",
-            "regime": "L2-resident (two lattices + slot table = 26 MB < 126 MB L2): "
+            "regime": "L2-resident (lattice + table of far places = 15 MB < 126 MB L2): "
                       "latency-bound, not DRAM-bound; see side.dram_128 for the "
                       "DRAM-resident figures",
             "achieved": round(achieved, 1), "peak": peak, "unit": "GB/s",
             "frac": round(achieved / peak, 4), "peak_kind": kind,
             "bytes_per_iteration": lb_bytes, "traffic": TRAFFIC_PER_LAUNCH.get(EDGE),
-            "note": "algorithmic bytes = 152 B per pore voxel (19 float32 read + written) + "
-                    "4 B voxel map per voxel, per iteration; time per iteration = flow loop "
-                    "events / iterations (one launch per iteration, graph node gaps "
-                    "included); traffic = DRAM bytes of one cold-cache iteration (the slot "
-                    "table read instead of the map)"}
+            "note": "algorithmic bytes = 152 B per pore voxel (19 float32 read + written) "
+                    "per iteration; time per iteration = flow loop events / iterations "
+                    "(one launch per iteration, graph node gaps included); traffic = DRAM "
+                    "bytes of one cold-cache iteration (the table of far places included)"}
     res = {"ms_per_step": total_ms / args.steps, "value": value, "e2e": e2e_value,
            "h2d": h2d, "d2h": d2h, "launches": launches, "roof": roof, "clocks": clk.summary(),
            "flow_ms": fl_ms, "adr_ms": ad_ms, "iters": iters[0], "adr_steps": nsteps[0],
@@ -391,7 +390,7 @@ def side_measurements(ctx, peak, kind):
                   ctx=ctx)
         ta = ctx.timing()
     fl_us = tf[0] / tf[1] * 1e3
-    fl_bytes = nf * LB_BYTES_PER_FLUID + 4 * n
+    fl_bytes = nf * LB_BYTES_PER_FLUID
     ad_us = ta[2] / ta[3] * 1e3
     ad_bytes = nf * ADR_BYTES_PER_SOLUTE
     dram = {
@@ -408,8 +407,8 @@ def side_measurements(ctx, peak, kind):
                       "achieved": round(ad_bytes / ad_us / 1e3, 1), "peak": peak, "unit": "GB/s",
                       "frac": round(ad_bytes / ad_us / 1e3 / peak, 4), "peak_kind": kind,
                       "bytes_per_launch": ad_bytes,
-                      "note": "algorithmic bytes = 28 B per solute voxel (C read + written, "
-                              "3 faces, flags, index); the kernel is bounded by instruction "
+                      "note": "algorithmic bytes = 20 B per solute voxel (C read + written, "
+                              "3 faces); the kernel is bounded by instruction "
                               "issue, not DRAM"},
     }
     g2 = disk_pack_2d(128, 0.6, SEED)

@@ -63,7 +63,12 @@ def footprint(req):
         ns = int(a["n_species"])
         limit = int(a["steps"]) if a["steps"] is not None else int(a["max_steps"])
         slots = ladder_slots(limit, float(a["ratio"]))
-        adr = n * (4 + 1 + 4 + 12 + 8 * ns) + 4 * nf * 2 + 4 * n * ns * slots + 4 * (limit + 1)
+        code = getattr(a["chem"], "biofilm_code", None)
+        nm = nf + (0 if code is None else int(np.count_nonzero(mat == code)))
+        # per voxel flags, scratch and one grid of a fetched snapshot; per solute
+        # voxel the list, neighbours, faces, flags and two states; the ladder
+        adr = n * (4 + 1 + 4 + 4 * ns) + nm * (4 + 24 + 24 + 4 + 8 * ns)
+        adr += 4 * n * ns * slots + 4 * (limit + 1)
     # the flow's small buffers stay with the context during its transport
     return common + max(flow, adr + min(flow, _FLOW_KEEP)) + (1 << 20)
 

@@ -8,9 +8,10 @@
 // smallest grids) and then by the arithmetic of the slots a block holds, about
 // 0.45 us for each further 128 slots of D3Q19 float64, 0.3 us of float32,
 // which sets the largest size taken.  us an iteration, launches -> cluster:
-// 16^3 float64 2.29 -> 1.09, 24^3 2.31 -> 1.94, 24^3 float32 2.15 -> 1.46;
-// D2Q9 64^2 float64 1.79 -> 0.82, 128^2 1.81 -> 1.26, float32 1.69 -> 0.93,
-// 150^2 float64 1.83 -> 1.61.
+// 16^3 float64 2.29 -> 1.04, 24^3 2.31 -> 1.75, 26^3 2.22 -> 1.93, 24^3 float32
+// 2.15 -> 1.30;
+// D2Q9 64^2 float64 1.79 -> 0.82, 128^2 1.81 -> 1.16, float32 1.69 ->
+// 0.86, 150^2 float64 1.83 -> 1.61.
 #include "cluster.cuh"
 #include "lb_core.cuh"
 
@@ -19,11 +20,11 @@ namespace prt {
 namespace {
 
 // Threads, hence slots, per block at most: where the launches catch up (D3Q19
-// float64 at 640 slots 2.68 against 2.32 us, at 384 1.94 against 2.31; float32
+// float64 at 640 slots 2.68 against 2.32 us, at 512 1.93 against 2.22; float32
 // at 640 1.81 against 2.15), or the registers of 1024 threads (D2Q9).
 template <class L, class M>
 constexpr int cluster_threads() {
-    return L::Q == 19 ? (sizeof(typename M::RA) == 8 ? 384 : 640) : 1024;
+    return L::Q == 19 ? (sizeof(typename M::RA) == 8 ? 512 : 640) : 1024;
 }
 
 template <class S>

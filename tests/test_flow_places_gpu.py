@@ -50,8 +50,8 @@ def grid(name):
 
 
 # voxels around what one cluster takes: one block, all 16, the most and one more
-EDGES = [("fp64", (1, 1, 128)), ("fp64", (8, 16, 16)), ("fp64", (16, 16, 24)), ("fp64", (16, 16, 25)),
-         ("fp32", (16, 16, 24)), ("fp32f", (16, 32, 20)), ("fp16", (10, 32, 32)), ("fp64", (128, 128)),
+EDGES = [("fp64", (1, 1, 128)), ("fp64", (8, 16, 16)), ("fp64", (16, 16, 32)), ("fp64", (16, 16, 33)),
+         ("fp32", (16, 16, 32)), ("fp32f", (16, 32, 20)), ("fp16", (10, 32, 32)), ("fp64", (128, 128)),
          ("fp32f", (129, 127)), ("fp64", (128, 129))]
 
 

@@ -1,6 +1,6 @@
 // batch_adr.cu -- the transport time loop of many solves per launch.
-// Built with -fmad=false like adr.cu: the per-voxel step is adr_voxel, the
-// check means are the numpy pairwise leaves and tree_mean and the stop rule
+// Built with -fmad=false like adr.cu: the per-voxel step is adr_voxel_step, the
+// check means are the numpy pairwise leaves and tree_means and the stop rule
 // is adr_check, so a job's snapshots and step count are bit-identical to the
 // single-solve loop.
 //

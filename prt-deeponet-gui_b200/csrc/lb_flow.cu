@@ -325,14 +325,12 @@ __global__ void nbr_fill_kernel(FlowMap fm, Grid g, int* __restrict__ nbr) {
 // -------------------------------------------------------------------------
 int flow_blocks(long long n) { return (int)((n + kFlowThreads - 1) / kFlowThreads); }
 
-// Step kernels go out with programmatic stream serialisation (pdl_enabled,
-// lb_core.cuh): kernel t+1 starts launching while kernel t drains, finds its
-// far places (the maps do not change during a solve) and waits in
-// griddepcontrol.wait for t's results.  Measured on the B200 with 128-thread
-// blocks: 64^3 float32 4.89 -> 4.82 us per iteration, float16 4.43 -> 4.18,
-// 128^3 float32 41.3 -> 40.6.  A grid of one resident wave releases the
-// next step only after its stores (pdl_late): 64^3 float32 collision
-// 4.60 -> 4.09 us.
+// Step kernels go out with programmatic stream serialisation: kernel t+1 starts
+// launching while kernel t drains, finds its far places (the tables do not
+// change during a solve) and waits in griddepcontrol.wait for t's results
+// (launched plainly 64^3 float32 takes 4.52 us an iteration, 54^3 float64
+// 4.20, against 4.03 and 3.92).  A grid of one resident wave releases the next
+// step only after its stores (pdl_late).
 
 // Blocks of `kern` the device holds at once.
 template <class K>

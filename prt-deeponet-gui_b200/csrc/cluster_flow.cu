@@ -89,7 +89,8 @@ __device__ __forceinline__ double cluster_cell(uint32_t own, const uint32_t (&fa
 
 // Block r of the cluster holds the slots [r span, (r + 1) span), one per
 // thread; element t of row i is slot r span + t, element T + t the place of
-// the thread's link of the pair (the row far places lie in).
+// the thread's link of the pair (the row far places lie in).  The solve is at
+// iteration 0, where the whole lattice is 0.
 template <class L, class M, int T>
 __global__ void __launch_bounds__(T, 1)
     lb_cluster_kernel(typename M::S* __restrict__ f, FlowMap fm, Grid g, LbParams kc, FlowCtrl* ctrl,

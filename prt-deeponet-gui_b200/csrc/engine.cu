@@ -656,6 +656,7 @@ extern "C" int prt_batch_add(prt_batch* b, prt_ctx* job) {
     b->jobs.push_back(job);
     job->batch = b;
     job->batch_c0 = c0;
+    job->flow.fresh = false;
     job->batch_g0_set = false;
     b->dirty = true;
     return PRT_OK;

@@ -100,6 +100,7 @@ struct FlowState {
     const uint8_t* d_mat = nullptr;  // material grid of the solve (borrowed)
     float* d_vel = nullptr;          // its output field (borrowed)
     bool field_ready = false;        // d_vel holds the final field
+    bool fresh = false;              // set up, and no loop or batch has had it yet
     // Ends the flow phase of a solve that goes on to its transport.  Device
     // buffers of at most keep_bytes stay with the context for its next solve
     // (set-up sizes them with ensure() and initialises what it reads), so a

@@ -679,6 +679,7 @@ extern "C" int prt_batch_remove(prt_batch* b, prt_ctx* job) {
             if (!fc.done) {
                 fc.it_base = count;
                 fc.iters = count;
+                job->flow.at = count;
                 BK(cudaMemcpyAsync(job->flow.ctrl.p, &fc, sizeof(fc), cudaMemcpyHostToDevice, s));
                 BK(cudaStreamSynchronize(s));
             }

@@ -72,24 +72,25 @@ __global__ void __launch_bounds__(kFlowThreads, REG ? 4 : M::min_blocks)
     if (late) griddep_launch_dependents();
 }
 
-// FlowConvergence.done() at the end of a chunk of `every` iterations
-// (prtlb_3d.py:220-235).  Also decides whether the while-graph goes on.
+// FlowConvergence.done() at the end of a chunk, the next multiple of `every` or
+// the cap (prtlb_3d.py:220-235).  Also decides whether the while-graph goes on.
 __global__ void flow_check_kernel(FlowCtrl* ctrl, const double* __restrict__ partials, int nb,
                                   cudaGraphConditionalHandle h, int use_handle) {
     const int done_before = ctrl->done;
     const long long base = ctrl->it_base;
-    const long long end = min(base + (long long)ctrl->every, ctrl->nit);
-    const bool full = (end - base) == ctrl->every;
-    // the partials of the chunk's last iteration are summed at every full
-    // chunk: for the convergence mean and the non-finite stop
+    const long long next = (base / ctrl->every + 1) * ctrl->every;
+    const long long end = min(next, ctrl->nit);
+    const bool sample = end == next;
+    // the partials of the sampled iteration are summed for the convergence
+    // mean and the non-finite stop
     double s = 0.0;
-    if (!done_before && full) s = block_sum_fixed(partials, nb);
+    if (!done_before && sample) s = block_sum_fixed(partials, nb);
     if (threadIdx.x != 0) return;
     if (done_before) {
         if (use_handle) cudaGraphSetConditional(h, 0);
         return;
     }
-    flow_ctrl_advance(ctrl, end, full && (end % ctrl->every) == 0, s);
+    flow_ctrl_advance(ctrl, end, sample, s);
     if (use_handle) cudaGraphSetConditional(h, ctrl->done ? 0 : 1);
 }
 

@@ -226,6 +226,7 @@ int prt::flow_setup(prt_ctx* ctx, const uint8_t* d_mat, const prt_flow_params* p
     F.d_vel = d_vel;
     F.field_ready = false;
     F.fresh = true;
+    F.at = 0;
     return PRT_OK;
 }
 
@@ -322,6 +323,25 @@ static cudaError_t flow_cluster(prt_ctx* ctx) {
                                F.partials.as<double>(), F.nb, ctx->stream);
 }
 
+// The iterations up to the next sampled one, for a solve that left a batch
+// between two: the loop's graph has the row parity and the sampled iteration
+// of a count that is a multiple of `every`.
+static cudaError_t flow_lead_in(prt_ctx* ctx) {
+    FlowState& F = ctx->flow;
+    const prt_flow_params& p = F.p;
+    const int n = (int)(F.at % p.every) ? p.every - (int)(F.at % p.every) : 0;
+    FlowCtrl* dctrl = F.ctrl.as<FlowCtrl>();
+    double* parts = F.partials.as<double>();
+    for (int k = 0; k < n; ++k) {
+        cudaError_t e = flow_launch_step(p.nd, p.precision, ((F.at + k) & 1) != 0, k == n - 1, F.f.p,
+                                         F.fm, F.g, F.kc, dctrl, k, parts, ctx->stream);
+        if (e != cudaSuccess) return e;
+    }
+    F.at = 0;
+    return n ? flow_launch_check(dctrl, parts, F.nb, cudaGraphConditionalHandle(0), 0, ctx->stream)
+             : cudaSuccess;
+}
+
 // Enqueues the whole flow loop of the set-up solve on the context's stream
 // without waiting (ev[0] / ev[1] bracket it): one launch of the WHILE graph,
 // or every chunk of the plain graph where conditional nodes are missing
@@ -339,6 +359,7 @@ int prt::flow_loop_async(prt_ctx* ctx) {
         }
         int rc = flow_graph(ctx);
         if (rc != PRT_OK) return rc;
+        CK(flow_lead_in(ctx));
         const long long chunks = F.graph.conditional ? 1 : (F.p.nit + F.p.every - 1) / F.p.every;
         for (long long r = 0; r < chunks; ++r) CK(cudaGraphLaunch(F.graph.exec, s));
     }

@@ -101,6 +101,7 @@ struct FlowState {
     float* d_vel = nullptr;          // its output field (borrowed)
     bool field_ready = false;        // d_vel holds the final field
     bool fresh = false;              // set up, and no loop or batch has had it yet
+    long long at = 0;                // the iteration its loop of launches begins at
     // Ends the flow phase of a solve that goes on to its transport.  Device
     // buffers of at most keep_bytes stay with the context for its next solve
     // (set-up sizes them with ensure() and initialises what it reads), so a

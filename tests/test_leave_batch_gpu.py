@@ -1,8 +1,9 @@
 """Solves that leave a batch part-way (prt_batch_remove) and go on by
-themselves (prt_flow_launch): the loop takes up the lattice and the count as
-the batch left them, so fields and counts are the single solve's bit for
-bit.  So they are when a finished loop, of its own or a batch's, is launched
-once more."""
+themselves (prt_flow_launch): the loop takes up the lattice, the count and
+the check schedule as the batch left them, so fields, counts and stop
+decisions are the single solve's bit for bit, also after an odd count and
+off the check interval.  So they are when a finished loop, of its own or a
+batch's, is launched once more."""
 
 import ctypes
 
@@ -11,10 +12,10 @@ import pytest
 
 pytestmark = pytest.mark.gpu
 
-# steps of a graph replay: off the check interval and on it
-LEFT = [20, 50]
+# steps of a graph replay: an odd count, one off the check interval, one on it
+LEFT = [7, 20, 50]
 SMALL, LARGE = 20, 34  # one cluster takes the first
-LOOPS = [("1", SMALL, "fp64"), ("1", SMALL, "fp16")]
+LOOPS = [("0", SMALL, "fp64"), ("1", SMALL, "fp64"), ("1", SMALL, "fp16"), ("1", LARGE, "fp32f")]
 
 
 def pack(edge, seed=4):
@@ -72,7 +73,7 @@ def same_flow(a, b):
     assert np.array_equal(a[0], b[0]), float(np.abs(a[0] - b[0]).max())
 
 
-@pytest.mark.parametrize("nit,tol", [(333, 0.0), (450, 0.0)])
+@pytest.mark.parametrize("nit,tol", [(333, 0.0), (450, 0.0), (2000, 2e-2)])
 @pytest.mark.parametrize("left", LEFT)
 @pytest.mark.parametrize("cluster,edge,precision", LOOPS)
 def test_flow_goes_on_after_a_batch(monkeypatch, cluster, edge, precision, left, nit, tol):
@@ -86,7 +87,7 @@ def test_flow_goes_on_after_a_batch(monkeypatch, cluster, edge, precision, left,
 
 def test_flow_of_a_plane_goes_on_after_a_batch():
     g = pack(40)[:, 5]
-    same_flow(flow(g, "fp64", 400, 0.0, 20), flow(g, "fp64", 400, 0.0))
+    same_flow(flow(g, "fp64", 400, 0.0, 7), flow(g, "fp64", 400, 0.0))
 
 
 @pytest.mark.parametrize("edge", [SMALL, LARGE])
@@ -98,3 +99,8 @@ def test_a_finished_flow_loop_launched_again_changes_nothing(edge):
 def test_a_loop_that_a_batch_finished_launched_again_changes_nothing():
     g = pack(SMALL)
     same_flow(flow(g, "fp64", 60, 0.0, 60), flow(g, "fp64", 60, 0.0))
+
+
+def test_a_flow_that_a_batch_leaves_just_below_its_cap():
+    g = pack(LARGE)
+    same_flow(flow(g, "fp64", 23, 0.0, 7), flow(g, "fp64", 23, 0.0))

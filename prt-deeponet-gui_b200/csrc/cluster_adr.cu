@@ -105,7 +105,7 @@ __global__ void __launch_bounds__(T, 1)
     const bool inlet = k < (unsigned)d.n0;
     const long long limit = ctrl->limit, pause = ctrl->n_pause;
     const int check = ctrl->check;
-    long long n = ctrl->n_base;
+    long long n = ctrl->n_base, next = (n / check + 1) * check;
     int go = !ctrl->done && n < pause;
     ClusterVoxel<ND> v;
     if (live) {
@@ -128,8 +128,11 @@ __global__ void __launch_bounds__(T, 1)
     }
     cluster_sync();
     while (go) {
-        const long long end = min(n + (long long)check, limit);
-        const bool due = end > n && end % check == 0;
+        // to the next check or the limit (a run that left a batch begins at any
+        // step)
+        const long long end = min(next, limit);
+        const bool due = end == next;
+        next += check;
         float cn[NS];
         for (++n; n <= end; ++n) {
             if (live) {
@@ -171,6 +174,7 @@ __global__ void __launch_bounds__(T, 1)
             if (t == 0) {
                 if (due) adr_check(ctrl, means, n, d.log, d.log_cap);
                 ctrl->n_base = n;
+                ctrl->n_stop = segment_end(n, ctrl->segment, check, limit);
                 if (n >= limit) ctrl->done = 1;
                 s_go = !ctrl->done && n < pause;
             }

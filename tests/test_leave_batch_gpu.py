@@ -1,14 +1,18 @@
 """Solves that leave a batch part-way (prt_batch_remove) and go on by
-themselves (prt_flow_launch): the loop takes up the lattice, the count and
-the check schedule as the batch left them, so fields, counts and stop
-decisions are the single solve's bit for bit, also after an odd count and
-off the check interval.  So they are when a finished loop, of its own or a
+themselves (prt_flow_launch, prt_adr_launch): the loop takes up the lattice or
+state, the count and the check schedule as the batch left them, so fields,
+counts and stop decisions are the single solve's bit for bit, also after an
+odd count and off the check interval.  So they are when a finished loop, of its own or a
 batch's, is launched once more."""
 
+import contextlib
 import ctypes
+import io
 
 import numpy as np
 import pytest
+
+from golden.fields import integer_velocity
 
 pytestmark = pytest.mark.gpu
 
@@ -104,3 +108,63 @@ def test_a_loop_that_a_batch_finished_launched_again_changes_nothing():
 def test_a_flow_that_a_batch_leaves_just_below_its_cap():
     g = pack(LARGE)
     same_flow(flow(g, "fp64", 23, 0.0, 7), flow(g, "fp64", 23, 0.0))
+
+
+def transport(g, v, steps, most, left=0, launches=1):
+    """(snapshots, times, steps, checks, last remainder) of a started run."""
+    from prtlb_gpu import _lib, adr, monod_chemistry
+    L = _lib.lib()
+    chem = monod_chemistry(0.5)
+    ctx = _lib.Context(0)
+    try:
+        mat8, vel32, geom = adr.stage_inputs(g, v, chem)
+        st = _lib.AdrStats()
+        ctx.check(L.prt_adr_stage(ctx.handle, mat8.ctypes.data_as(ctypes.c_void_p),
+                                  vel32.ctypes.data_as(ctypes.c_void_p), ctypes.byref(geom),
+                                  ctypes.byref(st)))
+        with contextlib.redirect_stdout(io.StringIO()):
+            S = adr.prepare(g.shape, adr.stats_dict(st), 8.0, 1.5, n_species=1, chem=chem, mat=g)
+        ctx.check(L.prt_adr_begin(ctx.handle, ctypes.byref(S.params)))
+        R = adr.run_params(S, steps, 2e-3, most, 1.12)
+        ctx.check(L.prt_adr_start(ctx.handle, ctypes.byref(R)))
+        if left:
+            assert left % S.check  # it leaves between two checks
+            in_batch(ctx, left)
+        for _ in range(launches):
+            ctx.check(L.prt_adr_launch(ctx.handle))
+            wait(ctx)
+        r = _lib.AdrResult()
+        ctx.check(L.prt_adr_finish(ctx.handle, ctypes.byref(r)))
+        ks = adr.ladder_steps(ctx)
+        picked = adr.pick(ks, int(r.steps), 4)
+        out, t = adr.outputs(ctx, S, 4, int(r.steps), ks, picked, steps, most, {}, 1.5, 0.0)
+        return out, t, r.steps, r.checks, r.last_rest
+    finally:
+        ctx.close()
+
+
+def same_transport(a, b):
+    assert a[2:] == b[2:]
+    assert np.array_equal(a[1], b[1])
+    assert np.array_equal(a[0], b[0]), float(np.abs(a[0] - b[0]).max())
+
+
+@pytest.mark.parametrize("steps,most", [(271, 0), (None, 6000)])
+@pytest.mark.parametrize("left", [7, 20])
+@pytest.mark.parametrize("edge", [SMALL, LARGE])
+def test_transport_goes_on_after_a_batch(monkeypatch, edge, left, steps, most):
+    g = pack(edge)
+    v = integer_velocity(g)
+    monkeypatch.setenv("PRT_CLUSTER", "0")
+    want = transport(g, v, steps, most)
+    assert want[3] > 0
+    same_transport(transport(g, v, steps, most, left), want)
+    monkeypatch.setenv("PRT_CLUSTER", "1")
+    same_transport(transport(g, v, steps, most, left), want)
+
+
+@pytest.mark.parametrize("edge", [SMALL, LARGE])
+def test_a_finished_transport_loop_launched_again_changes_nothing(edge):
+    g = pack(edge)
+    v = integer_velocity(g)
+    same_transport(transport(g, v, 271, 0, launches=2), transport(g, v, 271, 0))

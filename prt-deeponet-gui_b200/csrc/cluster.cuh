@@ -80,13 +80,15 @@ inline int cluster_span(long long n, int blocks) {
 }
 
 // Launches `kern` as one cluster, or returns cudaErrorNotSupported where the
-// device cannot place it.
+// device cannot place it.  smem_most: the most shared memory that any launch
+// of the kernel takes; the limit belongs to the kernel, not to the launch, so
+// every launch sets the same one and threads do not lower one another's.
 template <class K, class... A>
-inline cudaError_t launch_cluster(K kern, int blocks, int threads, size_t smem, cudaStream_t s,
-                                  A... args) {
+inline cudaError_t launch_cluster(K kern, int blocks, int threads, size_t smem, size_t smem_most,
+                                  cudaStream_t s, A... args) {
     cudaError_t e = cudaSuccess;
-    if (smem)
-        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem);
+    if (smem_most)
+        e = cudaFuncSetAttribute(kern, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)smem_most);
     if (e == cudaSuccess && blocks > 8)
         e = cudaFuncSetAttribute(kern, cudaFuncAttributeNonPortableClusterSizeAllowed, 1);
     cudaLaunchConfig_t cfg = {};

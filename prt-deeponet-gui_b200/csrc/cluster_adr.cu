@@ -189,7 +189,7 @@ template <int ND, int NS>
 cudaError_t run(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl, float* means, int blocks,
                 int span, cudaStream_t s) {
     auto kern = d.has_bf ? adr_cluster_kernel<ND, NS, true> : adr_cluster_kernel<ND, NS, false>;
-    return launch_cluster(kern, blocks, span, 0, s, d, p, ctrl, means, span);
+    return launch_cluster(kern, blocks, span, 0, 0, s, d, p, ctrl, means, span);
 }
 
 }  // namespace

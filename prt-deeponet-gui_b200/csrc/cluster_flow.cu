@@ -199,7 +199,7 @@ cudaError_t run(void* f, const FlowMap& fm, const Grid& g, const LbParams& k, Fl
     const int blocks = cluster_blocks(fm.nf), span = cluster_span(fm.nf, blocks);
     if (span > T) return cudaErrorNotSupported;
     const size_t smem = (size_t)L::Q * 2 * T * sizeof(typename M::S);
-    return launch_cluster(lb_cluster_kernel<L, M, T>, blocks, span, smem, s,
+    return launch_cluster(lb_cluster_kernel<L, M, T>, blocks, span, smem, smem, s,
                           static_cast<typename M::S*>(f), fm, g, k, ctrl, partials, span, nb);
 }
 

@@ -408,8 +408,9 @@ extern "C" int prt_walk_from_plane(prt_ctx* ctx, const uint8_t* mat, int32_t nd,
         bit_init_kernel<<<(used + kWalkThreads / 32 - 1) / (kWalkThreads / 32), kWalkThreads, 0,
                           s>>>(P.mat.as<uint8_t>(), w, b, pore_code, steps, seed, rest, counts);
         CK(cudaGetLastError());
-        const size_t smem = (size_t)b.rows * b.wpr * (3 * sizeof(unsigned) + sizeof(unsigned short));
-        const cudaError_t e = launch_cluster(bit_walk_kernel, kClusterMax, kBitThreads, smem, s, b,
+        constexpr size_t word = 3 * sizeof(unsigned) + sizeof(unsigned short);
+        const cudaError_t e = launch_cluster(bit_walk_kernel, kClusterMax, kBitThreads,
+                                             (size_t)b.rows * b.wpr * word, kBitWords * word, s, b,
                                              (const unsigned*)seed, (const unsigned*)rest, steps,
                                              counts);
         walked = e != cudaErrorNotSupported;

@@ -48,7 +48,8 @@ struct Transfer {
     void* pin[kWorkers] = {};
     cudaEvent_t ev[kWorkers] = {};
     int n = 0;
-    cudaError_t ensure(int workers, size_t chunk);
+    // Chunks to be had for `workers` threads, fewer or 0 where pinning fails.
+    int ensure(int workers, size_t chunk);
     void release();
 };
 

@@ -7,7 +7,8 @@
 // it over the bus and copies it between its pinned buffer and its own part
 // of the caller's memory.  Measured on a host with 16 cores: five 33 MB
 // snapshots into fresh memory 76 ms plainly (with one more host copy each),
-// a 85 MB field 17 ms.  Small copies and pinned memory take the plain path.
+// a 85 MB field 17 ms.  Small copies, pinned memory and a context that cannot
+// pin a chunk take the plain path.
 #include <atomic>
 #include <system_error>
 #include <thread>
@@ -58,13 +59,18 @@ void work(const prt_ctx* ctx, Transfer* t, int w, char* host, char* dev, size_t 
     if (e != cudaSuccess) error->store((int)e);
 }
 
-cudaError_t staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out) {
-    Transfer* t = &ctx->transfer;
+// Host threads for a copy of `bytes` from or to `host`: 0 where the plain path
+// is the one.
+int workers(prt_ctx* ctx, const void* host, size_t bytes) {
+    if (bytes < kStagedFrom || !pageable(host)) return 0;
     const unsigned cores = std::thread::hardware_concurrency();
     const int want = (int)std::min<size_t>({(size_t)Transfer::kWorkers, (size_t)std::max(1u, cores / 2),
                                             (bytes + kChunk - 1) / kChunk});
-    cudaError_t e = t->ensure(want, kChunk);
-    if (e != cudaSuccess) return e;
+    return ctx->transfer.ensure(want, kChunk);
+}
+
+cudaError_t staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out, int want) {
+    Transfer* t = &ctx->transfer;
     std::atomic<size_t> next{0};
     std::atomic<int> error{0};
     std::thread th[Transfer::kWorkers];
@@ -83,17 +89,16 @@ cudaError_t staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out) 
 
 }  // namespace
 
-cudaError_t Transfer::ensure(int workers, size_t chunk) {
+int Transfer::ensure(int workers, size_t chunk) {
     for (; n < workers; ++n) {
-        cudaError_t e = cudaHostAlloc(&pin[n], chunk, cudaHostAllocDefault);
-        if (e != cudaSuccess) return e;
-        e = cudaEventCreateWithFlags(&ev[n], cudaEventDisableTiming);
-        if (e != cudaSuccess) {
+        if (cudaHostAlloc(&pin[n], chunk, cudaHostAllocDefault) != cudaSuccess) break;
+        if (cudaEventCreateWithFlags(&ev[n], cudaEventDisableTiming) != cudaSuccess) {
             cudaFreeHost(pin[n]);
-            return e;
+            break;
         }
     }
-    return cudaSuccess;
+    if (n < workers) cudaGetLastError();  // the copy goes another way
+    return std::min(n, workers);
 }
 
 void Transfer::release() {
@@ -104,17 +109,17 @@ void Transfer::release() {
 }
 
 cudaError_t copy_out(prt_ctx* ctx, void* host, const void* dev, size_t bytes) {
-    if (bytes >= kStagedFrom && pageable(host))
+    if (const int w = workers(ctx, host, bytes))
         return staged(ctx, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)),
-                      bytes, true);
+                      bytes, true, w);
     cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 cudaError_t copy_in(prt_ctx* ctx, void* dev, const void* host, size_t bytes) {
-    if (bytes >= kStagedFrom && pageable(host))
+    if (const int w = workers(ctx, host, bytes))
         return staged(ctx, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev),
-                      bytes, false);
+                      bytes, false, w);
     return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream);
 }
 

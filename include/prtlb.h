@@ -304,11 +304,14 @@ int prt_flow_finish(prt_ctx* ctx, float* vel_out, prt_flow_info* info);
  * own flow solve (after prt_flow_finish). */
 int prt_adr_stage_flow(prt_ctx* ctx, const prt_adr_geom* geom, prt_adr_stats* stats);
 
-/* Ends the flow phase of ctx: its lattice, maps and tables are freed, those of
- * at most 32 MiB stay for the context's next solve (the material grid and the
- * field staged for transport are kept).  A context in a batch may call it once its
+/* Frees the lattice, maps and tables of ctx (keeps the material grid and the
+ * field staged for transport).  A context in a batch may call it once its
  * flow solve is finished (prt_flow_finish). */
 int prt_flow_release(prt_ctx* ctx);
+
+/* The same, but up to 32 MiB of them stay with the context for its next flow
+ * solve (so back-to-back small solves skip the allocator). */
+int prt_flow_end(prt_ctx* ctx);
 
 /* Sets up the transport run of prt_adr_run (after prt_adr_begin) without
  * running its loop; no progress callback. */

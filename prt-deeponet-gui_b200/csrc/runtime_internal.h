@@ -9,6 +9,7 @@
 #include <cstdio>
 #include <cstdlib>
 #include <cstring>
+#include <iterator>
 #include <string>
 #include <vector>
 
@@ -103,18 +104,21 @@ struct FlowState {
     bool field_ready = false;        // d_vel holds the final field
     bool fresh = false;              // set up, and no loop or batch has had it yet
     long long at = 0;                // the iteration its loop of launches begins at
-    // Ends the flow phase of a solve that goes on to its transport.  Device
-    // buffers of at most keep_bytes stay with the context for its next solve
-    // (set-up sizes them with ensure() and initialises what it reads), so a
-    // batch of small solves does not pay cudaFree / cudaMalloc for each.
+    // Ends the flow phase of a solve.  The smallest of its device buffers stay
+    // with the context, keep_bytes of them together at most, for its next solve
+    // (set-up sizes them with ensure() and initialises what it reads).
     void release_lattices(size_t keep_bytes) {
         DevBuf* all[] = {&f, &fluid, &partials, &count, &flag, &cnt, &cells, &nbr, &link, &pack};
+        std::sort(std::begin(all), std::end(all),
+                  [](const DevBuf* a, const DevBuf* b) { return a->bytes < b->bytes; });
         bool freed = false;
-        for (DevBuf* b : all)
-            if (b->bytes > keep_bytes) {
-                b->release();
-                freed = true;
-            }
+        size_t kept = 0;
+        for (DevBuf* b : all) {
+            kept += b->bytes;
+            if (kept <= keep_bytes) continue;
+            freed = freed || b->p != nullptr;
+            b->release();
+        }
         if (freed) {  // the cached loop graph holds device pointers
             graph.release();
             key = FlowKey();

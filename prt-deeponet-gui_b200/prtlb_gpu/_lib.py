@@ -151,6 +151,7 @@ _PROTOS = {
     "prt_adr_stage_flow": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(AdrGeom),
                                           ctypes.POINTER(AdrStats)]),
     "prt_flow_release": (ctypes.c_int, [ctypes.c_void_p]),
+    "prt_flow_end": (ctypes.c_int, [ctypes.c_void_p]),
     "prt_adr_start": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(AdrRunParams)]),
     "prt_adr_finish": (ctypes.c_int, [ctypes.c_void_p, ctypes.POINTER(AdrResult)]),
     "prt_flow_launch": (ctypes.c_int, [ctypes.c_void_p]),

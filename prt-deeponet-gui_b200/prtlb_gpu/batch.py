@@ -38,8 +38,9 @@ ADR_DEFAULTS = dict(n_species=2, steps=None, tol=2e-3, max_steps=100000, ratio=1
 # Idle contexts kept for the next solves on a device (at most _POOL_CAP):
 # a solve that takes one reuses its device buffers instead of allocating
 # them, and a finished solve's context costs no cudaFree.  What a kept
-# context holds: the material grid and velocity field of its last solve and
-# the transport buffers up to the keep size of prt_adr_end (256 MiB each).
+# context holds: the material grid and velocity field of its last solve, the
+# transport buffers up to the keep size of prt_adr_end (256 MiB each) and
+# what prt_flow_end keeps of the flow phase (32 MiB together).
 _POOL_CAP = 64
 _pool = {}
 _pool_lock = threading.Lock()
@@ -299,7 +300,7 @@ class Batch(object):
         L = _lib.lib()
         for ctx in self._unlattice:
             if ctx.handle:
-                ctx.check(L.prt_flow_release(ctx.handle))
+                ctx.check(L.prt_flow_end(ctx.handle))
         self._unlattice = []
         for ctx in self._graveyard:
             _return_context(ctx, self.device)
@@ -377,8 +378,8 @@ class Batch(object):
                              mat=req.mat)
         job.S = S
         ctx.check(L.prt_adr_begin(ctx.handle, ctypes.byref(S.params)))
-        # the lattices are freed once the device is idle (a free now would
-        # wait for the launch in flight)
+        # the flow phase ends once the device is idle (a free now would wait
+        # for the launch in flight)
         self._unlattice.append(ctx)
         R = _adr.run_params(S, a["steps"], a["tol"], a["max_steps"], a["ratio"])
         ctx.check(L.prt_adr_start(ctx.handle, ctypes.byref(R)))

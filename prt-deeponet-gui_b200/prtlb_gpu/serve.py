@@ -33,8 +33,8 @@ def ladder_slots(limit, ratio):
     return k + 2
 
 
-# what prt_flow_release keeps of a flow phase at most: ten buffers of 32 MiB
-_FLOW_KEEP = 10 * (32 << 20)
+# what prt_flow_end keeps of a flow phase at most
+_FLOW_KEEP = 32 << 20
 
 
 def footprint(req):

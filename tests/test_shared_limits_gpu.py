@@ -1,5 +1,6 @@
-"""What calls of one process share: a limit that belongs to a kernel."""
+"""What calls of one process share, and what a context gives back."""
 
+import ctypes
 import threading
 
 import numpy as np
@@ -37,3 +38,38 @@ def test_walks_of_two_sizes_side_by_side():
     for t in threads:
         t.join()
     assert not bad, bad
+
+
+def test_flow_release_gives_the_memory_back():
+    """prt_flow_release frees the lattice, maps and tables whatever their size
+    (here under 32 MiB each); a context whose flow phase was ended with
+    prt_flow_end solves on with the buffers it kept."""
+    from prtlb_gpu import _lib, random_pack
+    from prtlb_gpu.flow import flow_params
+    from prtlb_gpu.serve import device_memory
+    L = _lib.lib()
+    g, p = flow_params(random_pack((60, 60, 60), 0.5, 3.0, 5.0, seed=1), 3, "flow", 100, 2e-6, 0.8,
+                       3.0 / 16.0, 0.0, "fp32")
+    ctx = _lib.Context(0)
+
+    def solve():
+        vel = np.empty((3,) + g.shape, np.float32)
+        ctx.check(L.prt_flow(ctx.handle, g.ctypes.data_as(ctypes.c_void_p), ctypes.byref(p),
+                             vel.ctypes.data_as(ctypes.c_void_p), None))
+        return vel
+
+    try:
+        solve()
+        ctx.check(L.prt_flow_release(ctx.handle))
+        before = device_memory(0)[0]
+        want = solve()
+        assert device_memory(0)[0] <= before - (8 << 20)  # the lattice alone: 8.2 MB
+        ctx.check(L.prt_flow_release(ctx.handle))
+        assert device_memory(0)[0] == before
+        assert np.array_equal(solve(), want)
+        ctx.check(L.prt_flow_end(ctx.handle))
+        held = before - device_memory(0)[0]
+        assert 0 < held <= (40 << 20)  # at most 32 MiB, and the allocator's rounding
+        assert np.array_equal(solve(), want)
+    finally:
+        ctx.close()

@@ -46,6 +46,7 @@ extern "C" int prt_create(int device, prt_ctx** out) {
         delete c;
         return PRT_E_CUDA;
     }
+    transfer_open(device);
     *out = c;
     return PRT_OK;
 }
@@ -57,7 +58,7 @@ extern "C" void prt_destroy(prt_ctx* c) {
     cudaStreamSynchronize(c->stream);
     c->adr.release();
     c->prep.release();
-    c->transfer.release();
+    transfer_close(c->device);
     FlowState& f = c->flow;
     DevBuf* all[] = {&f.f,    &f.fluid, &f.partials, &f.ctrl, &f.out5, &f.count,
                      &f.mat,  &f.vel,   &f.flag,     &f.cnt,  &f.cells, &f.nbr, &f.link, &f.pack};

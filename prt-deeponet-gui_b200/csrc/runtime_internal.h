@@ -42,8 +42,8 @@ struct DevBuf {
     T* as() const { return static_cast<T*>(p); }
 };
 
-// Pinned chunks of a context for copies from and to pageable memory
-// (transfer.cu), one per copying thread; made at the first large copy.
+// Pinned chunks for copies from and to pageable memory (transfer.cu), one per
+// copying thread.
 struct Transfer {
     static constexpr int kWorkers = 8;
     void* pin[kWorkers] = {};
@@ -206,7 +206,6 @@ struct prt_ctx {
     prt::FlowState flow;
     prt::AdrState adr;
     prt::PrepState prep;
-    prt::Transfer transfer;
     bool flow_armed = false;  // flow set up, its time loop not finished
     bool adr_armed = false;   // transport run set up, its time loop not finished
     prt_batch* batch = nullptr;  // the batch holding this context, if any
@@ -320,6 +319,10 @@ int adr_loop_async(prt_ctx* ctx);
 // Copies on the context's stream between device memory and the caller's
 // (transfer.cu).  copy_out returns with the data in place; after copy_in the
 // caller's memory has been read.
+// A device's contexts share its pinned chunks: transfer_open and transfer_close
+// count them, and the last one's end gives the chunks back.
+void transfer_open(int device);
+void transfer_close(int device);
 cudaError_t copy_out(prt_ctx* ctx, void* host, const void* dev, size_t bytes);
 cudaError_t copy_in(prt_ctx* ctx, void* dev, const void* host, size_t bytes);
 // Takes ctx out of its batch (engine.cu); used by prt_destroy.

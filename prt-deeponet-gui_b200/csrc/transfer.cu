@@ -2,14 +2,15 @@
 //
 // A plain copy from or to pageable memory is staged by the driver on one
 // host thread; taking a result into fresh memory also faults its pages in
-// one by one.  Large copies therefore go through pinned chunks of the
-// context with several host threads: each thread takes the next chunk, moves
+// one by one.  Large copies therefore go through pinned chunks with several
+// host threads: each thread takes the next chunk, moves
 // it over the bus and copies it between its pinned buffer and its own part
 // of the caller's memory.  Measured on a host with 16 cores: five 33 MB
 // snapshots into fresh memory 76 ms plainly (with one more host copy each),
-// a 85 MB field 17 ms.  Small copies, pinned memory and a context that cannot
-// pin a chunk take the plain path.
+// a 85 MB field 17 ms.  Small copies and pinned memory take the plain path, and
+// so does a copy that gets no chunk: none can be pinned, or all are in use.
 #include <atomic>
+#include <mutex>
 #include <system_error>
 #include <thread>
 
@@ -23,6 +24,39 @@ namespace {
 // a copy is worth the threads (they cost about 0.2 ms together).
 constexpr size_t kChunk = size_t(1) << 20;
 constexpr size_t kStagedFrom = size_t(4) << 20;
+// Copies of a device that run on chunks at a time: 32 MiB of pinned memory, and
+// 32 host threads.
+constexpr int kSets = 4;
+
+// The sets of chunks of a device; a copy has one to itself while it runs.  A
+// set given back may still be the source of a copy in flight on its last
+// user's stream; its chunks' events say when (work).
+struct DeviceSets {
+    Transfer set[kSets];
+    bool lent[kSets] = {};
+    int contexts = 0;
+};
+std::mutex sets_mu;
+constexpr int kDevices = 64;  // a device beyond has none
+DeviceSets sets_of[kDevices];
+
+Transfer* take_set(int device) {
+    if (device >= kDevices) return nullptr;
+    std::lock_guard<std::mutex> lk(sets_mu);
+    DeviceSets& d = sets_of[device];
+    for (int i = 0; i < kSets; ++i)
+        if (!d.lent[i]) {
+            d.lent[i] = true;
+            return &d.set[i];
+        }
+    return nullptr;
+}
+
+void give_set(int device, Transfer* t) {
+    std::lock_guard<std::mutex> lk(sets_mu);
+    DeviceSets& d = sets_of[device];
+    d.lent[t - d.set] = false;
+}
 
 bool pageable(const void* p) {
     cudaPointerAttributes a;
@@ -59,18 +93,16 @@ void work(const prt_ctx* ctx, Transfer* t, int w, char* host, char* dev, size_t 
     if (e != cudaSuccess) error->store((int)e);
 }
 
-// Host threads for a copy of `bytes` from or to `host`: 0 where the plain path
-// is the one.
-int workers(prt_ctx* ctx, const void* host, size_t bytes) {
-    if (bytes < kStagedFrom || !pageable(host)) return 0;
+// Whether the copy ran on pinned chunks, with its error in *e.
+bool staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out, cudaError_t* e) {
+    if (bytes < kStagedFrom || !pageable(host)) return false;
+    Transfer* t = take_set(ctx->device);
+    if (!t) return false;
     const unsigned cores = std::thread::hardware_concurrency();
-    const int want = (int)std::min<size_t>({(size_t)Transfer::kWorkers, (size_t)std::max(1u, cores / 2),
-                                            (bytes + kChunk - 1) / kChunk});
-    return ctx->transfer.ensure(want, kChunk);
-}
-
-cudaError_t staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out, int want) {
-    Transfer* t = &ctx->transfer;
+    const int want = t->ensure(
+        (int)std::min<size_t>({(size_t)Transfer::kWorkers, (size_t)std::max(1u, cores / 2),
+                               (bytes + kChunk - 1) / kChunk}),
+        kChunk);
     std::atomic<size_t> next{0};
     std::atomic<int> error{0};
     std::thread th[Transfer::kWorkers];
@@ -81,10 +113,12 @@ cudaError_t staged(prt_ctx* ctx, char* host, char* dev, size_t bytes, bool out, 
             break;  // no thread to be had: the others take its chunks
         }
     }
-    work(ctx, t, 0, host, dev, bytes, out, &next, &error);
+    if (want) work(ctx, t, 0, host, dev, bytes, out, &next, &error);
     for (int w = 1; w < want; ++w)
         if (th[w].joinable()) th[w].join();
-    return (cudaError_t)error.load();
+    give_set(ctx->device, t);
+    *e = (cudaError_t)error.load();
+    return want > 0;
 }
 
 }  // namespace
@@ -108,18 +142,34 @@ void Transfer::release() {
     }
 }
 
+void transfer_open(int device) {
+    if (device >= kDevices) return;
+    std::lock_guard<std::mutex> lk(sets_mu);
+    sets_of[device].contexts += 1;
+}
+
+void transfer_close(int device) {
+    if (device >= kDevices) return;
+    std::lock_guard<std::mutex> lk(sets_mu);
+    DeviceSets& d = sets_of[device];
+    if (--d.contexts > 0) return;
+    for (Transfer& t : d.set) t.release();
+}
+
 cudaError_t copy_out(prt_ctx* ctx, void* host, const void* dev, size_t bytes) {
-    if (const int w = workers(ctx, host, bytes))
-        return staged(ctx, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)),
-                      bytes, true, w);
-    cudaError_t e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
+    cudaError_t e = cudaSuccess;
+    if (staged(ctx, static_cast<char*>(host), const_cast<char*>(static_cast<const char*>(dev)), bytes,
+               true, &e))
+        return e;
+    e = cudaMemcpyAsync(host, dev, bytes, cudaMemcpyDeviceToHost, ctx->stream);
     return e == cudaSuccess ? cudaStreamSynchronize(ctx->stream) : e;
 }
 
 cudaError_t copy_in(prt_ctx* ctx, void* dev, const void* host, size_t bytes) {
-    if (const int w = workers(ctx, host, bytes))
-        return staged(ctx, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev),
-                      bytes, false, w);
+    cudaError_t e = cudaSuccess;
+    if (staged(ctx, const_cast<char*>(static_cast<const char*>(host)), static_cast<char*>(dev), bytes,
+               false, &e))
+        return e;
     return cudaMemcpyAsync(dev, host, bytes, cudaMemcpyHostToDevice, ctx->stream);
 }
 

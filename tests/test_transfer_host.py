@@ -1,5 +1,7 @@
 """Copies from and to pageable memory (transfer.cu) on the CPU, with fakes of
-the CUDA calls: the bytes arrive whatever pinned memory can be had."""
+the CUDA calls: the bytes arrive whatever pinned memory can be had, and the
+contexts of a device share a bounded number of chunks, which the last of them
+gives back."""
 
 import os
 import shutil
@@ -14,7 +16,9 @@ PROGRAM = r"""
 #include <cstdio>
 #include <cstring>
 #include <vector>
-static int pins_left, pinned, plain;
+#include <atomic>
+#include <thread>
+static std::atomic<int> pins_left, pinned, plain;
 static cudaError_t fake_pin(void** p, size_t n, unsigned) {
     if (pins_left <= 0) return cudaErrorMemoryAllocation;
     --pins_left; ++pinned; *p = ::operator new(n);
@@ -46,12 +50,29 @@ static cudaError_t ok() { return cudaSuccess; }
 
 static bool both_ways(size_t n) {
     prt_ctx ctx;
+    prt::transfer_open(0);
     std::vector<char> a(n), b(n), c(n);
     for (size_t i = 0; i < n; ++i) a[i] = (char)(i * 2654435761u >> 13);
     const bool good = prt::copy_in(&ctx, b.data(), a.data(), n) == cudaSuccess &&
                       prt::copy_out(&ctx, c.data(), b.data(), n) == cudaSuccess && c == a;
-    ctx.transfer.release();
-    return good && pinned == 0;
+    prt::transfer_close(0);
+    return good;
+}
+
+// Copies of `threads` contexts at a time: the most chunks that were pinned.
+static int together(int threads) {
+    pins_left = 1000;
+    std::atomic<int> bad{0};
+    std::vector<std::thread> th;
+    prt::transfer_open(0);
+    for (int i = 0; i < threads; ++i)
+        th.emplace_back([&] {
+            for (int r = 0; r < 5; ++r) bad += !both_ways((size_t(6) << 20) + 11 * r);
+        });
+    for (auto& t : th) t.join();
+    const int most = pinned;  // chunks stay while a context is open
+    prt::transfer_close(0);
+    return bad || pinned ? -1 : most;
 }
 
 int main() {
@@ -59,11 +80,15 @@ int main() {
     for (int left : {100, 1, 0}) {  // every chunk, one chunk and none can be pinned
         pins_left = left;
         plain = 0;
-        if (!both_ways(big) || plain != (left ? 0 : 2)) { printf("pins %d\n", left); return 1; }
+        if (!both_ways(big) || pinned != 0 || plain != (left ? 0 : 2)) { printf("pins %d\n", left); return 1; }
     }
     pins_left = 100;
     plain = 0;
     if (!both_ways((size_t(4) << 20) - 1) || plain != 2 || pins_left != 100) return 2;  // a small copy
+    for (int threads : {1, 12}) {
+        const int most = together(threads);
+        if (most < 1 || most > (threads == 1 ? 8 : 32)) { printf("%d: %d\n", threads, most); return 3; }
+    }
     return 0;
 }
 """

@@ -237,7 +237,7 @@ int rebuild(prt_batch* b) {
     }
     // plain tables of far places: each solve chose them against the whole L2;
     // in a batch a class reads them while all its jobs have one and all the
-    // flow jobs' lattices and tables together fit in three quarters of it, else
+    // flow jobs' lattices and tables together are let in by batch_use_nbr, else
     // the packed ones (the same places, so the fields do not change)
     {
         long long ws = 0, l2 = 0;
@@ -251,7 +251,7 @@ int rebuild(prt_batch* b) {
             l2 = ctx->l2_bytes;
             if (!F.fm.nbr && F.fm.nf > 0) b->flow_table[flow_class(F.p.nd, F.p.precision)] = false;
         }
-        if (ws > l2 / 4 * 3)
+        if (!batch_use_nbr(ws, l2))
             for (int c = 0; c < kFlowClasses; ++c) b->flow_table[c] = false;
     }
     const int njobs = (int)b->order.size();

@@ -275,6 +275,14 @@ inline bool flow_use_nbr(int q, long long nf, long long rs, long long es, long l
     return nf > 0 && q * rs * es + flow_nbr_bytes(q, nf) <= l2_bytes / 4 * 3;
 }
 
+// The same for a batch whose flow lattices and plain tables take ws bytes
+// together.  PRT_NBR_TABLE=1, which gives every solve its plain table, holds
+// for batches too.
+inline bool batch_use_nbr(long long ws, long long l2_bytes) {
+    const char* v = std::getenv("PRT_NBR_TABLE");
+    return (v && v[0] == '1') || ws <= l2_bytes / 4 * 3;
+}
+
 // Constants of one flow solve (the TRT rates of _trt_minus and the Guo
 // force terms), shared by every entry point that runs a flow solve.
 inline void fill_lbconst(LbParams& k, int nd, double force, double tau, double magic, float scale) {

@@ -87,20 +87,21 @@ __device__ __forceinline__ const float* apart(const float* p, int n) {
     return q;
 }
 
-// A load through the read-only path (the buffer is not written by this
-// launch), issued where it stands; and the same only where u >= 0, or only
-// where it is not, else 0: the far value that the upwind side does not need
-// is not read.
+// A load of the state, issued where it stands; and the same only where u >= 0,
+// or only where it is not, else 0: the far value that the upwind side does not
+// need is not read.  Not through the read-only path (.nc): with programmatic
+// launch a step's blocks are resident while the step before writes what they
+// will read.
 __device__ __forceinline__ float ld_early(const float* p) {
     float v;
-    asm volatile("ld.global.nc.f32 %0, [%1];" : "=f"(v) : "l"(p));
+    asm volatile("ld.global.f32 %0, [%1];" : "=f"(v) : "l"(p));
     return v;
 }
 __device__ __forceinline__ float ld_if_up(const float* p, float u) {
     float v;
     asm volatile(
         "{\n.reg .pred q;\nsetp.ge.f32 q, %2, 0f00000000;\nmov.f32 %0, 0f00000000;\n"
-        "@q ld.global.nc.f32 %0, [%1];\n}"
+        "@q ld.global.f32 %0, [%1];\n}"
         : "=&f"(v)
         : "l"(p), "f"(u));
     return v;
@@ -109,7 +110,7 @@ __device__ __forceinline__ float ld_if_down(const float* p, float u) {
     float v;
     asm volatile(
         "{\n.reg .pred q;\nsetp.ltu.f32 q, %2, 0f00000000;\nmov.f32 %0, 0f00000000;\n"
-        "@q ld.global.nc.f32 %0, [%1];\n}"
+        "@q ld.global.f32 %0, [%1];\n}"
         : "=&f"(v)
         : "l"(p), "f"(u));
     return v;

@@ -362,7 +362,10 @@ static long long resident_blocks(K kern) {
 // it (24^3: 2.35 -> 2.02, 40^3 2.43 -> 2.11, 128^2 first order 2.36 -> 2.05);
 // between the two only after its stores (pdl_late), or the next step's blocks
 // would slow the running one (64^3, four chemicals: 4.85 against 5.55).
-// PRT_PDL=0 launches every step plainly.
+// PRT_PDL=0 launches every step plainly.  The first step after a chunk's end
+// always goes out plainly (in a loop's graph it is the first node and so does
+// anyway): the control block is then in place before any step of the chunk is
+// resident, and the steps may take it as read-only.
 template <int ND, int NS>
 static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctrl, int k,
                           cudaStream_t s) {
@@ -382,7 +385,7 @@ static cudaError_t step_t(const AdrDev& d, const prt_adr_params& p, AdrCtrl* ctr
     cfg.attrs = attr;
     const long long resident = resident_blocks(kern);
     const int late = pdl_late(nb <= resident && 2 * nb > resident) ? 1 : 0;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl_enabled() && k > 0 ? 1 : 0;
     return cudaLaunchKernelEx(&cfg, kern, d, p, ctrl, k, late, 2 * nb > resident ? 1 : 0);
 }
 

@@ -331,7 +331,10 @@ int flow_blocks(long long n) { return (int)((n + kFlowThreads - 1) / kFlowThread
 // change during a solve) and waits in griddepcontrol.wait for t's results
 // (launched plainly 64^3 float32 takes 4.52 us an iteration, 54^3 float64
 // 4.20, against 4.03 and 3.92).  A grid of one resident wave releases the next
-// step only after its stores (pdl_late).
+// step only after its stores (pdl_late).  The first step after a check goes out
+// plainly (in a loop's graph it is the first node and so does anyway): the
+// check's control block is then in place before any step of the chunk is
+// resident, and the steps may take it as read-only.
 
 // Blocks of `kern` the device holds at once.
 template <class K>
@@ -361,7 +364,7 @@ static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Gr
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
-    cfg.numAttrs = pdl_enabled() ? 1 : 0;
+    cfg.numAttrs = pdl_enabled() && kstep > 0 ? 1 : 0;
     // D3Q19 float64 stages its gather in shared memory, because in registers it
     // takes 118 of them; a solve whose blocks all fit at four an SM has the
     // registers (54^3: 4.16 -> 3.94 us an iteration, 44^3 3.23 -> 3.07; beyond

@@ -63,6 +63,24 @@ def test_transport_steps_under_every_release(monkeypatch, pdl, late):
         assert np.array_equal(out, z["out"]), (name, float(np.abs(out - z["out"]).max()))
 
 
+@pytest.mark.parametrize("pdl,late", RELEASES)
+def test_direct_launches_under_every_release(monkeypatch, pdl, late):
+    """Without a graph a chunk's first step follows the check kernel in the
+    stream; the steps read the control block that it leaves."""
+    from prtlb_gpu import sphere_pack_3d
+    g = sphere_pack_3d(24, 0.45, 0)
+    want = flow(g, "fp64", nit=333, tol=1e-3)
+    monkeypatch.setenv("PRT_GRAPHS", "0")
+    monkeypatch.setenv("PRT_PDL", pdl)
+    monkeypatch.setenv("PRT_PDL_LATE", late)
+    same(flow(g, "fp64", nit=333, tol=1e-3), want)
+    for name in ADR[2:4]:
+        z = load_golden(name)
+        out, tn, info, prog = run(z, name)
+        assert np.array_equal(prog, z["progress"]), name
+        assert np.array_equal(out, z["out"]), (name, float(np.abs(out - z["out"]).max()))
+
+
 def test_transport_graph_follows_every_change(monkeypatch):
     from prtlb_gpu import _lib, solve_adr
     ctx = _lib.Context(0)

@@ -26,8 +26,12 @@ __device__ __forceinline__ unsigned cluster_rank() {
 }
 
 // Every thread of every block of the cluster; writes before it are visible
-// after it.
+// after it.  The .aligned forms ask that a warp's threads arrive together, and
+// the loops come here from branches that part a warp (the last live slot,
+// thread 0), so the warp is brought together first; that costs nothing, the
+// forms without .aligned 1-5 % of a step.
 __device__ __forceinline__ void cluster_sync() {
+    __syncwarp();
     asm volatile(
         "barrier.cluster.arrive.release.aligned;\nbarrier.cluster.wait.acquire.aligned;" ::
             : "memory");

@@ -22,3 +22,14 @@ def test_no_read_only_load_by_hand():
     assert SOURCES
     for path in SOURCES:
         assert ".nc." not in code(path), path
+
+
+def test_aligned_cluster_barriers_follow_a_warp_barrier():
+    """The .aligned forms need a converged warp, which code behind a divergent
+    branch does not promise."""
+    found = 0
+    for path in SOURCES:
+        for before in re.split(r"asm volatile\(\s*\"barrier\.cluster\.\S+\.aligned", code(path))[:-1]:
+            assert before.rstrip().endswith("__syncwarp();"), path
+            found += 1
+    assert found

@@ -106,7 +106,8 @@ enum class Fresh { none, index, base };
 // Precision modes: storage type S, arithmetic R for the symmetric part and
 // RA for the momentum and the antisymmetric non-equilibrium part (a small
 // difference of two O(u) numbers), and the resident blocks of kFlowThreads
-// per SM the register budget is cut for (single-solve and batched steps).
+// per SM the register budget is cut for (single-solve and batched steps;
+// narrow: D2Q9 single solves that save a wave by it, 0 where none does).
 // `fresh`: see Fresh; `regrouped`: see collide_regrouped.
 // `staged`: D3Q19's arrived populations go to shared memory by cp.async, so no
 // register waits on a gather load.  Only float64 gains by it (80^3 9.8 against
@@ -119,6 +120,7 @@ struct ModeF64 {  // the reference's arithmetic
     using R = double;
     using RA = double;
     static constexpr int min_blocks = 7;
+    static constexpr int narrow_blocks = 9;
     static constexpr Fresh fresh = Fresh::base;
     static constexpr bool regrouped = true;
     static constexpr int batch_min_blocks = 6;
@@ -130,6 +132,7 @@ struct ModeF32 {  // float32 populations, float32 collision
     using RA = float;
     // 64 registers (8 blocks per SM)
     static constexpr int min_blocks = 8;
+    static constexpr int narrow_blocks = 10;
     static constexpr Fresh fresh = Fresh::index;
     static constexpr bool regrouped = true;
     static constexpr int batch_min_blocks = 8;
@@ -143,6 +146,7 @@ struct ModeF32D {  // float32 populations, float64 momentum
     // (917 blocks) still fits one wave at 8 blocks per SM (5.67 -> 5.41 us
     // per iteration; 128^3 unchanged)
     static constexpr int min_blocks = 8;
+    static constexpr int narrow_blocks = 0;
     static constexpr Fresh fresh = Fresh::index;
     static constexpr bool regrouped = false;
     static constexpr int batch_min_blocks = 8;
@@ -153,6 +157,7 @@ struct ModeF16 {  // scaled float16 populations, float32 collision
     using R = float;
     using RA = float;
     static constexpr int min_blocks = 6;
+    static constexpr int narrow_blocks = 10;
     static constexpr Fresh fresh = Fresh::index;
     static constexpr bool regrouped = false;
     static constexpr int batch_min_blocks = 6;

@@ -26,6 +26,7 @@
 // Populations are stored shifted, h_i = f_i - w_i: the non-equilibrium part
 // that carries the viscous stress is of the order of the force (1e-7) and
 // would drown next to w_i ~ 0.3 in float32 (prtlb_2d.py:354-362).
+#include <algorithm>
 #include <cstdlib>
 
 #include "lb_core.cuh"
@@ -45,16 +46,29 @@ namespace prt {
 // 96^3 float64 27.1 -> 16.2, float32 11.8 -> 10.7, 64^3 unchanged within 5 %.
 // A grid of one wave whose threads overlap the next voxel's loads with this
 // one's collision (two cp.async stages) was slower beyond the L2 (192^3 122).
-// REG: the form of a D3Q19 float64 step that gathers into registers, four
-// blocks an SM (see launch_step_one).
-template <class L, class M, Far F, bool ODD, bool CHECK, bool REG>
-__global__ void __launch_bounds__(kFlowThreads, REG ? 4 : M::min_blocks)
+enum class Form {
+    wide,    // the mode's own
+    four,    // D3Q19 float64 gathered into registers, four blocks an SM
+    halves,  // the same with blocks of half the size, ten an SM (unsampled steps)
+    narrow   // D2Q9 with fewer registers and more blocks an SM (see launch_step_one)
+};
+template <Form W>
+__host__ __device__ constexpr int form_threads() {
+    return W == Form::halves ? kFlowThreads / 2 : kFlowThreads;
+}
+template <class M, Form W>
+__host__ __device__ constexpr int form_blocks() {
+    return W == Form::four ? 4 : W == Form::halves ? 10 : W == Form::narrow ? M::narrow_blocks : M::min_blocks;
+}
+
+template <class L, class M, Far F, bool ODD, bool CHECK, Form W>
+__global__ void __launch_bounds__(form_threads<W>(), form_blocks<M, W>())
     lb_step_kernel(typename M::S* __restrict__ f, FlowMap fm, Grid g, LbParams kc,
                    const FlowCtrl* __restrict__ ctrl, int kstep, double* __restrict__ partials,
                    int late, int turn) {
     if (!late) griddep_launch_dependents();
     const int b = ODD && turn ? gridDim.x - 1 - blockIdx.x : blockIdx.x;
-    const int k = b * kFlowThreads + threadIdx.x;
+    const int k = b * form_threads<W>() + threadIdx.x;
     const Lat<typename M::S> lat = lattice<L>(f, fm.rs, ODD);
     // the pore maps never change during a solve: the far places are looked
     // up while the previous iteration may still be running
@@ -65,7 +79,9 @@ __global__ void __launch_bounds__(kFlowThreads, REG ? 4 : M::min_blocks)
     if (ctrl->done || it >= ctrl->nit) return;  // uniform over the grid
     double acc = 0.0;
     if (k < fm.nf) {
-        const double ux = lb_cell<L, M, M::staged && L::Q == 19 && !REG, REG>(lat, kc, k, far);
+        constexpr bool reg = W == Form::four || W == Form::halves;
+        constexpr bool index = reg || (W == Form::narrow && sizeof(typename M::S) == 8);
+        const double ux = lb_cell<L, M, M::staged && L::Q == 19 && !reg, index>(lat, kc, k, far);
         if (CHECK) acc = ux;
     }
     if (CHECK) block_sum_store(acc, partials + b);
@@ -338,9 +354,9 @@ int flow_blocks(long long n) { return (int)((n + kFlowThreads - 1) / kFlowThread
 
 // Blocks of `kern` the device holds at once.
 template <class K>
-static long long resident_blocks(K kern) {
+static long long resident_blocks(K kern, int threads) {
     int per_sm = 0, dev = 0, sms = 0;
-    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, kFlowThreads, 0) !=
+    if (cudaOccupancyMaxActiveBlocksPerMultiprocessor(&per_sm, kern, threads, 0) !=
             cudaSuccess ||
         cudaGetDevice(&dev) != cudaSuccess ||
         cudaDeviceGetAttribute(&sms, cudaDevAttrMultiProcessorCount, dev) != cudaSuccess) {
@@ -350,39 +366,80 @@ static long long resident_blocks(K kern) {
     return (long long)per_sm * sms;
 }
 
-template <class L, class M, bool ODD, bool CHECK>
-static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Grid& g,
-                                   const LbParams& k, const FlowCtrl* ctrl, int kstep,
-                                   double* partials, cudaStream_t s) {
-    const int nb = flow_blocks(fm.nf);
+// Launches the step in form W and returns true if its blocks are resident at
+// once (or ALWAYS), with the launch's error in *e.
+template <class L, class M, bool ODD, bool CHECK, Form W, bool ALWAYS>
+static bool launch_form(typename M::S* f, const FlowMap& fm, const Grid& g, const LbParams& k,
+                        const FlowCtrl* ctrl, int kstep, double* partials, cudaStream_t s,
+                        cudaError_t* e) {
+    constexpr int threads = form_threads<W>();
+    // both places' kernels are held to the same register budget
+    static const long long resident =
+        resident_blocks(lb_step_kernel<L, M, Far::table, ODD, CHECK, W>, threads);
+    const long long nb = ((long long)fm.nf + threads - 1) / threads;
+    const bool one_wave = nb <= resident;
+    if (!ALWAYS && !one_wave) return false;
     cudaLaunchConfig_t cfg = {};
-    cfg.gridDim = dim3(nb);
-    cfg.blockDim = dim3(kFlowThreads);
-    cfg.dynamicSmemBytes = 0;
+    cfg.gridDim = dim3((unsigned)nb);
+    cfg.blockDim = dim3(threads);
     cfg.stream = s;
     cudaLaunchAttribute attr[1];
     attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
     attr[0].val.programmaticStreamSerializationAllowed = 1;
     cfg.attrs = attr;
     cfg.numAttrs = pdl_enabled() && kstep > 0 ? 1 : 0;
+    auto kern = lb_step_kernel<L, M, Far::table, ODD, CHECK, W>;
+    if constexpr (ALWAYS)
+        if (!fm.nbr) kern = lb_step_kernel<L, M, Far::packed, ODD, CHECK, W>;
+    *e = cudaLaunchKernelEx(&cfg, kern, f, fm, g, k, ctrl, kstep, partials,
+                            pdl_late(one_wave) ? 1 : 0, one_wave ? 0 : 1);
+    return true;
+}
+
+// The waves that nb blocks of 128 take in form W.
+template <class L, class M, Form W>
+static long long waves(long long nb) {
+    static const long long resident = std::max(
+        resident_blocks(lb_step_kernel<L, M, Far::table, false, false, W>, kFlowThreads), 1ll);
+    return (nb + resident - 1) / resident;
+}
+
+template <class L, class M, bool ODD, bool CHECK>
+static cudaError_t launch_step_one(typename M::S* f, const FlowMap& fm, const Grid& g,
+                                   const LbParams& k, const FlowCtrl* ctrl, int kstep,
+                                   double* partials, cudaStream_t s) {
+    cudaError_t e = cudaSuccess;
     // D3Q19 float64 stages its gather in shared memory, because in registers it
     // takes 118 of them; a solve whose blocks all fit at four an SM has the
-    // registers (54^3: 4.16 -> 3.94 us an iteration, 44^3 3.23 -> 3.07; beyond
-    // one such wave it loses, 60^3 5.3 against 5.6).
+    // registers (54^3: 4.16 -> 3.94 us an iteration, 44^3 3.23 -> 3.07).  One
+    // that fits at five an SM gathers into 96 registers, in blocks of 64 that
+    // spread evenly over the SMs (57^3 4.76 -> 4.54, 56^3 4.61 -> 4.51, 59^3
+    // 4.77 -> 4.80; in blocks of 128 57^3 4.67); beyond, staging wins (60^3
+    // 5.3 against 5.6).
     if constexpr (M::staged && L::Q == 19) {
-        auto reg = lb_step_kernel<L, M, Far::table, ODD, CHECK, true>;
-        static const long long wave = resident_blocks(reg);
-        if (fm.nbr && nb <= wave)
-            return cudaLaunchKernelEx(&cfg, reg, f, fm, g, k, ctrl, kstep, partials,
-                                      pdl_late(true) ? 1 : 0, 0);
+        if (fm.nbr && launch_form<L, M, ODD, CHECK, Form::four, false>(f, fm, g, k, ctrl, kstep,
+                                                                       partials, s, &e))
+            return e;
+        if constexpr (!CHECK)
+            if (fm.nbr && launch_form<L, M, ODD, CHECK, Form::halves, false>(f, fm, g, k, ctrl, kstep,
+                                                                             partials, s, &e))
+                return e;
     }
-    auto kern = fm.nbr ? lb_step_kernel<L, M, Far::table, ODD, CHECK, false>
-                       : lb_step_kernel<L, M, Far::packed, ODD, CHECK, false>;
-    // both forms are held to the same register budget
-    static const long long resident = resident_blocks(kern);
-    const bool one_wave = nb <= resident;
-    return cudaLaunchKernelEx(&cfg, kern, f, fm, g, k, ctrl, kstep, partials,
-                              pdl_late(one_wave) ? 1 : 0, one_wave ? 0 : 1);
+    // D2Q9 takes the form of more blocks an SM where that saves a wave: us an
+    // iteration, wide / narrow, float64 500^2 (1172 blocks, 1036 / 1332 at
+    // once) 4.26 / 3.48, 530^2 4.45 / 3.84, 700^2 6.46 / 5.86, float32 560^2
+    // (1469 blocks, 1332 / 1480) 3.59 / 3.20, float16 3.53 / 3.22; with as many
+    // waves float32 600^2 3.72 / 3.81, 800^2 5.40 / 5.54, float16 400^2 2.37 /
+    // 2.43.
+    if constexpr (L::Q == 9 && M::narrow_blocks > 0) {
+        const long long nb = flow_blocks(fm.nf);
+        if (waves<L, M, Form::narrow>(nb) < waves<L, M, Form::wide>(nb)) {
+            launch_form<L, M, ODD, CHECK, Form::narrow, true>(f, fm, g, k, ctrl, kstep, partials, s, &e);
+            return e;
+        }
+    }
+    launch_form<L, M, ODD, CHECK, Form::wide, true>(f, fm, g, k, ctrl, kstep, partials, s, &e);
+    return e;
 }
 
 template <class L, class M>

@@ -65,10 +65,16 @@ def footprint(req):
         slots = ladder_slots(limit, float(a["ratio"]))
         code = getattr(a["chem"], "biofilm_code", None)
         nm = nf + (0 if code is None else int(np.count_nonzero(mat == code)))
+        # neighbours: 16-bit distances, or places where some distance may exceed
+        # 16 bits (two planes of the first axis reach that far at most)
+        plane = n // max(int(mat.shape[0]), 1)
+        near = (8 if 2 * plane <= 0xffff else 16) * nd
         # per voxel flags, scratch and one grid of a fetched snapshot; per solute
-        # voxel the list, neighbours, faces, flags and two states; the ladder
-        adr = n * (4 + 1 + 4 + 4 * ns) + nm * (4 + 24 + 24 + 4 + 8 * ns)
-        adr += 4 * n * ns * slots + 4 * (limit + 1)
+        # voxel the list, neighbours, faces, flags, the tree of its means (below
+        # a byte) and two states, with the inlet plane's own values behind their
+        # rows; the ladder
+        adr = n * (4 + 1 + 4 + 4 * ns) + nm * (4 + near + 8 * nd + 4 + 1)
+        adr += 8 * ns * (nm + plane + 32) + 4 * n * ns * slots + 4 * (limit + 1)
     # the flow's small buffers stay with the context during its transport
     return common + max(flow, adr + min(flow, _FLOW_KEEP)) + (1 << 20)
 

@@ -216,6 +216,7 @@ extern "C" int prt_physics_stage(prt_ctx* ctx, const float* out, const uint8_t* 
     CK(P.mat.ensure((size_t)g.n));
     CK(copy_in(ctx, P.out.p, out, (size_t)nf * 4));
     CK(copy_in(ctx, P.mat.p, mat, (size_t)g.n));
+    CK(cudaStreamSynchronize(ctx->stream));  // pinned arrays are read by now, too
     P.staged_out = nf;
     P.staged_mat = g.n;
     return PRT_OK;

@@ -317,8 +317,8 @@ int adr_run_finish(prt_ctx* ctx, prt_adr_result* res);
 int flow_loop_async(prt_ctx* ctx);
 int adr_loop_async(prt_ctx* ctx);
 // Copies on the context's stream between device memory and the caller's
-// (transfer.cu).  copy_out returns with the data in place; after copy_in the
-// caller's memory has been read.
+// (transfer.cu).  copy_out returns with the data in place; after copy_in
+// pageable memory has been read, pinned memory once the stream was waited for.
 // A device's contexts share its pinned chunks: transfer_open and transfer_close
 // count them, and the last one's end gives the chunks back.
 void transfer_open(int device);

@@ -1,4 +1,5 @@
-"""What calls of one process share, and what a context gives back."""
+"""What calls of one process share, what a context gives back, and when the
+caller's memory is its own again."""
 
 import ctypes
 import threading
@@ -71,5 +72,30 @@ def test_flow_release_gives_the_memory_back():
         held = before - device_memory(0)[0]
         assert 0 < held <= (40 << 20)  # at most 32 MiB, and the allocator's rounding
         assert np.array_equal(solve(), want)
+    finally:
+        ctx.close()
+
+
+def test_a_pinned_result_is_the_callers_again_once_staged():
+    """prt_physics_stage has read pinned arrays when it returns: overwriting
+    them at once changes nothing of the statistics."""
+    import torch
+    from prtlb_gpu import _lib
+    L = _lib.lib()
+    n_t, ns, shape = 6, 4, (128, 128, 96)
+    dims = (ctypes.c_int32 * 3)(*shape)
+    out = torch.empty((n_t, ns) + shape, dtype=torch.float32, pin_memory=True)
+    mat = torch.full(shape, 2, dtype=torch.uint8).pin_memory()
+    ctx = _lib.Context(0)
+    try:
+        for value in (0.25, 0.5, 0.75):
+            out.fill_(value)
+            ctx.check(L.prt_physics_stage(ctx.handle, ctypes.c_void_p(out.data_ptr()),
+                                          ctypes.c_void_p(mat.data_ptr()), 3, dims, n_t, ns))
+            out[n_t - 1].fill_(2.0)  # the last to be copied
+            st = _lib.PhysicsStats()
+            ctx.check(L.prt_physics_stats_dev(ctx.handle, None, None, 3, dims, n_t, ns, 2,
+                                              ctypes.byref(st)))
+            assert [st.pore_max[j] for j in range(ns)] == [value] * ns
     finally:
         ctx.close()

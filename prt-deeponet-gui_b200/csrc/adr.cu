@@ -154,7 +154,7 @@ __global__ void adr_tables_kernel(const float* __restrict__ vel, AdrDev d, float
     const VoxelPos v = voxel_pos(c, g);
     for (int i = 0; i < d.nd; ++i) {
         const int a = (d.nd == 3) ? i : (i == 0 ? 0 : 2);
-        const long long at = (long long)i * d.nm + k;
+        const size_t at = axis_place<true>(i, (unsigned)k, d.nm);
         const int4 q = neighbours(d, map, (int)k, i, fl, v);
         if (near) {
             const unsigned u = (unsigned)k;

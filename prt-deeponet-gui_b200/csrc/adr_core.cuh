@@ -119,7 +119,8 @@ __device__ __forceinline__ float ld_if_down(const float* p, float u) {
 // What one transport step needs of solute voxel k that does not change during
 // a run: per axis the distances to its neighbours (x, y down to the far low and
 // the low, z, w up to the high and the far high) and its low and high face velocity, and its flags where the run
-// reads them.  WIDE: from AdrDev::nb instead of AdrDev::near.
+// reads them.  WIDE: from AdrDev::nb instead of AdrDev::near.  BIG: the tables
+// may exceed 32-bit places.
 template <int ND>
 struct VoxelSetup {
     int4 nb[ND];
@@ -127,21 +128,21 @@ struct VoxelSetup {
     uint32_t fl;
 };
 
-template <int ND, bool BF, bool WIDE>
+template <int ND, bool BF, bool WIDE, bool BIG = WIDE>
 __device__ __forceinline__ VoxelSetup<ND> voxel_setup(const AdrDev& d, const prt_adr_params& p,
                                                       unsigned k) {
     VoxelSetup<ND> s;
-    const unsigned nm = (unsigned)d.nm;
 #pragma unroll
     for (int i = 0; i < ND; ++i) {
+        const size_t at = axis_place<BIG>(i, k, d.nm);
         if constexpr (WIDE) {
-            const int4 q = __ldg(d.nb + (i * nm + k));
+            const int4 q = __ldg(d.nb + at);
             s.nb[i] = make_int4((int)k - q.x, (int)k - q.y, q.z - (int)k, q.w - (int)k);
         } else {
-            const uint2 q = __ldg(d.near + (i * nm + k));
+            const uint2 q = __ldg(d.near + at);
             s.nb[i] = make_int4(q.x & 0xffffu, q.x >> 16, q.y & 0xffffu, q.y >> 16);
         }
-        s.fc[i] = __ldg(d.face + (i * nm + k));
+        s.fc[i] = __ldg(d.face + at);
     }
     s.fl = (BF || (p.abio_on && p.surface_only)) ? __ldg(d.cflags + k) : 0u;
     return s;

@@ -110,7 +110,7 @@ __global__ void __launch_bounds__(T, 1)
     ClusterVoxel<ND> v;
     if (live) {
         const VoxelSetup<ND> s = d.near ? voxel_setup<ND, BF, false>(d, p, k)
-                                        : voxel_setup<ND, BF, true>(d, p, k);
+                                        : voxel_setup<ND, BF, true, false>(d, p, k);
         v.fl = s.fl;
         const uint32_t base = shared_address(&st[0][0][0]);
         auto place = [&](unsigned q) { return in_block(base + (q % span) * 4, q / span); };

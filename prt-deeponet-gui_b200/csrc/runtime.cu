@@ -649,7 +649,8 @@ extern "C" int prt_adr_begin(prt_ctx* ctx, const prt_adr_params* p) {
     A.p = *p;
     A.d.ns = p->ns;
     const size_t nm = (size_t)std::max(A.d.nm, 1ll);
-    // the neighbours: 16-bit distances where they suffice, else places
+    // the neighbours: 16-bit distances where they suffice (adr_use_near), else
+    // places
     int* map = A.tmp.as<int>();
     unsigned* d_reach = reinterpret_cast<unsigned*>(A.vstats.as<char>() + 52);
     CK(adr_launch_map(A.d, map, d_reach, s));
@@ -658,7 +659,7 @@ extern "C" int prt_adr_begin(prt_ctx* ctx, const prt_adr_params* p) {
     CK(cudaStreamSynchronize(s));
     A.d.near = nullptr;
     A.d.nb = nullptr;
-    if (reach <= 0xffffu && !wide_neighbours()) {
+    if (adr_use_near(reach, p->nd, A.d.nm) && !wide_neighbours()) {
         CK(A.near.ensure(nm * p->nd * sizeof(uint2)));
         A.d.near = A.near.as<uint2>();
     } else {

@@ -341,7 +341,8 @@ typedef struct prt_batch prt_batch;
  * `graph_steps` steps (0: 20). */
 int prt_batch_create(int device, int32_t graph_steps, prt_batch** out);
 
-/* Waits for the batch's work and frees it; the jobs are left as they are. */
+/* Waits for the batch's work and frees it; jobs still in it are taken out as by
+ * prt_batch_remove. */
 void prt_batch_destroy(prt_batch* b);
 
 const char* prt_batch_last_error(const prt_batch* b);

@@ -401,6 +401,35 @@ int ensure_graph(prt_batch* b) {
     return PRT_OK;
 }
 
+// The count of a job that leaves before its loop has ended, to its control block
+// (the batch writes it there only on the steps that check); the batch's work
+// is done.
+cudaError_t write_back(const prt_batch* b, prt_ctx* job) {
+    if (!job->batch_g0_set) return cudaSuccess;
+    const long long count = b->steps_run - job->batch_g0;
+    cudaStream_t s = job->stream;
+    const auto copy = [s](void* dst, const void* src, size_t n, cudaMemcpyKind kind) {
+        const cudaError_t e = cudaMemcpyAsync(dst, src, n, kind, s);
+        return e == cudaSuccess ? cudaStreamSynchronize(s) : e;
+    };
+    cudaError_t e;
+    if (job->flow_armed) {
+        FlowCtrl fc;
+        e = copy(&fc, job->flow.ctrl.p, sizeof(fc), cudaMemcpyDeviceToHost);
+        if (e != cudaSuccess || fc.done) return e;
+        fc.it_base = count;
+        fc.iters = count;
+        job->flow.at = count;
+        return copy(job->flow.ctrl.p, &fc, sizeof(fc), cudaMemcpyHostToDevice);
+    }
+    AdrCtrl ac;
+    e = copy(&ac, job->adr.ctrl.p, sizeof(ac), cudaMemcpyDeviceToHost);
+    if (e != cudaSuccess || ac.done) return e;
+    ac.n_base = count;
+    ac.n_stop = segment_end(count, ac.segment, ac.check, ac.limit);
+    return copy(job->adr.ctrl.p, &ac, sizeof(ac), cudaMemcpyHostToDevice);
+}
+
 }  // namespace
 
 void prt::batch_detach(prt_ctx* c) {
@@ -621,7 +650,11 @@ extern "C" void prt_batch_destroy(prt_batch* b) {
     if (b->stream) cudaStreamSynchronize(b->stream);
     {
         std::lock_guard<std::mutex> lk(b->mu);
-        for (prt_ctx* c : b->jobs) c->batch = nullptr;
+        for (prt_ctx* c : b->jobs) {
+            write_back(b, c);  // an unfinished job goes on from where it was
+            c->batch = nullptr;
+            c->batch_g0_set = false;
+        }
         b->jobs.clear();
     }
     b->graph.release();
@@ -672,35 +705,8 @@ extern "C" int prt_batch_remove(prt_batch* b, prt_ctx* job) {
     if (!b || !job) return bfail(b, PRT_E_INVALID, "null argument");
     if (job->batch != b) return bfail(b, PRT_E_INVALID, "the context is not in this batch");
     if (b->in_flight) return bfail(b, PRT_E_STATE, "wait for the launch before removing jobs");
-    // a job leaving before its loop ended gets its count written back: the
-    // batch writes it to the control block only on the steps that check
-    if (job->batch_g0_set) {
-        BK(cudaSetDevice(b->device));
-        const long long count = b->steps_run - job->batch_g0;
-        cudaStream_t s = job->stream;
-        if (job->flow_armed) {
-            FlowCtrl fc;
-            BK(cudaMemcpyAsync(&fc, job->flow.ctrl.p, sizeof(fc), cudaMemcpyDeviceToHost, s));
-            BK(cudaStreamSynchronize(s));
-            if (!fc.done) {
-                fc.it_base = count;
-                fc.iters = count;
-                job->flow.at = count;
-                BK(cudaMemcpyAsync(job->flow.ctrl.p, &fc, sizeof(fc), cudaMemcpyHostToDevice, s));
-                BK(cudaStreamSynchronize(s));
-            }
-        } else {
-            AdrCtrl ac;
-            BK(cudaMemcpyAsync(&ac, job->adr.ctrl.p, sizeof(ac), cudaMemcpyDeviceToHost, s));
-            BK(cudaStreamSynchronize(s));
-            if (!ac.done) {
-                ac.n_base = count;
-                ac.n_stop = segment_end(count, ac.segment, ac.check, ac.limit);
-                BK(cudaMemcpyAsync(job->adr.ctrl.p, &ac, sizeof(ac), cudaMemcpyHostToDevice, s));
-                BK(cudaStreamSynchronize(s));
-            }
-        }
-    }
+    BK(cudaSetDevice(b->device));
+    BK(write_back(b, job));
     batch_detach(job);
     return PRT_OK;
 }

@@ -27,7 +27,7 @@ def pack(edge, seed=4):
     return random_pack((edge, edge - 3, edge + 2), 0.5, 2.0, 3.5, seed=seed)
 
 
-def in_batch(ctx, steps, done=0):
+def in_batch(ctx, steps, done=0, remove=True):
     """`steps` steps of the started solve inside a batch, which it then leaves."""
     from prtlb_gpu import _lib
     from prtlb_gpu.batch import Batch
@@ -38,7 +38,8 @@ def in_batch(ctx, steps, done=0):
         b._check(L.prt_batch_add(b.handle, ctx.handle))
         b._check(L.prt_batch_run(b.handle, steps, ctypes.byref(n)))
         assert n.value == done
-        b._check(L.prt_batch_remove(b.handle, ctx.handle))
+        if remove:
+            b._check(L.prt_batch_remove(b.handle, ctx.handle))
     finally:
         b.close()
 
@@ -50,7 +51,7 @@ def wait(ctx):
         ctx.check(_lib.lib().prt_ctx_busy(ctx.handle, ctypes.byref(busy)))
 
 
-def flow(g, precision, nit, tol, left=0, launches=1):
+def flow(g, precision, nit, tol, left=0, launches=1, remove=True):
     """(field, iterations, converged, change, permeability) of a started solve."""
     from prtlb_gpu import _lib
     from prtlb_gpu.flow import flow_params
@@ -60,7 +61,7 @@ def flow(g, precision, nit, tol, left=0, launches=1):
     try:
         ctx.check(L.prt_flow_start(ctx.handle, g8.ctypes.data_as(ctypes.c_void_p), ctypes.byref(p)))
         if left:
-            in_batch(ctx, left, int(left >= nit))
+            in_batch(ctx, left, int(left >= nit), remove)
         for _ in range(launches):
             ctx.check(L.prt_flow_launch(ctx.handle))
             wait(ctx)
@@ -108,6 +109,11 @@ def test_a_loop_that_a_batch_finished_launched_again_changes_nothing():
 def test_a_flow_that_a_batch_leaves_just_below_its_cap():
     g = pack(LARGE)
     same_flow(flow(g, "fp64", 23, 0.0, 7), flow(g, "fp64", 23, 0.0))
+
+
+def test_a_flow_goes_on_after_its_batch_was_destroyed():
+    g = pack(SMALL)
+    same_flow(flow(g, "fp64", 333, 0.0, 20, remove=False), flow(g, "fp64", 333, 0.0))
 
 
 def transport(g, v, steps, most, left=0, launches=1):

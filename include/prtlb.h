@@ -324,7 +324,8 @@ int prt_adr_finish(prt_ctx* ctx, prt_adr_result* res);
 /* Concurrent solves: enqueue the whole flow loop of a started solve
  * (prt_flow_start), or the whole transport loop of a started run
  * (prt_adr_start), on the context's own stream and return at once; many
- * contexts then run side by side on one GPU, each loop as one CUDA graph.
+ * contexts then run side by side on one GPU, each loop as one launch.  A solve
+ * that left a batch goes on from where it was.
  * prt_ctx_busy reports whether the enqueued loop is still running; the
  * results are read with prt_flow_finish / prt_adr_finish (which wait). */
 int prt_flow_launch(prt_ctx* ctx);
@@ -357,7 +358,8 @@ int prt_batch_add(prt_batch* b, prt_ctx* job);
  * launches.  A batch keeps its jobs' iteration / step counts implicitly and
  * writes them to a job's control block only on the steps that check or end
  * it, so removing an unfinished job writes its count back; it can then join
- * another batch (prt_batch_add) and go on from where it was. */
+ * another batch (prt_batch_add) or run by itself (prt_flow_launch,
+ * prt_adr_launch), and goes on from where it was. */
 int prt_batch_remove(prt_batch* b, prt_ctx* job);
 
 /* Enqueues `steps` batch steps and returns without waiting. */

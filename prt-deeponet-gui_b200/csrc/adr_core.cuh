@@ -212,8 +212,8 @@ __device__ __forceinline__ float transport_one(const float* __restrict__ Ck,
 // the division (t > 0).  r t <= 0.49 c with c not tiny: the two roundings of
 // the products and the two of the reference's cap move either side by less
 // than 1e-6 of it, and the least product that passes, 4.9e-31, is far above
-// the subnormal range.  r <= 0 <= c: the cap is at least +0.  A NaN or an
-// infinite r fails both.
+// the subnormal range.  r <= 0 <= c: the cap is at least +0.  A NaN fails both;
+// an infinite r passes only with an infinite c, where the cap is infinite too.
 __device__ __forceinline__ bool below_half(float r, float c, float t) {
     return (r * t <= 0.49f * c && c >= 1e-30f) || (r <= 0.f && c >= 0.f);
 }

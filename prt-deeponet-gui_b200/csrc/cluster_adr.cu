@@ -7,9 +7,9 @@
 //
 // Bound by the barrier and shared-memory latency (0.85 us a step on the
 // smallest grids), then by the arithmetic of the voxels a block holds.  us a
-// step, launches -> cluster: Monod 16^3 2.02 -> 0.97, 24^3 2.03 -> 1.23, 28^3
-// 1.99 -> 1.39; four chemicals 24^3 3.12 -> 2.51, 28^3 3.19 -> 3.00; 2D first
-// order 64^2 1.94 -> 0.91, 128^2 2.06 -> 1.17.
+// step, launches -> cluster: Monod 16^3 2.02 -> 0.97, 24^3 2.01 -> 1.20, 28^3
+// 1.99 -> 1.39; four chemicals 24^3 3.12 -> 2.44, 28^3 3.19 -> 3.00; 2D first
+// order 64^2 1.94 -> 0.88, 128^2 1.99 -> 1.13.
 #include "adr_core.cuh"
 #include "cluster.cuh"
 

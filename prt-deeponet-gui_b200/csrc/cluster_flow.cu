@@ -8,8 +8,8 @@
 // smallest grids) and then by the arithmetic of the slots a block holds, about
 // 0.45 us for each further 128 slots of D3Q19 float64, 0.3 us of float32,
 // which sets the largest size taken.  us an iteration, launches -> cluster:
-// 16^3 float64 2.29 -> 1.04, 24^3 2.31 -> 1.75, 26^3 2.22 -> 1.93, 24^3 float32
-// 2.15 -> 1.30;
+// 16^3 float64 2.29 -> 1.02, 24^3 2.31 -> 1.75, 26^3 2.22 -> 1.93, 24^3 float32
+// 2.15 -> 1.33;
 // D2Q9 64^2 float64 1.79 -> 0.82, 128^2 1.81 -> 1.16, float32 1.69 ->
 // 0.86, 150^2 float64 1.83 -> 1.61.
 #include "cluster.cuh"

@@ -223,7 +223,6 @@ __global__ void fluid_flag_kernel(const uint8_t* __restrict__ mat, long long n, 
     if (c < n) flag[c] = (mat[c] == pore) ? 1 : 0;
 }
 
-// imap[cells[k]] = k (imap was filled with -1 first).
 // imap[cells[k]] = k (imap was filled with -1 first); then cells[k] is
 // rewritten from the voxel index to the packed coordinates.
 __global__ void imap_scatter_kernel(int* __restrict__ cells, int nf, int* __restrict__ imap,

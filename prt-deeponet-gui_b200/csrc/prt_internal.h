@@ -270,7 +270,7 @@ inline long long flow_pack_bytes(int q, long long nf) {
 
 // Whether a solve with nf pore voxels, rows of rs elements and populations
 // of es bytes gets the plain table on a device with l2_bytes of L2: when the
-// lattice and the table fit in half of it.
+// lattice and the table fit in three quarters of it.
 inline bool flow_use_nbr(int q, long long nf, long long rs, long long es, long long l2_bytes) {
     return nf > 0 && q * rs * es + flow_nbr_bytes(q, nf) <= l2_bytes / 4 * 3;
 }

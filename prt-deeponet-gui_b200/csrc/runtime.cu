@@ -1,7 +1,7 @@
 // runtime.cu -- the C ABI of libprtlb.so (include/prtlb.h): contexts, device
-// buffers, and the two time loops run as CUDA graphs with a device-side
-// while-condition, so a whole flow solve or transport solve is one graph
-// launch and the host waits once.
+// buffers, and the two time loops run inside one cluster (small grids) or as
+// CUDA graphs with a device-side while-condition, so a whole flow solve or
+// transport solve is one launch and the host waits once.
 #include <cstdlib>
 #include <new>
 

@@ -5,8 +5,9 @@ chemistry into float32 lattice numbers on the host, with the same numpy
 scalar types and promotion the reference uses, so the time step, check
 interval and every coefficient are the reference's to the last bit.  The
 per-voxel work -- face tables, the fused transport + reaction step, the
-snapshot ladder and the convergence means -- runs in libprtlb.so as one CUDA
-graph with a device-side while condition.  Snapshot picking and the ``info``
+snapshot ladder and the convergence means -- runs in libprtlb.so as one kernel
+of a thread-block cluster for a small grid, else as one CUDA graph with a
+device-side while condition.  Snapshot picking and the ``info``
 dict (prtlb_3d.py:1550-1595) are host logic over the step numbers.
 
 Keyword-only additions: ``device`` and ``ctx``.

@@ -411,9 +411,9 @@ class Batch(object):
 
 class StreamBatch(Batch):
     """The same interface over concurrent single-solve loops: every solve
-    runs its own flow loop, then its own transport loop, each as one CUDA
-    graph launched on the solve's own stream (prt_flow_launch /
-    prt_adr_launch), so many solves share the GPU at once and each keeps the
+    runs its own flow loop, then its own transport loop, each as one launch (a
+    CUDA graph, or a cluster's kernel for a small grid) on the solve's own
+    stream (prt_flow_launch / prt_adr_launch), so many solves share the GPU at once and each keeps the
     single-solve kernels.  wait() returns when at least one solve finished
     its current loop (or after `poll_s` with nothing finished)."""
 

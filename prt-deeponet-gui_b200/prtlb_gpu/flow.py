@@ -3,8 +3,9 @@
 Signatures, defaults, returned array, ``info`` keys, refusals and warnings
 follow the reference (3D/tools/prtlb_2d.py:348-486, prtlb_3d.py:348-456,
 FlowConvergence prtlb_3d.py:168-252, _checked_flow prtlb_3d.py:267-316).
-The solve itself runs in libprtlb.so: one CUDA graph per solve whose body is
-50 fused stream-collide iterations plus the convergence check.
+The solve itself runs in libprtlb.so: one kernel of a thread-block cluster for
+a small grid, else one CUDA graph per solve whose body is 50 fused
+stream-collide iterations plus the convergence check.
 
 Keyword-only additions: ``precision`` ("fp64" default = the reference's
 arithmetic; "fp32" stores f_i - w_i in float32 and forms the momentum and

@@ -20,8 +20,8 @@ arguments and outputs:
                          stencil, no walk)
 
 The reference labels components with scipy and walks with a Python queue,
-one voxel at a time; here each level of the walk is one kernel launch over
-the grid.  Results are bit-identical to the reference's (tests/test_prep.py).
+one voxel at a time; here the walk runs level by level on bit masks inside one
+kernel, or on large grids with a kernel launch per level.  Results are bit-identical to the reference's (tests/test_prep.py).
 """
 
 import ctypes
